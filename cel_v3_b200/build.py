@@ -22,7 +22,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # keeps the remaining scalar code faithful too.
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompiler", "-fPIC,-ffp-contract=off,-O2",
          "-I", INCLUDE, "--expt-relaxed-constexpr"]
-SOURCES = ["api.cu", "spmv.cu", "blas1.cu", "pcg.cu", "krylov.cu", "ir.cu", "ru.cu", "elm.cu", "noalloc.cu",
+SOURCES = ["api.cu", "spmv.cu", "blas1.cu", "pcg.cu", "pcg_onchip.cu", "krylov.cu", "ir.cu", "ru.cu", "elm.cu", "noalloc.cu",
            "batched.cu", "selftest.cu", "multirhs.cu", "adjoint.cu", "dist.cu", "dist_solve.cu", "assemble.cu",
            "blockjacobi.cu"]
 

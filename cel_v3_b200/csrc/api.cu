@@ -362,6 +362,7 @@ void free_mat_arrays(celg_mat* m) {
   cudaFree(m->csr.dict);
   cudaFree(m->csr.pid);
   cudaFree(m->csr.pat);
+  sell_free(m->csr);
   cudaFree(m->jad.begin);
   cudaFree(m->jad.ci);
   cudaFree(m->jad.v);
@@ -591,6 +592,7 @@ extern "C" int celg_destroy(celg_handle* h) {
   cudaFree(h->ru_state_d);
   cudaFreeHost(h->ru_state_h);
   cudaFree(h->hist_d);
+  cudaFree(h->oc_slots);
   cudaFree(h->gm_work);
   cudaFree(h->gm_state_d);
   cudaFreeHost(h->gm_state_h);
@@ -780,6 +782,8 @@ extern "C" int celg_mat_scale_diagonal(celg_mat* m) {
   if (!st) st = launch_row_scale(m->h, m);
   if (st) return st;
   m->scaled = true;
+  CELG_CUDA(cudaStreamSynchronize(m->h->stream));
+  sell_free(m->csr);
   st = launch_jacobi_setup(m->h, m);  // jacobi = sqrt|d| / d
   if (st) return st;
   if (m->jad.mmax >= 0) st = build_jad(m);

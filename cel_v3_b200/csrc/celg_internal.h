@@ -38,6 +38,12 @@ struct CsrDev {
   uint8_t* pid = nullptr;
   int* pat = nullptr;
   int npat = 0;
+  // copy in slices of 32 rows for the one-kernel solve (pcg_onchip.cu)
+  double* sell_v = nullptr;
+  float* sell_v32 = nullptr;
+  int* sell_c = nullptr;     // columns (no row patterns)
+  int* sell_base = nullptr;  // first entry / 32 of each slice (no row patterns)
+  long sell_total = -1;      // entries; -1: not looked at yet, 0: not worth it
 };
 
 struct JadDev {
@@ -88,6 +94,9 @@ struct celg_handle {
   std::vector<celg::GraphEntry> graphs;
   double* hist_d = nullptr;
   int hist_cap = 0;
+  // exchange slots of the one-kernel solve (oc_cap doubles and a tail)
+  double* oc_slots = nullptr;
+  size_t oc_cap = 0;
   // host-buffer solve staging (stable pointers keep cached graphs valid)
   double* sb = nullptr;
   double* sx = nullptr;
@@ -184,6 +193,8 @@ int ensure_f32(celg_handle* h, size_t n);
 int ensure_offset_dict(celg_handle* h, celg_mat* m);
 // the same for any CSR array set (left unset beyond 256 distinct offsets)
 int build_offset_dict_csr(celg_handle* h, CsrDev& A);
+// pcg_onchip.cu: drop the sliced copy (the values changed, or the matrix goes)
+void sell_free(CsrDev& A);
 int alloc_csr(celg_mat* m, int n, int nnz, int ncols);
 int finish_csr(celg_handle* h, celg_mat* m, int base);
 void free_mat_arrays(celg_mat* m);

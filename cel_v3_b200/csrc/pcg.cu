@@ -232,7 +232,16 @@ int pcg_run(celg_handle* h, const PcgBind<VT>& B, const celg_params* p, const vo
   if (st) return st;
   CELG_CUDA(cudaMemsetAsync(h->err_d, 0, sizeof(int), h->stream));
 
-  if (!graphs_enabled()) {
+  bool onchip = false;
+  if (graphs_enabled() && !B.jad && !B.bj) {
+    CELG_CUDA(cudaEventRecord(h->ev0, h->stream));
+    st = pcg_onchip<VT>(h, *B.A, B, p, hist_cap, &onchip);
+    if (st) return st;
+    if (onchip) CELG_CUDA(cudaEventRecord(h->ev1, h->stream));
+  }
+  if (onchip) {
+    // one kernel, which leaves its state in h->state_h
+  } else if (!graphs_enabled()) {
     CELG_CUDA(cudaEventRecord(h->ev0, h->stream));
     st = run_host_loop(h, B, p, PcgArgs{h->state_d, h->hist_d, hist_cap, p->iter_max, 0, h->err_d});
     if (st) return st;
@@ -250,8 +259,9 @@ int pcg_run(celg_handle* h, const PcgBind<VT>& B, const celg_params* p, const vo
     CELG_CUDA(cudaGraphLaunch(ge->exec, h->stream));
     CELG_CUDA(cudaEventRecord(h->ev1, h->stream));
   }
-  CELG_CUDA(cudaMemcpyAsync(h->state_h, h->state_d, sizeof(PcgState), cudaMemcpyDeviceToHost,
-                            h->stream));
+  if (!onchip)
+    CELG_CUDA(cudaMemcpyAsync(h->state_h, h->state_d, sizeof(PcgState), cudaMemcpyDeviceToHost,
+                              h->stream));
   CELG_CUDA(cudaMemcpyAsync(h->scal_h + 8, h->err_d, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   CELG_CUDA(cudaStreamSynchronize(h->stream));
   cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1);

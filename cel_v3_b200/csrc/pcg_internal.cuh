@@ -30,7 +30,7 @@ struct PcgArgs {
 // Vectors and matrix one PCG solve runs on.
 template <typename VT>
 struct PcgBind {
-  const CsrDev* A = nullptr;
+  CsrDev* A = nullptr;
   const JadDev* jad = nullptr;  // FP64 JAD path when set
   const VT* vals = nullptr;     // CSR values used by the iteration
   const double* verify_vals = nullptr;  // FP64 values for the final check (null: skip)
@@ -59,6 +59,11 @@ int ensure_state(celg_handle* h, int hist_cap);
 template <typename VT>
 int pcg_run(celg_handle* h, const PcgBind<VT>& B, const celg_params* p, const void* mat,
             PcgState* out_state);
+// pcg_onchip.cu: the solve as one cooperative kernel, its state left in
+// h->state_h; *done = false when the system does not fit it
+template <typename VT>
+int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_params* p, int hist_cap,
+               bool* done);
 int copy_history(celg_handle* h, int len, celg_result* res);
 
 template <typename VT>

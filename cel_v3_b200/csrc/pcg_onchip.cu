@@ -1,0 +1,740 @@
+// pcg_onchip.cu -- the whole Jacobi-PCG solve of a small or medium system in
+// one cooperative kernel (the loop of pcg.cu, same arithmetic, same bits).
+//
+// What bounds a small solve is not memory but the chain of dependent steps:
+// as three graph kernels an iteration of a 32^3 system took 20 us, of which
+// the work is under one.  Here one CTA per SM keeps its rows' r, p, x, v and
+// J in shared memory for the whole solve; only p (gathered by other CTAs)
+// and the reduction terms go through L2, and an iteration is three grid-wide
+// exchanges instead of three kernels and a loop node.
+//
+// Work split.  A unit is what one warp contributes to the reduction tree of
+// celg_device.cuh: rows 1024 t + 32 w + lane + 256 k (k = 0..3) of tile t,
+// warp w.  Its warp sum depends on nothing else, so units (8 per tile) are
+// dealt to the CTAs in equal contiguous runs, one warp per unit at a time,
+// and every SM gets the same share to within 128 rows (whole 1024-row tiles
+// leave a system of 200 tiles 148 SMs with two tiles on some and one on
+// most).
+//
+// Exchanges.  A warp sum is published by storing it over a sentinel (a NaN
+// pattern that no published value has); CTA 0 polls the slots, folds them in
+// the tree's order and publishes the totals the same way, and every other
+// CTA polls that one word: two trips through L2 with the data in them.
+// (All CTAs polling all slots needs one trip, but 128 CTAs spinning on the
+// same 2 KB hold up the stores: 9100 cycles an exchange against 2000.)  The
+// slots of an iteration are set back to the sentinel once they are known to
+// have been read.  p is published by a release of one arrival counter, which
+// a thread of each CTA acquires (2400 cycles; a flag per CTA: 4200).  Every
+// wait is bounded (kWaitLimitNs).
+//
+// Matrix.  Values in slices of 32 rows, entry e of the slice's lane l at
+// e * 32 + l, so that a warp's loads are whole lines (row-major values would
+// touch 14 lines per load for 7 entries a row, 32 for 16 and more).  With
+// row patterns (spmv_kernels.cuh) the columns come from the pattern table
+// and the slices are kPatLen wide; units whose values fit keep them in
+// shared memory.  Otherwise int32 columns are stored like the values.
+#include <cooperative_groups.h>
+#include <cub/cub.cuh>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+#include <mutex>
+
+#include "graph.cuh"
+#include "pcg_internal.cuh"
+
+namespace celg {
+
+// 16 warps at 128 registers: at 32 warps and 64 registers the gathers in
+// flight per lane are fewer and every barrier costs more (53^3: 10.1 against
+// 8.7 us an iteration; 200k unstructured rows: 32 against 22)
+constexpr int kOcThreads = 512;
+constexpr int kUnitRows = 128;
+constexpr int kOcMaxSmem = 227 * 1024;
+constexpr int kOcTail = 64;  // doubles after the slots: the totals (kSlotSets), the arrival counter
+// slot sets: p.v, (r.z, r.r) twice, ||b||^2, set-up (r.z, r.r), verification
+// (pairs at even positions)
+enum OcSlot { kSlotUpd0 = 0, kSlotUpd1 = 2, kSlotInit = 4, kSlotPv = 6, kSlotB = 7, kSlotVer = 8, kSlotSets = 9 };
+// longest row of a sliced matrix: with at most 2^16 slices (kOcMaxUnits) the
+// sum of the slice widths stays within an int
+constexpr int kMaxWidth = 32767;
+constexpr long kOcMaxUnits = 1L << 14;
+constexpr unsigned long long kSentinel = ~0ull;
+
+template <typename VT>
+struct OcArgs {
+  int n, ntiles, slots, ncache;
+  const VT* sv;       // sliced values
+  const int* sc;      // sliced columns (no row patterns)
+  const int* sbase;   // first entry of each slice / 32 (no row patterns)
+  const int* rp;
+  const uint8_t* pid;
+  const int* pat;
+  int pat_ints;
+  const VT* b;
+  VT* x;
+  const VT* J;
+  VT* p;
+  double* slot;       // kSlotSets x 8 ntiles
+  double* total;      // kSlotSets + 1, pairs 16-byte aligned
+  unsigned* arrive;
+  PcgState* out;      // pinned host memory
+  double* hist;
+  int hist_cap, iter_max, x0_mode, verify;
+  double eps_abs, eps_rel;
+};
+
+__device__ __forceinline__ void publish(double* q, double v) {
+  unsigned long long u = (unsigned long long)__double_as_longlong(v);
+  if (u == kSentinel) u = 0x7ff8000000000000ull;
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(q), "l"(u) : "memory");
+}
+
+__device__ __forceinline__ void load2(const double* q, unsigned long long& a, unsigned long long& b) {
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(q) : "memory");
+}
+
+__device__ __forceinline__ bool poll_more(unsigned i, unsigned long long& t0, int* abort_) {
+  if ((i & 63u) != 63u) return true;
+  const unsigned long long t = global_ns();
+  if (!t0) t0 = t;
+  if (t - t0 <= kWaitLimitNs && !*(volatile int*)abort_) return true;
+  *(volatile int*)abort_ = 1;
+  return false;
+}
+
+// The eight warp sums of a tile, waited for, added in warp order.
+__device__ __forceinline__ double tile_sum(const double* q, int* abort_) {
+  unsigned long long w[8];
+  unsigned long long t0 = 0;
+  for (unsigned i = 0;; ++i) {
+#pragma unroll
+    for (int u = 0; u < 8; u += 2) load2(q + u, w[u], w[u + 1]);
+    bool ok = true;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) ok = ok && w[u] != kSentinel;
+    if (ok || !poll_more(i, t0, abort_)) break;
+  }
+  double s = __longlong_as_double((long long)w[0]);
+#pragma unroll
+  for (int u = 1; u < 8; ++u) s = dadd(s, __longlong_as_double((long long)w[u]));
+  return s;
+}
+
+// Shared memory of a CTA: fold scratch, the tile sums of up to two
+// reductions, the pattern table, then per unit slot the row data.
+template <typename VT>
+struct OcSmem {
+  double* red;   // 16
+  int* abort_;
+  double* tp;    // 2 ntiles
+  int* pat;
+  int* meta;     // row length (and pattern index << 16)
+  VT *r, *p, *x, *J, *v, *val;
+  size_t bytes;
+  __host__ __device__ OcSmem(unsigned char* base, int ntiles, int pat_ints, int slots, int ncache) {
+    size_t o = 0;
+    auto take = [&](size_t b) {
+      unsigned char* q = base + o;
+      o += (b + 15) & ~(size_t)15;
+      return q;
+    };
+    red = (double*)take(16 * sizeof(double));
+    abort_ = (int*)take(16);
+    tp = (double*)take(2 * sizeof(double) * (size_t)ntiles);
+    pat = (int*)take(sizeof(int) * (size_t)pat_ints);
+    const size_t rows = (size_t)slots * kUnitRows;
+    meta = (int*)take(sizeof(int) * rows);
+    r = (VT*)take(sizeof(VT) * rows);
+    p = (VT*)take(sizeof(VT) * rows);
+    x = (VT*)take(sizeof(VT) * rows);
+    J = (VT*)take(sizeof(VT) * rows);
+    v = (VT*)take(sizeof(VT) * rows);
+    val = (VT*)take(sizeof(VT) * (size_t)ncache * kUnitRows * kPatLen);
+    bytes = o;
+  }
+};
+
+// values stream from L2 once an iteration; kept out of the small L1 that the
+// gathers live in
+__device__ __forceinline__ double ld_stream(const double* p) {
+  double v;
+  asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_stream(const float* p) {
+  float v;
+  asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int ld_stream(const int* p) {
+  int v;
+  asm("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
+// Row sum of one row of a lane (row k of unit slot `slot`), 0 + v0 x0 + v1 x1
+// + ... in stored order.  The gathers are ordinary loads: src is written by
+// other CTAs between two calls.
+template <typename VT, bool PAT>
+__device__ __forceinline__ VT row_sum(const OcArgs<VT>& a, const OcSmem<VT>& sm, const VT* src, int slot, int k,
+                                      int unit, int lane) {
+  const int tile = unit >> 3, w = unit & 7;
+  const int meta = sm.meta[slot * kUnitRows + k * 32 + lane];
+  VT t = VT(0);
+  if constexpr (PAT) {
+    const int len = meta & 0xffff;
+    const VT* xr = src + (tile * kTile + k * 256 + w * 32 + lane);
+    const int4* pq = reinterpret_cast<const int4*>(sm.pat + (meta >> 16) * kPatLen);
+    VT xv[kPatLen], vv[kPatLen];
+    if (len > 0) {  // the pattern's padding reads src[row]
+      const int4 q0 = pq[0], q1 = pq[1];
+      xv[0] = xr[q0.x];
+      xv[1] = xr[q0.y];
+      xv[2] = xr[q0.z];
+      xv[3] = xr[q0.w];
+      xv[4] = xr[q1.x];
+      xv[5] = xr[q1.y];
+      xv[6] = xr[q1.z];
+      xv[7] = xr[q1.w];
+    }
+    if (slot < a.ncache) {
+      const VT* cv = sm.val + (size_t)(slot * 4 + k) * (kPatLen * 32) + lane;
+#pragma unroll
+      for (int e = 0; e < kPatLen; ++e)
+        if (e < len) vv[e] = cv[e * 32];
+    } else {
+      const VT* gv = a.sv + (size_t)(tile * 32 + k * 8 + w) * (kPatLen * 32) + lane;
+#pragma unroll
+      for (int e = 0; e < kPatLen; ++e)
+        if (e < len) vv[e] = ld_stream(gv + e * 32);
+    }
+#pragma unroll
+    for (int e = 0; e < kPatLen; ++e)
+      if (e < len) t = vadd(t, vmul(vv[e], xv[e]));
+  } else {
+    constexpr int C = 8;  // entries per round
+    const size_t at = (size_t)__ldg(a.sbase + tile * 32 + k * 8 + w) * 32 + lane;
+    for (int e0 = 0; e0 < meta; e0 += C) {
+      int c[C];
+      VT xv[C], vv[C];
+#pragma unroll
+      for (int e = 0; e < C; ++e)
+        if (e0 + e < meta) {
+          c[e] = ld_stream(a.sc + at + (e0 + e) * 32);
+          vv[e] = ld_stream(a.sv + at + (e0 + e) * 32);
+        }
+#pragma unroll
+      for (int e = 0; e < C; ++e)
+        if (e0 + e < meta) xv[e] = src[c[e]];
+#pragma unroll
+      for (int e = 0; e < C; ++e)
+        if (e0 + e < meta) t = vadd(t, vmul(vv[e], xv[e]));
+    }
+  }
+  return t;
+}
+
+// Row sums of all of the CTA's rows into sm.v (one 32-row group per warp at
+// a time), then a barrier.
+template <typename VT, bool PAT>
+__device__ __forceinline__ void cta_spmv(const OcArgs<VT>& a, const OcSmem<VT>& sm, const VT* src, int u0, int nu) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int g = warp; g < 4 * nu; g += blockDim.x >> 5)
+    sm.v[g * 32 + lane] = row_sum<VT, PAT>(a, sm, src, g >> 2, g & 3, u0 + (g >> 2), lane);
+  __syncthreads();
+}
+
+// All CTAs' stores so far become visible to all CTAs.  The counter starts at
+// -1 (the 0xff fill), so after `epoch` exchanges (from 1) it is epoch G - 1.
+template <typename VT>
+__device__ __forceinline__ void grid_exchange(const OcArgs<VT>& a, const OcSmem<VT>& sm, unsigned epoch) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.arrive) : "memory");
+    unsigned long long t0 = 0;
+    for (unsigned i = 0;; ++i) {
+      unsigned f;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(a.arrive) : "memory");
+      if ((int)(f + 1u - epoch * gridDim.x) >= 0 || !poll_more(i, t0, sm.abort_)) break;
+    }
+  }
+  __syncthreads();
+}
+
+// The NR sums whose warp terms are in slot set `set`, in the order of
+// grid_finish; the same value in every thread of every CTA.
+template <int NR, typename VT>
+__device__ __forceinline__ void grid_sum(const OcArgs<VT>& a, const OcSmem<VT>& sm, int set, double (&tot)[NR]) {
+  if (blockIdx.x == 0) {
+    const double* q = a.slot + (size_t)set * 8 * a.ntiles;
+    for (int t = threadIdx.x; t < NR * a.ntiles; t += blockDim.x) sm.tp[t] = tile_sum(q + (size_t)t * 8, sm.abort_);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < 8 * NR) {
+      const double* tp = sm.tp + (warp >> 3) * a.ntiles;
+      double s = 0.0;
+      for (int k = (warp & 7) * 32 + lane; k < a.ntiles; k += kLanes) s = dadd(s, tp[k]);
+      s = warp_fold(s);
+      if (lane == 0) sm.red[warp] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      tot[r] = sm.red[8 * r];
+#pragma unroll
+      for (int g = 1; g < 8; ++g) tot[r] = dadd(tot[r], sm.red[8 * r + g]);
+    }
+    if (threadIdx.x < NR) publish(a.total + set + threadIdx.x, threadIdx.x ? tot[NR - 1] : tot[0]);
+  } else {
+    if (threadIdx.x == 0) {
+      unsigned long long t0 = 0, w0, w1;
+      for (unsigned i = 0;; ++i) {
+        if constexpr (NR == 2) {
+          load2(a.total + set, w0, w1);
+        } else {
+          asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w0) : "l"(a.total + set) : "memory");
+          w1 = 0;
+        }
+        if ((w0 != kSentinel && w1 != kSentinel) || !poll_more(i, t0, sm.abort_)) break;
+      }
+      sm.red[0] = __longlong_as_double((long long)w0);
+      sm.red[1] = __longlong_as_double((long long)w1);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < NR; ++r) tot[r] = sm.red[r];
+    __syncthreads();  // before the next sum writes red
+  }
+}
+
+template <typename VT, bool PAT>
+__global__ void __launch_bounds__(kOcThreads, 1) pcg_onchip_kernel(OcArgs<VT> a) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const OcSmem<VT> sm(smem, a.ntiles, a.pat_ints, a.slots, a.ncache);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = kOcThreads / 32;
+  const int nunits = a.ntiles * 8;
+  const int u0 = blockIdx.x * a.slots;
+  const int nu = max(0, min(a.slots, nunits - u0));
+  double* slot_of = a.slot;
+  auto slots = [&](int set) { return slot_of + (size_t)set * nunits; };
+  unsigned epoch = 1;
+  if (threadIdx.x == 0) *sm.abort_ = 0;
+  for (int q = threadIdx.x; q < a.pat_ints; q += kOcThreads) sm.pat[q] = a.pat[q];
+
+  // ---- x0, ||b||, row lengths, values --------------------------------------
+  for (int sl = warp; sl < nu; sl += nwarps) {
+    const int unit = u0 + sl, tile = unit >> 3, w = unit & 7;
+    double acc = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = sl * kUnitRows + k * 32 + lane;
+      const int row = tile * kTile + k * 256 + w * 32 + lane;
+      int meta = 0;
+      VT x0 = VT(0), J = VT(0);
+      if (row < a.n) {
+        meta = a.rp[row + 1] - a.rp[row];
+        if constexpr (PAT) meta |= (int)a.pid[row] << 16;
+        const VT bi = a.b[row];
+        acc = dadd(acc, dmul(D(bi), D(bi)));
+        J = a.J[row];
+        if (a.x0_mode == CELG_X0_USER) {
+          x0 = a.x[row];
+        } else {
+          x0 = a.x0_mode == CELG_X0_REF_ONES ? VT(1) : VT(0);
+          a.x[row] = x0;
+        }
+      }
+      sm.meta[i] = meta;
+      sm.x[i] = x0;
+      sm.J[i] = J;
+      sm.p[i] = sm.r[i] = sm.v[i] = VT(0);
+      if constexpr (PAT) {
+        if (sl < a.ncache) {
+          const size_t s = (size_t)(tile * 32 + k * 8 + w) * (kPatLen * 32) + lane;
+          for (int e = 0; e < (meta & 0xffff); ++e)
+            sm.val[(size_t)(sl * 4 + k) * (kPatLen * 32) + e * 32 + lane] = a.sv[s + e * 32];
+        }
+      }
+    }
+    acc = warp_fold(acc);
+    if (lane == 0) publish(slots(kSlotB) + unit, acc);
+  }
+  grid_exchange(a, sm, epoch++);
+  double one[1], two[2];
+  grid_sum<1>(a, sm, kSlotB, one);
+  const double bnorm = sqrt(one[0]);
+  double eps = a.eps_abs;
+  if (a.eps_rel > 0.0 && a.eps_rel * bnorm > eps) eps = a.eps_rel * bnorm;
+
+  // ---- r = b - A x, p = J r -------------------------------------------------
+  cta_spmv<VT, PAT>(a, sm, a.x, u0, nu);
+  for (int sl = warp; sl < nu; sl += nwarps) {
+    const int unit = u0 + sl, tile = unit >> 3, w = unit & 7;
+    double rp = 0.0, rr = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = sl * kUnitRows + k * 32 + lane;
+      const int row = tile * kTile + k * 256 + w * 32 + lane;
+      if (row < a.n) {
+        const VT ri = R<VT>(__dsub_rn(D(a.b[row]), D(vadd(VT(0), sm.v[i]))));
+        const double z = dmul(D(ri), D(sm.J[i]));
+        const VT pi = R<VT>(z);
+        sm.r[i] = ri;
+        sm.p[i] = pi;
+        a.p[row] = pi;
+        rp = dadd(rp, dmul(D(ri), z));
+        rr = dadd(rr, dmul(D(ri), D(ri)));
+      }
+    }
+    rp = warp_fold(rp);
+    rr = warp_fold(rr);
+    if (lane == 0) {
+      publish(slots(kSlotInit) + unit, rp);
+      publish(slots(kSlotInit + 1) + unit, rr);
+    }
+  }
+  grid_exchange(a, sm, epoch++);
+  grid_sum<2>(a, sm, kSlotInit, two);
+  double alpha = two[0], norm = sqrt(two[1]), sigma = 0.0, beta = 0.0, pvd = 0.0, rz = 0.0;
+  int iter = 0, err = 0;
+  const bool scribe = blockIdx.x == 0 && threadIdx.x == 0;
+  if (scribe && a.hist && a.hist_cap > 0) a.hist[0] = norm;
+  bool act = iter < a.iter_max && fabs(alpha) > kRealSmall && norm > eps;
+  int stop = *(volatile int*)sm.abort_;
+
+  while (act && !stop) {
+    // v = A p, p.v
+    cta_spmv<VT, PAT>(a, sm, a.p, u0, nu);
+    for (int sl = warp; sl < nu; sl += nwarps) {
+      double acc = 0.0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int i = sl * kUnitRows + k * 32 + lane;
+        const VT vi = vadd(VT(0), sm.v[i]);
+        sm.v[i] = vi;
+        acc = dacc_prod(acc, vi, sm.p[i]);
+      }
+      acc = warp_fold(acc);
+      if (lane == 0) publish(slots(kSlotPv) + u0 + sl, acc);
+    }
+    grid_sum<1>(a, sm, kSlotPv, one);
+    pvd = one[0];
+    sigma = alpha / pvd;
+    if (!isfinite(sigma)) {
+      err = kErrBreakdown;
+      act = false;
+      break;
+    }
+    // r += (-sigma) v, r.z, r.r
+    const int us = (iter & 1) ? kSlotUpd1 : kSlotUpd0, uo = (iter & 1) ? kSlotUpd0 : kSlotUpd1;
+    for (int sl = warp; sl < nu; sl += nwarps) {
+      double t0 = 0.0, t1 = 0.0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int i = sl * kUnitRows + k * 32 + lane;
+        const VT ri = R<VT>(dadd(D(sm.r[i]), dmul(-sigma, D(sm.v[i]))));
+        sm.r[i] = ri;
+        const double z = dmul(D(ri), D(sm.J[i]));
+        t0 = dadd(t0, dmul(D(ri), z));
+        t1 = dadd(t1, dmul(D(ri), D(ri)));
+      }
+      t0 = warp_fold(t0);
+      t1 = warp_fold(t1);
+      if (lane == 0) {
+        publish(slots(us) + u0 + sl, t0);
+        publish(slots(us + 1) + u0 + sl, t1);
+      }
+    }
+    grid_sum<2>(a, sm, us, two);
+    rz = two[0];
+    beta = rz / alpha;
+    alpha = rz;
+    norm = sqrt(two[1]);
+    ++iter;
+    if (scribe && a.hist && iter < a.hist_cap) a.hist[iter] = norm;
+    act = iter < a.iter_max && fabs(alpha) > kRealSmall && norm > eps;
+    // x += sigma p, p = beta p + J r.  Every CTA has read this iteration's
+    // p.v slots and the last iteration's r.z, r.r slots: back to the
+    // sentinel, ordered before their next use by the exchange below.
+    for (int sl = warp; sl < nu; sl += nwarps) {
+      const int unit = u0 + sl, tile = unit >> 3, w = unit & 7;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int i = sl * kUnitRows + k * 32 + lane;
+        const int row = tile * kTile + k * 256 + w * 32 + lane;
+        const double pi = D(sm.p[i]);
+        sm.x[i] = R<VT>(dadd(D(sm.x[i]), dmul(sigma, pi)));
+        if (act) {
+          const VT pn = R<VT>(dadd(dmul(beta, pi), dmul(D(sm.r[i]), D(sm.J[i]))));
+          sm.p[i] = pn;
+          if (row < a.n) a.p[row] = pn;
+        }
+      }
+      if (lane < 3) {
+        double* q = slots(lane == 0 ? kSlotPv : uo + lane - 1) + unit;
+        *reinterpret_cast<unsigned long long*>(q) = kSentinel;
+      }
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 3) {
+      double* q = a.total + (threadIdx.x == 0 ? kSlotPv : uo + threadIdx.x - 1);
+      *reinterpret_cast<unsigned long long*>(q) = kSentinel;
+    }
+    stop = *(volatile int*)sm.abort_;
+    if (act) {
+      grid_exchange(a, sm, epoch++);
+      stop = *(volatile int*)sm.abort_;
+    }
+  }
+
+  // ---- x out, ||b - A x|| ------------------------------------------------------
+  for (int sl = warp; sl < nu; sl += nwarps) {
+    const int unit = u0 + sl, tile = unit >> 3, w = unit & 7;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int row = tile * kTile + k * 256 + w * 32 + lane;
+      if (row < a.n) a.x[row] = sm.x[sl * kUnitRows + k * 32 + lane];
+    }
+  }
+  double vres = 0.0;
+  if (a.verify && !stop) {
+    grid_exchange(a, sm, epoch++);
+    cta_spmv<VT, PAT>(a, sm, a.x, u0, nu);
+    for (int sl = warp; sl < nu; sl += nwarps) {
+      const int unit = u0 + sl, tile = unit >> 3, w = unit & 7;
+      double acc = 0.0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int row = tile * kTile + k * 256 + w * 32 + lane;
+        if (row < a.n) {
+          const double ri = __dsub_rn(D(a.b[row]), dadd(0.0, D(sm.v[sl * kUnitRows + k * 32 + lane])));
+          acc = dadd(acc, dmul(ri, ri));
+        }
+      }
+      acc = warp_fold(acc);
+      if (lane == 0) publish(slots(kSlotVer) + unit, acc);
+    }
+    grid_sum<1>(a, sm, kSlotVer, one);
+    vres = bnorm > 0.0 ? sqrt(one[0]) / bnorm : sqrt(one[0]);
+  }
+  if (scribe) {
+    PcgState* o = a.out;
+    o->alpha = alpha;
+    o->sigma = sigma;
+    o->beta = beta;
+    o->norm = norm;
+    o->bnorm = bnorm;
+    o->eps = eps;
+    o->pvd = pvd;
+    o->rz = rz;
+    o->vres = vres;
+    o->iter = iter;
+    o->active = act ? 1 : 0;
+    o->err = *(volatile int*)sm.abort_ ? kErrTimeout : err;
+    o->hist_len = iter + 1;
+    o->xpend = o->xprev = 0;
+    o->sigprev = 0.0;
+  }
+}
+
+// ---- sliced matrix copy -----------------------------------------------------------
+
+// longest row of each slice of 32 rows, and of the matrix
+__global__ void slice_width_kernel(int n, long nslices, const int* __restrict__ rp, int* __restrict__ width,
+                                   int* __restrict__ longest) {
+  const int lane = threadIdx.x & 31;
+  for (long s = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5; s < nslices;
+       s += ((long)gridDim.x * blockDim.x) >> 5) {
+    const long row = s * 32 + lane;
+    int len = row < n ? rp[row + 1] - rp[row] : 0;
+    for (int off = 16; off >= 1; off >>= 1) len = max(len, __shfl_xor_sync(0xffffffffu, len, off));
+    if (lane == 0) {
+      width[s] = min(len, kMaxWidth);
+      atomicMax(longest, len);
+    }
+  }
+}
+
+// base == nullptr: slices of kPatLen entries a row
+template <typename VT>
+__global__ void slice_fill_kernel(int n, const int* __restrict__ rp, const int* __restrict__ ci,
+                                  const VT* __restrict__ v, const int* __restrict__ base,
+                                  VT* __restrict__ sv, int* __restrict__ sc) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    const int b = rp[i], len = rp[i + 1] - b;
+    const size_t at = (base ? (size_t)base[i >> 5] : (size_t)(i >> 5) * kPatLen) * 32 + (i & 31);
+    for (int e = 0; e < len; ++e) {
+      sv[at + (size_t)e * 32] = v[b + e];
+      if (sc) sc[at + (size_t)e * 32] = ci[b + e];
+    }
+  }
+}
+
+void sell_free(CsrDev& A) {
+  cudaFree(A.sell_v);
+  cudaFree(A.sell_v32);
+  cudaFree(A.sell_c);
+  cudaFree(A.sell_base);
+  A.sell_v = nullptr;
+  A.sell_v32 = nullptr;
+  A.sell_c = A.sell_base = nullptr;
+  A.sell_total = -1;
+}
+
+static double*& sell_vals(CsrDev& A, const double*) { return A.sell_v; }
+static float*& sell_vals(CsrDev& A, const float*) { return A.sell_v32; }
+
+// Builds the sliced copy once; *ok = false when its padding is not worth it
+// (more than twice the entries plus one slice row per slice: a few very long
+// rows among short ones), which leaves the matrix to the graph of sweeps.
+template <typename VT>
+static int ensure_sell(celg_handle* h, CsrDev& A, const VT* vals, bool* ok) {
+  *ok = false;
+  const bool pat = A.pid != nullptr;
+  const long nslices = ntiles_of(A.n) * (kTile / 32);
+  if (A.sell_total < 0) {
+    if (pat) {
+      A.sell_total = nslices * kPatLen * 32;
+    } else {
+      int *width = nullptr, *base = nullptr;
+      void* tmp = nullptr;
+      size_t tmp_bytes = 0;
+      cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, width, base, (int)nslices + 1, h->stream);
+      cudaError_t e = cudaMalloc(&width, sizeof(int) * (nslices + 1));
+      if (e == cudaSuccess) e = cudaMalloc(&base, sizeof(int) * (nslices + 1));
+      if (e == cudaSuccess) e = cudaMalloc(&tmp, std::max<size_t>(tmp_bytes, 16));
+      if (e == cudaSuccess) e = cudaMemsetAsync(width + nslices, 0, sizeof(int), h->stream);
+      int total = 0, longest = 0;
+      int* longest_d = h->err_d + 5;
+      if (e == cudaSuccess) e = cudaMemsetAsync(longest_d, 0, sizeof(int), h->stream);
+      if (e == cudaSuccess) {
+        slice_width_kernel<<<(int)std::min(nslices / 8 + 1, 2048L), 256, 0, h->stream>>>(A.n, nslices, A.rp, width,
+                                                                                        longest_d);
+        e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, width, base, (int)nslices + 1, h->stream);
+      }
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(&total, base + nslices, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(&longest, longest_d, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+      cudaFree(width);
+      cudaFree(tmp);
+      if (e != cudaSuccess || longest > kMaxWidth || 32L * total > 2L * A.nnz + 32 * nslices) {
+        cudaFree(base);
+        A.sell_total = 0;
+        return e != cudaSuccess ? cuda_status(e, "sliced matrix") : CELG_OK;
+      }
+      A.sell_base = base;
+      A.sell_total = 32L * total;
+    }
+  }
+  if (A.sell_total == 0) return CELG_OK;
+  VT*& sv = sell_vals(A, vals);
+  const bool need_c = !pat && !A.sell_c;
+  if (!sv) {
+    cudaError_t e = cudaMalloc(&sv, sizeof(VT) * (size_t)A.sell_total);
+    if (e == cudaSuccess && need_c) e = cudaMalloc(&A.sell_c, sizeof(int) * (size_t)A.sell_total);
+    if (e == cudaSuccess) {
+      slice_fill_kernel<VT><<<(int)std::min(((long)A.n + 255) / 256, (long)h->sms * 8), 256, 0, h->stream>>>(
+          A.n, A.rp, A.ci, vals, pat ? nullptr : A.sell_base, sv, need_c ? A.sell_c : nullptr);
+      e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) {
+      sell_free(A);
+      return cuda_status(e, "sliced matrix");
+    }
+  }
+  *ok = true;
+  return CELG_OK;
+}
+
+// Most rows a system may have for the one-kernel solve (CELG_ONCHIP_ROWS
+// overrides: 0 sends every solve through the graph of sweeps).
+static long onchip_max_rows() {
+  const char* e = std::getenv("CELG_ONCHIP_ROWS");
+  return e ? std::atol(e) : 1L << 30;
+}
+
+// *done stays false when the device cannot hold the grid at once (fewer SMs
+// at this process's disposal than the device has).
+template <typename VT, bool PAT>
+static int launch_onchip(celg_handle* h, const OcArgs<VT>& a, int grid, size_t smem, bool* done) {
+  if (const int st = allow_dynamic_smem<pcg_onchip_kernel<VT, PAT>>((int)smem)) return st;
+  OcArgs<VT> arg = a;
+  void* params[] = {&arg};
+  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)pcg_onchip_kernel<VT, PAT>, dim3(grid),
+                                                    dim3(kOcThreads), params, smem, h->stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    (void)cudaGetLastError();
+    return CELG_OK;
+  }
+  CELG_CUDA(e);
+  *done = true;
+  return CELG_OK;
+}
+
+template <typename VT>
+int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_params* p, int hist_cap, bool* done) {
+  *done = false;
+  const long n = A.n;
+  if (n < 1 || n > onchip_max_rows()) return CELG_OK;
+  const long nt = ntiles_of(n), nunits = nt * 8;
+  if (nunits > kOcMaxUnits) return CELG_OK;
+  const int slots = (int)((nunits + h->sms - 1) / h->sms);
+  const int grid = (int)((nunits + slots - 1) / slots);
+  const bool pat = A.pid != nullptr;
+  const int pat_ints = pat ? A.npat * kPatLen : 0;
+  const size_t base = OcSmem<VT>(nullptr, (int)nt, pat_ints, slots, 0).bytes;
+  if (base > (size_t)kOcMaxSmem) return CELG_OK;
+  const size_t per_cached = sizeof(VT) * kUnitRows * kPatLen;
+  const int ncache = pat ? (int)std::min<size_t>((size_t)slots, (kOcMaxSmem - base) / per_cached) : 0;
+  const size_t smem = OcSmem<VT>(nullptr, (int)nt, pat_ints, slots, ncache).bytes;
+  bool ok = false;
+  int st = ensure_sell<VT>(h, A, B.vals, &ok);
+  if (st || !ok) return st;
+  const size_t nslot = (size_t)kSlotSets * nunits;
+  if (nslot > h->oc_cap) {
+    CELG_CUDA(cudaStreamSynchronize(h->stream));
+    cudaFree(h->oc_slots);
+    h->oc_slots = nullptr;
+    h->oc_cap = 0;
+    CELG_CUDA(cudaMalloc(&h->oc_slots, sizeof(double) * (nslot + kOcTail)));
+    h->oc_cap = nslot;
+  }
+  OcArgs<VT> a;
+  a.n = (int)n;
+  a.ntiles = (int)nt;
+  a.slots = slots;
+  a.ncache = ncache;
+  a.sv = sell_vals(A, B.vals);
+  a.sc = A.sell_c;
+  a.sbase = A.sell_base;
+  a.rp = A.rp;
+  a.pid = A.pid;
+  a.pat = A.pat;
+  a.pat_ints = pat_ints;
+  a.b = B.b;
+  a.x = B.x;
+  a.J = B.J;
+  a.p = B.p;
+  a.slot = h->oc_slots;
+  a.total = h->oc_slots + (nslot + (nslot & 1));
+  a.arrive = reinterpret_cast<unsigned*>(a.total + kSlotSets + 7);
+  a.out = h->state_h;
+  a.hist = h->hist_d;
+  a.hist_cap = hist_cap;
+  a.iter_max = p->iter_max;
+  a.x0_mode = p->x0_mode;
+  a.verify = B.verify_vals != nullptr;
+  a.eps_abs = p->eps_abs;
+  a.eps_rel = p->eps_rel;
+  CELG_CUDA(cudaMemsetAsync(h->oc_slots, 0xff, sizeof(double) * (nslot + kOcTail), h->stream));
+  return pat ? launch_onchip<VT, true>(h, a, grid, smem, done) : launch_onchip<VT, false>(h, a, grid, smem, done);
+}
+
+template int pcg_onchip<double>(celg_handle*, CsrDev&, const PcgBind<double>&, const celg_params*, int, bool*);
+template int pcg_onchip<float>(celg_handle*, CsrDev&, const PcgBind<float>&, const celg_params*, int, bool*);
+
+}  // namespace celg

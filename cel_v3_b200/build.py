@@ -24,7 +24,7 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompiler", "-fPIC,-
          "-I", INCLUDE, "--expt-relaxed-constexpr"]
 SOURCES = ["api.cu", "spmv.cu", "blas1.cu", "pcg.cu", "pcg_onchip.cu", "krylov.cu", "ir.cu", "ru.cu", "elm.cu", "noalloc.cu",
            "batched.cu", "selftest.cu", "multirhs.cu", "adjoint.cu", "dist.cu", "dist_solve.cu", "assemble.cu",
-           "blockjacobi.cu"]
+           "blockjacobi.cu", "row_forms.cu"]
 
 
 def _newer(target, deps):

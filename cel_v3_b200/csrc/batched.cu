@@ -810,8 +810,7 @@ void batch_free(Batch* b) {
   cudaFree(b->A.ci);
   cudaFree(b->A.v);
   cudaFree(b->A.ci8);
-  cudaFree(b->A.pid);
-  cudaFree(b->A.pat);
+  row_forms_free(b->A);
   cudaFree(b->A.dict);
   cudaFree(b->J);
   cudaFree(b->B);
@@ -922,7 +921,13 @@ static int batch_build(celg_handle* h, int count, celg_mat* const* mats, const s
   // 1-byte column offsets when the systems together use at most 256
   // distinct offsets col - row (7-point systems: -1, 0, 1 and +-side,
   // +-side^2 per distinct side): 9 instead of 12 bytes per non-zero
-  if (!st) st = build_offset_dict_csr(h, A);
+  // (row patterns, when there are so few systems that theirs fit the table)
+  if (!st) st = row_forms_search(h, A, false, nullptr);
+  if (!st) {
+    const cudaError_t e2 = cudaStreamSynchronize(h->stream);
+    st = e2 == cudaSuccess ? row_forms_build(h, A, false) : cuda_status(e2, "batch row forms");
+  }
+  if (!st && !A.pid) st = build_offset_dict_csr(h, A);
   if (st) {
     batch_free(bt);
     return st;

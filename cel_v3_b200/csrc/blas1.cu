@@ -142,7 +142,7 @@ int launch_jacobi_setup(celg_handle* h, celg_mat* m) {
                                                              m->scaled ? m->scale : nullptr,
                                                              m->diag, m->jacobi);
   CELG_CUDA(cudaGetLastError());
-  return CELG_OK;
+  return row_forms_jacobi(h, m->csr, m->jacobi);
 }
 
 int launch_row_scale(celg_handle* h, celg_mat* m) {

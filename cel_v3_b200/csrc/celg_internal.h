@@ -15,6 +15,17 @@ namespace celg {
 // Device copy of a CSR matrix, 0-based.  row_ptr has n+1+4 entries and
 // cols/vals nnz+4 (tails filled with nnz / 0) so that the 16-byte rounded
 // bulk copies of the SpMV pipeline never leave the allocation.
+// Runs of x that a tile needs for the column offsets of a row table
+// (csr_win_kernel).
+constexpr int kWinSegs = 8;
+struct WinPlan {
+  int nseg = 0;          // 0: no plan (too many runs or too much to stage)
+  int total = 0;         // staged elements of a tile
+  int start[kWinSegs];   // first offset of the run from the tile's first row, a multiple of 4
+  int len[kWinSegs];     // elements, a multiple of 4
+  int base[kWinSegs];    // position in the stage
+};
+
 struct CsrDev {
   int n = 0;
   int nnz = 0;
@@ -32,12 +43,24 @@ struct CsrDev {
   int* dict = nullptr;    // ndict offsets, ascending
   int ndict = 0;
   int cap_dict = 0;       // staging capacity with 16-entry alignment
-  // row patterns (spmv_kernels.cuh, kPatLen/kPatMax): one pattern index per
-  // row (n + 16 bytes) and the pattern table (npat x 8 column offsets), when
-  // the dictionary's rows fit them
+  // row patterns (row_forms.cu): one pattern index per row (n + 16 bytes)
+  // and the pattern table (npat x 8 column offsets; the arrays after pat are
+  // parts of its allocation)
   uint8_t* pid = nullptr;
   int* pat = nullptr;
   int npat = 0;
+  int* plen = nullptr;       // entries of each pattern
+  int* prep = nullptr;       // a row of each pattern
+  // row table: the values too are those of the pattern index (npat x 8)
+  double* rowv = nullptr;
+  float* rowv32 = nullptr;
+  WinPlan win;
+  // Jacobi value of each pattern index, when all its rows have the same
+  double* jtab = nullptr;
+  float* jtab32 = nullptr;
+  bool jtab_ok = false;
+  bool juni = false;         // one value for all rows
+  double jval = 0.0;
   // copy in slices of 32 rows for the one-kernel solve (pcg_onchip.cu)
   double* sell_v = nullptr;
   float* sell_v32 = nullptr;
@@ -78,6 +101,9 @@ struct celg_handle {
   int* err_d = nullptr;      // device error word (bounded waits)
   double* scal_d = nullptr;  // small device scalars for blas1 results
   double* scal_h = nullptr;  // pinned mirror
+  // row-form search (row_forms.cu): its sets on the device and a pinned copy
+  void* rows_d = nullptr;
+  void* rows_h = nullptr;
   // PCG work vectors
   double* wr = nullptr;
   double* wp = nullptr;
@@ -161,6 +187,8 @@ int launch_spmv_csr(celg_handle* h, const CsrDev& A, const double* x, double* y,
 int launch_spmv_csr_f32(celg_handle* h, const CsrDev& A, const float* x, float* y, int accumulate);
 int launch_spmv_jad(celg_handle* h, const CsrDev& A, const JadDev& J, const double* x, double* y);
 int csr_compute_cap(celg_handle* h, CsrDev& A);
+int csr_span_launch(celg_handle* h, const CsrDev& A, int* out);
+void csr_set_cap(CsrDev& A, int span);
 
 // blas1.cu
 int launch_dot(celg_handle* h, long n, const double* a, const double* b, double* out_d, int take_sqrt);
@@ -195,6 +223,12 @@ int ensure_offset_dict(celg_handle* h, celg_mat* m);
 int build_offset_dict_csr(celg_handle* h, CsrDev& A);
 // pcg_onchip.cu: drop the sliced copy (the values changed, or the matrix goes)
 void sell_free(CsrDev& A);
+// row_forms.cu
+size_t row_sets_bytes();
+int row_forms_search(celg_handle* h, const CsrDev& A, bool with_values, const int* bad);
+int row_forms_build(celg_handle* h, CsrDev& A, bool with_values);
+int row_forms_jacobi(celg_handle* h, CsrDev& A, const double* J);
+void row_forms_free(CsrDev& A);
 int alloc_csr(celg_mat* m, int n, int nnz, int ncols);
 int finish_csr(celg_handle* h, celg_mat* m, int base);
 void free_mat_arrays(celg_mat* m);

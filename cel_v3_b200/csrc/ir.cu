@@ -118,6 +118,9 @@ int ir_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const celg
   B.q = q32;
   B.v = v32;
   B.J = m->jacobi32;
+  if (m->csr.jtab_ok) B.jtab = m->csr.jtab32;
+  B.juni = m->csr.juni;
+  B.jval = (float)m->csr.jval;
 
   cudaEvent_t e0, e1;
   CELG_CUDA(cudaEventCreate(&e0));

@@ -92,21 +92,6 @@ void graph_cache_drop_matrix(celg_handle* h, const void* m) {
   }
 }
 
-// A CSR sweep of the solve: FP64 with the 1-byte column offsets when the
-// matrix has them (same values in the same order, so the same sums), else
-// with the int32 columns.
-template <typename VT, class Epi>
-static int csr_sweep(celg_handle* h, const PcgBind<VT>& B, const VT* vals, const VT* x, const Epi& epi) {
-  if constexpr (std::is_same<VT, double>::value) {
-    if (B.dict) {
-      bool done = false;
-      const int st = launch_csr_compact<double>(h, *B.A, vals, x, epi, nullptr, 0, &done);
-      if (done) return st;
-    }
-  }
-  return launch_csr<VT>(h, *B.A, vals, x, epi);
-}
-
 template <typename VT>
 static int pcg_setup(celg_handle* h, const PcgBind<VT>& B, const celg_params* p, PcgArgs a) {
   const long n = B.A->n;
@@ -121,7 +106,20 @@ static int pcg_setup(celg_handle* h, const PcgBind<VT>& B, const celg_params* p,
     }
     if (B.bj) return bj_pcg_setup_tail(h, B, a);
   }
-  return csr_sweep<VT>(h, B, B.vals, B.x, EpiInit<VT>{B.b, B.r, B.p, B.J, a});
+  return launch_csr<VT>(h, *B.A, B.vals, B.x, EpiInit<VT>{B.b, B.r, B.p, B.J, a});
+}
+
+// K2 and K3 of an iteration, J read from its array (K2 32 n bytes, K3 56 n
+// and 32 n), through the row table's index (7 n less) or, one value for all
+// rows, not at all (8 n less: 242 against 267 us an
+// iteration at 256^3).
+template <typename VT, class JS>
+static int pcg_vectors(celg_handle* h, const PcgBind<VT>& B, PcgArgs a, int phase, JS J) {
+  const long n = B.A->n;
+  if (const int st = launch_tile(h, n, OpUpdate<VT, JS>{B.r, B.v, J, a, 0.0})) return st;
+  if (phase == 1) return launch_tile(h, n, OpDirectionDefer<VT, JS>{B.p, B.q, B.r, J, B.x, a});
+  if (phase == 2) return launch_tile(h, n, OpDirectionPair<VT, JS>{B.p, B.q, B.r, J, B.x, a});
+  return launch_tile(h, n, OpDirectionX<VT, JS>{B.p, B.r, J, B.x, a});
 }
 
 // phase 0: one iteration, K3 = OpDirectionX.  Phases 1 and 2: the even and
@@ -129,16 +127,15 @@ static int pcg_setup(celg_handle* h, const PcgBind<VT>& B, const celg_params* p,
 // directions are B.p and B.q in turn.
 template <typename VT>
 static int pcg_body(celg_handle* h, const PcgBind<VT>& B, PcgArgs a, int phase = 0) {
-  const long n = B.A->n;
   VT* pc = phase == 2 ? B.q : B.p;
   int s2 = CELG_OK;
   if constexpr (std::is_same<VT, double>::value) {
     if (B.jad)
       s2 = launch_jad(h, *B.A, *B.jad, B.p, EpiAp<double>{B.v, B.p, a});
     else
-      s2 = csr_sweep<VT>(h, B, B.vals, pc, EpiAp<VT>{B.v, pc, a});
+      s2 = launch_csr<VT>(h, *B.A, B.vals, pc, EpiAp<VT>{B.v, pc, a});
   } else {
-    s2 = csr_sweep<VT>(h, B, B.vals, pc, EpiAp<VT>{B.v, pc, a});
+    s2 = launch_csr<VT>(h, *B.A, B.vals, pc, EpiAp<VT>{B.v, pc, a});
   }
   if constexpr (std::is_same<VT, double>::value) {
     if (B.bj) {
@@ -147,11 +144,10 @@ static int pcg_body(celg_handle* h, const PcgBind<VT>& B, PcgArgs a, int phase =
       return s2;
     }
   }
-  if (!s2) s2 = launch_tile(h, n, OpUpdate<VT>{B.r, B.v, B.J, a, 0.0});
   if (s2) return s2;
-  if (phase == 1) return launch_tile(h, n, OpDirectionDefer<VT>{B.p, B.q, B.r, B.J, B.x, a});
-  if (phase == 2) return launch_tile(h, n, OpDirectionPair<VT>{B.p, B.q, B.r, B.J, B.x, a});
-  return launch_tile(h, n, OpDirectionX<VT>{B.p, B.r, B.J, B.x, a});
+  if (B.juni) return pcg_vectors<VT>(h, B, a, phase, JUni<VT>{B.jval});
+  if (B.jtab) return pcg_vectors<VT>(h, B, a, phase, JTab<VT>{B.jtab, B.A->pid});
+  return pcg_vectors<VT>(h, B, a, phase, JArr<VT>{B.J});
 }
 
 // Two iterations: a pair when B.q is set, else the one-iteration body twice.
@@ -173,7 +169,7 @@ static int pcg_tail(celg_handle* h, const PcgBind<VT>& B, PcgArgs a) {
       if (!st) st = launch_tile(h, n, OpVerifyNat{B.b, B.v, a.st});
       return st;
     }
-    return csr_sweep<double>(h, B, B.verify_vals, B.x, EpiVerify{B.b, a.st});
+    return launch_csr<double>(h, *B.A, B.verify_vals, B.x, EpiVerify{B.b, a.st});
   }
   return CELG_OK;
 }
@@ -212,12 +208,12 @@ template <typename VT>
 static std::string pcg_key(const PcgBind<VT>& B, const celg_params* p, int hist_cap,
                            const void* mat) {
   char buf[640];
-  std::snprintf(buf, sizeof(buf), "pcg%d|%p|%d|%d|%p|%p|%p|%p|%p|%p|%p|%d|%.17g|%.17g|%d|%d|%p|%p|%p|%d|%p|%d",
+  std::snprintf(buf, sizeof(buf), "pcg%d|%p|%d|%d|%p|%p|%p|%p|%p|%p|%p|%d|%.17g|%.17g|%d|%d|%p|%p|%p|%d|%p|%d|%p",
                 (int)sizeof(VT), mat, B.A->n, B.jad ? 1 : 0, (const void*)B.b, (const void*)B.x,
                 (const void*)B.r, (const void*)B.p, (const void*)B.q, (const void*)B.v, (const void*)B.J,
                 p->x0_mode, p->eps_abs, p->eps_rel, p->iter_max, hist_cap,
                 (const void*)B.vals, (const void*)B.verify_vals, (const void*)B.bj, B.bs,
-                (const void*)B.z, B.dict ? 1 : 0);
+                (const void*)B.z, B.dict ? 1 : 0, (const void*)B.jtab);
   return std::string(buf);
 }
 
@@ -313,7 +309,10 @@ int pcg_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const cel
   if (!jad) {
     st = ensure_offset_dict(h, m);
     if (st) return st;
-    B.dict = m->csr.ci8 != nullptr;
+    B.dict = m->csr.pid || m->csr.ci8;
+    if (m->csr.jtab_ok) B.jtab = m->csr.jtab;
+    B.juni = m->csr.juni;
+    B.jval = m->csr.jval;
   }
   if (p->precond == CELG_PRECOND_BLOCK_JACOBI) {
     if (jad) return CELG_ERR_ARG;
@@ -338,12 +337,16 @@ int pcg_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const cel
   std::memset(&s, 0, sizeof(s));
   const int ret = pcg_run<double>(h, B, p, m, &s);
   h->last_iters = s.iter;
-  // K1 reads 8 bytes per non-zero and one per row with the row patterns, 9 per
-  // non-zero with the 1-byte offsets, else 12; the paired K3 reads and stores
-  // x once per two iterations (92 instead of 96 bytes per row)
-  h->last_bytes_per_iter =
-      (B.dict && m->csr.pid ? 8.0 * m->csr.nnz + 1.0 * n : (B.dict ? 9.0 : 12.0) * m->csr.nnz) +
-      4.0 * (n + 1) + (B.q ? 92.0 : 96.0) * n;
+  // K1 reads one byte per row with the row table; 8 bytes per non-zero and
+  // one per row with the row patterns, 9 per non-zero with the 1-byte offsets,
+  // else 12, and the row pointer; the paired K3 reads and stores x once per
+  // two iterations (92 instead of 96 bytes per row), and with the Jacobi table
+  // K2 and K3 read a byte instead of J (14 less)
+  const double mat_bytes =
+      (jad || !m->csr.rowv ? (m->csr.pid ? 8.0 * m->csr.nnz + 1.0 * n : (B.dict ? 9.0 : 12.0) * m->csr.nnz) +
+                                 4.0 * (n + 1)
+                           : 1.0 * n);
+  h->last_bytes_per_iter = mat_bytes + ((B.q ? 92.0 : 96.0) - (B.juni ? 16.0 : B.jtab ? 14.0 : 0.0)) * n;
   if (res) {
     res->iter_done = s.iter;
     res->final_norm2 = s.norm;

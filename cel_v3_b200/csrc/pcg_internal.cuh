@@ -45,9 +45,37 @@ struct PcgBind {
   const double* bj = nullptr;
   int bs = 0;
   double* z = nullptr;
-  // FP64 CSR sweeps read the 1-byte column offsets (A->ci8) instead of the
-  // int32 columns: 9 instead of 12 bytes per non-zero
+  // the CSR sweeps read row patterns or 1-byte column offsets instead of the
+  // int32 columns
   bool dict = false;
+  // Jacobi value of each row-table index (null: K2 and K3 read J), and of
+  // all rows when juni
+  const VT* jtab = nullptr;
+  bool juni = false;
+  VT jval = VT(0);
+};
+
+// J(i) from its array, or through the row's index in the row table
+template <typename VT>
+struct JArr {
+  const VT* J;
+  __device__ VT operator()(long i) const { return __ldg(J + i); }
+  __device__ VT stream(long i) const { return __ldcs(J + i); }
+};
+template <typename VT>
+struct JTab {
+  const VT* tab;
+  const uint8_t* pid;
+  __device__ VT operator()(long i) const { return __ldg(tab + __ldg(pid + i)); }
+  __device__ VT stream(long i) const { return __ldg(tab + __ldg(pid + i)); }
+};
+
+// J the same for all rows
+template <typename VT>
+struct JUni {
+  VT J;
+  __device__ VT operator()(long) const { return J; }
+  __device__ VT stream(long) const { return J; }
 };
 
 // blockjacobi.cu: the block-Jacobi forms of the set-up and of K2/K3
@@ -181,10 +209,13 @@ struct EpiAp {
   __device__ bool active() const { return *(volatile int*)&a.st->active != 0; }
   // p(i) is loaded after the row's gathers: issued before them it cost 23 us
   // per 256^3 sweep (290 -> 267 us)
-  __device__ void row(long i, VT s, double* acc) const {
+  __device__ void row(long i, VT s, double* acc) const { row_x(i, s, __ldg(p + i), acc); }
+  // p is the sweep's x: taken from the staged window where there is one
+  static constexpr bool kTakesX = true;
+  __device__ void row_x(long i, VT s, VT pi, double* acc) const {
     const VT vi = vadd(VT(0), s);
     v[i] = vi;
-    acc[0] = dacc_prod(acc[0], vi, __ldg(p + i));
+    acc[0] = dacc_prod(acc[0], vi, pi);
   }
   __device__ void finish(double* tot) const {
     PcgState* st = a.st;
@@ -202,14 +233,14 @@ struct EpiAp {
 // iteration's x += sigma p (:263-265) is left to K3, which reads the old p
 // anyway, so this sweep reads neither x nor p; K2 marks it pending.  Each x
 // element gets the same operation in the same iteration as before.
-template <typename VT>
+template <typename VT, class JS = JArr<VT>>
 struct OpUpdate {
   static constexpr int NRED = 2;
   static constexpr int kTilesPerPass = sizeof(VT) == 4 ? 2 : 1;
   struct Regs { VT r, v, J; };
   VT* r;
   const VT* v;
-  const VT* J;
+  JS J;
   PcgArgs a;
   double sg;
   __device__ bool prepare() {
@@ -225,7 +256,7 @@ struct OpUpdate {
   __device__ void load(long i, Regs& g) const {
     g.r = r[i];
     g.v = __ldcs(v + i);
-    g.J = __ldg(J + i);
+    g.J = J(i);
   }
   __device__ void compute(long i, Regs& g, double* acc) const {
     const VT ri = R<VT>(dadd(D(g.r), dmul(-sg, D(g.v))));
@@ -252,7 +283,7 @@ struct OpUpdate {
 // K3 of the PCG: x += sigma p when K2 left it pending (also after K2 ended
 // the solve), then p = beta p + J r (:282) while the solve goes on.  The
 // last CTA clears the pending mark.
-template <typename VT>
+template <typename VT, class JS = JArr<VT>>
 struct OpDirectionX {
   static constexpr int NRED = 0;
   static constexpr int kTilesPerPass = sizeof(VT) == 4 ? 2 : 1;
@@ -260,7 +291,7 @@ struct OpDirectionX {
   struct Regs { VT p, r, J, x; };
   VT* p;
   const VT* r;
-  const VT* J;
+  JS J;
   VT* x;
   PcgArgs a;
   double bt = 0.0, sg = 0.0;
@@ -279,7 +310,7 @@ struct OpDirectionX {
     g.p = p[i];
     if (act) {
       g.r = __ldcs(r + i);
-      g.J = __ldcs(J + i);
+      g.J = J.stream(i);
     }
     if (xp) g.x = __ldcs(x + i);
   }
@@ -299,7 +330,7 @@ struct OpDirectionX {
 // and each element gets the same operations in the same order as with
 // OpDirectionX.  When K2 ended the solve in the even iteration, the even
 // sweep applies its own update at once.
-template <typename VT>
+template <typename VT, class JS = JArr<VT>>
 struct OpDirectionDefer {
   static constexpr int NRED = 0;
   static constexpr int kTilesPerPass = sizeof(VT) == 4 ? 2 : 1;
@@ -308,7 +339,7 @@ struct OpDirectionDefer {
   const VT* p;
   VT* q;
   const VT* r;
-  const VT* J;
+  JS J;
   VT* x;
   PcgArgs a;
   double bt = 0.0, sg = 0.0;
@@ -327,7 +358,7 @@ struct OpDirectionDefer {
     g.p = __ldcs(p + i);
     if (act) {
       g.r = __ldcs(r + i);
-      g.J = __ldcs(J + i);
+      g.J = J.stream(i);
     } else if (xp) {
       g.x = __ldcs(x + i);
     }
@@ -345,7 +376,7 @@ struct OpDirectionDefer {
   }
 };
 
-template <typename VT>
+template <typename VT, class JS = JArr<VT>>
 struct OpDirectionPair {
   static constexpr int NRED = 0;
   static constexpr int kTilesPerPass = sizeof(VT) == 4 ? 2 : 1;
@@ -354,7 +385,7 @@ struct OpDirectionPair {
   VT* p;
   const VT* q;
   const VT* r;
-  const VT* J;
+  JS J;
   VT* x;
   PcgArgs a;
   double bt = 0.0, sg = 0.0, sp = 0.0;
@@ -374,7 +405,7 @@ struct OpDirectionPair {
     if (xp || act) g.q = q[i];
     if (act) {
       g.r = __ldcs(r + i);
-      g.J = __ldcs(J + i);
+      g.J = J.stream(i);
     }
     if (xq || xp) g.x = __ldcs(x + i);
   }

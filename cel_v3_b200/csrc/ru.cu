@@ -144,13 +144,14 @@ struct EpiRuResidual {
 // operation rounded once); its dot products stay FP64 on exact products.
 // Done in FP64 and rounded back, the update took three more conversions per
 // element, and the sweep was bound by the conversion rate, not by memory.
+template <class JS>
 struct OpRuStep {
   static constexpr int NRED = 2;
   static constexpr int kTilesPerPass = 2;
   struct Regs { float r, v, J; };
   float* r;
   const float* v;
-  const float* J;
+  JS J;
   RuArgs a;
   float nsg;
   __device__ bool prepare() {
@@ -164,7 +165,7 @@ struct OpRuStep {
   __device__ void load(long i, Regs& g) const {
     g.r = r[i];
     g.v = __ldcs(v + i);
-    g.J = __ldg(J + i);
+    g.J = J(i);
   }
   __device__ void compute(long i, Regs& g, double* acc) const {
     const float ri = fadd(g.r, fmul(nsg, g.v));
@@ -286,8 +287,9 @@ static int ru_setup(celg_handle* h, celg_mat* m, const double* b, double* x, con
 // the paired direction sweep of the PCG (OpDirectionDefer, OpDirectionPair)
 // with the correction d in place of x, so d is read and stored once per
 // pair.
+template <class JS>
 static int ru_body(celg_handle* h, celg_mat* m, const double* b, double* x, RuArgs a, float* r,
-                   float* pv, float* pq, float* v, float* d, bool odd, bool in_graph) {
+                   float* pv, float* pq, float* v, float* d, bool odd, bool in_graph, JS J) {
   const long n = m->csr.n;
   if (in_graph) {
     int st = capture_new_handle(h, 0, &a.cond_update);
@@ -296,7 +298,7 @@ static int ru_body(celg_handle* h, celg_mat* m, const double* b, double* x, RuAr
   PcgArgs pa = a.pcg();
   float* pc = odd ? pq : pv;
   int st = launch_csr<float>(h, m->csr, m->csr.v32, pc, EpiAp<float>{v, pc, pa});
-  if (!st) st = launch_tile(h, n, OpRuStep{r, v, m->jacobi32, a, 0.0f});
+  if (!st) st = launch_tile(h, n, OpRuStep<JS>{r, v, J, a, 0.0f});
   auto update = [&]() -> int {
     int s2 = launch_tile(h, n, OpRuFlush{x, d, pc, odd ? pv : nullptr, a, 0});
     if (!s2)
@@ -306,9 +308,8 @@ static int ru_body(celg_handle* h, celg_mat* m, const double* b, double* x, RuAr
   };
   if (!st) st = in_graph ? capture_if(h, a.cond_update, update) : update();
   if (st) return st;
-  const float* J = m->jacobi32;
-  if (odd) return launch_tile(h, n, OpDirectionPair<float>{pv, pq, r, J, d, pa});
-  return launch_tile(h, n, OpDirectionDefer<float>{pv, pq, r, J, d, pa});
+  if (odd) return launch_tile(h, n, OpDirectionPair<float, JS>{pv, pq, r, J, d, pa});
+  return launch_tile(h, n, OpDirectionDefer<float, JS>{pv, pq, r, J, d, pa});
 }
 
 static int ru_tail(celg_handle* h, celg_mat* m, const double* b, double* x, RuArgs a, float* d) {
@@ -343,6 +344,13 @@ int ru_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const celg
   float* pq = d + cap;
   CELG_CUDA(cudaMemsetAsync(h->err_d, 0, sizeof(int), h->stream));
 
+  auto body = [&](RuArgs a, bool odd, bool in_graph) -> int {
+    if (m->csr.juni)
+      return ru_body(h, m, b, x, a, r, pv, pq, v, d, odd, in_graph, JUni<float>{(float)m->csr.jval});
+    if (m->csr.jtab_ok)
+      return ru_body(h, m, b, x, a, r, pv, pq, v, d, odd, in_graph, JTab<float>{m->csr.jtab32, m->csr.pid});
+    return ru_body(h, m, b, x, a, r, pv, pq, v, d, odd, in_graph, JArr<float>{m->jacobi32});
+  };
   char kb[512];
   std::snprintf(kb, sizeof(kb), "ru|%p|%d|%p|%p|%p|%d|%.17g|%.17g|%.17g|%d", (const void*)m,
                 m->csr.n, (const void*)b, (const void*)x, (const void*)r, p->x0_mode, p->eps_abs,
@@ -354,7 +362,7 @@ int ru_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const celg
     st = ru_setup(h, m, b, x, p, a0, r, pv, d);
     for (int it = 0; !st && it < p->iter_max; it += 8) {
       for (int k = 0; k < 8 && !st; ++k)
-        st = ru_body(h, m, b, x, a0, r, pv, pq, v, d, (k & 1) != 0, false);
+        st = body(a0, (k & 1) != 0, false);
       if (st) break;
       CELG_CUDA(cudaMemcpyAsync(sh, sd, sizeof(RuState), cudaMemcpyDeviceToHost, h->stream));
       CELG_CUDA(cudaStreamSynchronize(h->stream));
@@ -371,8 +379,8 @@ int ru_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const celg
         int s2 = ru_setup(h, m, b, x, p, a, r, pv, d);
         if (!s2)
           s2 = capture_while(h, cond, [&]() -> int {
-            int s3 = ru_body(h, m, b, x, a, r, pv, pq, v, d, false, true);
-            if (!s3) s3 = ru_body(h, m, b, x, a, r, pv, pq, v, d, true, true);
+            int s3 = body(a, false, true);
+            if (!s3) s3 = body(a, true, true);
             return s3;
           });
         if (!s2) s2 = ru_tail(h, m, b, x, a, d);
@@ -400,7 +408,7 @@ int ru_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const celg
   // 16 n), K3 (p, r, J read, p stored, d read and stored once per pair of
   // iterations: 20 n on average); 5 bytes per non-zero with the 1-byte
   // column offsets, else 8
-  h->last_bytes_per_iter = (m->csr.ci8 ? 5.0 : 8.0) * m->csr.nnz + 4.0 * (n + 1) + 44.0 * n;
+  h->last_bytes_per_iter = (m->csr.pid ? 4.0 : m->csr.ci8 ? 5.0 : 8.0) * m->csr.nnz + 4.0 * (n + 1) + 44.0 * n;
   if (res) {
     res->iter_done = s.s.iter;
     res->final_norm2 = s.norm64;

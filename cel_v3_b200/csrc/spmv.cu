@@ -31,21 +31,21 @@ __global__ void subtile_span_kernel(const int* __restrict__ rp, int n, int* out)
   if ((threadIdx.x & 31) == 0) atomicMax(out, best);
 }
 
-// Staging capacity: the largest sub-tile span if four stages of it fit two
-// CTAs per SM (113 KB each), otherwise as much as four stages in one CTA
-// allow; sub-tiles above the capacity are read from global memory instead.
-int csr_compute_cap(celg_handle* h, CsrDev& A) {
-  int* d = h->err_d + 1;  // scratch int next to the error word
-  CELG_CUDA(cudaMemsetAsync(d, 0, sizeof(int), h->stream));
+int csr_span_launch(celg_handle* h, const CsrDev& A, int* out) {
+  CELG_CUDA(cudaMemsetAsync(out, 0, sizeof(int), h->stream));
   if (A.n > 0) {
     const long nsub = ((long)A.n + kSub - 1) / kSub;
     const int grid = (int)std::max(1L, std::min((long)h->sms * 4, (nsub + 255) / 256));
-    subtile_span_kernel<<<grid, 256, 0, h->stream>>>(A.rp, A.n, d);
+    subtile_span_kernel<<<grid, 256, 0, h->stream>>>(A.rp, A.n, out);
     CELG_CUDA(cudaGetLastError());
   }
-  int span = 0;
-  CELG_CUDA(cudaMemcpyAsync(&span, d, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  CELG_CUDA(cudaStreamSynchronize(h->stream));
+  return CELG_OK;
+}
+
+// Staging capacity: the largest sub-tile span if four stages of it fit two
+// CTAs per SM (113 KB each), otherwise as much as four stages in one CTA
+// allow; sub-tiles above the capacity are read from global memory instead.
+void csr_set_cap(CsrDev& A, int span) {
   int cap = std::max(16, (span + 3) & ~3);
   const int two_cta = 113 * 1024, one_cta = 227 * 1024;
   if (csr_smem_bytes(cap, 8) > two_cta) {
@@ -54,6 +54,15 @@ int csr_compute_cap(celg_handle* h, CsrDev& A) {
     cap = std::max(16, lim & ~3);
   }
   A.cap = cap;
+}
+
+int csr_compute_cap(celg_handle* h, CsrDev& A) {
+  int* d = h->err_d + 1;  // scratch int next to the error word
+  if (const int st = csr_span_launch(h, A, d)) return st;
+  int span = 0;
+  CELG_CUDA(cudaMemcpyAsync(&span, d, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  CELG_CUDA(cudaStreamSynchronize(h->stream));
+  csr_set_cap(A, span);
   return CELG_OK;
 }
 

@@ -19,6 +19,7 @@
 // order; the result is written through perm (y(perm(i)) = tmp(i), :325).
 #pragma once
 #include "celg_device.cuh"
+#include "celg_internal.h"
 
 namespace celg {
 
@@ -428,6 +429,424 @@ __global__ void __launch_bounds__(kCsrThreads, sizeof(VT) == 4 ? 4 : (sizeof(CT)
   if constexpr (!kB && NR > 0) {
     double tot[NR > 0 ? NR : 1];
     if (red.finish && grid_finish<(NR > 0 ? NR : 1)>(red, tot, scratch, s_flag, j, 1)) ep.finish(tot);
+  }
+}
+
+// A lane's copy of the row-table entry it used last.  Neighbouring rows of a
+// grid mostly share an index, so the copy is refreshed only when some lane
+// of the warp meets another one: read for every row, the table's shared-
+// memory loads took as much of the L1 data pipe as the gathers.
+template <typename VT>
+struct RowEntry {
+  int id = -1, len = 0;
+  int off[kPatLen];
+  VT val[kPatLen];
+  __device__ __forceinline__ void take(int want, const int* s_off, const VT* s_val, const int* s_len) {
+    if (!__any_sync(0xffffffffu, want != id)) return;
+    if (want != id && want >= 0) {
+      len = s_len[want];
+      const int4* pq = reinterpret_cast<const int4*>(s_off + want * kPatLen);
+      const int4 q0 = pq[0], q1 = pq[1];
+      off[0] = q0.x; off[1] = q0.y; off[2] = q0.z; off[3] = q0.w;
+      off[4] = q1.x; off[5] = q1.y; off[6] = q1.z; off[7] = q1.w;
+      const VT* vs = s_val + want * kPatLen;
+      constexpr int kVec = 16 / (int)sizeof(VT);
+#pragma unroll
+      for (int u = 0; u < kPatLen; u += kVec) {
+        if constexpr (sizeof(VT) == 8) {
+          const double2 t = *reinterpret_cast<const double2*>(vs + u);
+          val[u] = t.x; val[u + 1] = t.y;
+        } else {
+          const float4 t = *reinterpret_cast<const float4*>(vs + u);
+          val[u] = t.x; val[u + 1] = t.y; val[u + 2] = t.z; val[u + 3] = t.w;
+        }
+      }
+      id = want;
+    }
+  }
+  // x of the row's entries (the padding of a short row reads x(row); the
+  // eighth entry is read for full rows only)
+  __device__ __forceinline__ void gather(const VT* xr, VT (&xv)[kPatLen]) const {
+#pragma unroll
+    for (int u = 0; u < kPatLen; ++u)
+      if (u < kPatLen - 1 || len == kPatLen) xv[u] = ldg_at(xr, off[u]);
+  }
+};
+
+constexpr int kTabRows = 2;  // rows of a lane in flight together
+
+// Row table sweep (row_forms.cu): the matrix is one byte per row, an index
+// into a table of whole rows in shared memory.  With so little to stream
+// there is nothing to stage: a lane takes its four rows of a tile in turn, the
+// gathers of one in flight at a time, the next tile's bytes loaded a tile
+// ahead.  What bounds it is the L1 data pipe (2.7 wavefronts a gather).
+// Tile sums as in tile_kernel (warp sums parked, one fold per kHeldTiles).
+template <typename VT, class Epi>
+__global__ void __launch_bounds__(kLanes, 3)
+    csr_tab_kernel(const uint8_t* __restrict__ pid, const int* __restrict__ pat, const int* __restrict__ plen,
+                   const VT* __restrict__ rowv, int npat, int n, const VT* __restrict__ x, Epi epi, RedCtx red) {
+  constexpr int NR = Epi::NRED;
+  constexpr int NR1 = NR > 0 ? NR : 1;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ double held[NR > 0 ? kHeldTiles : 1][NR1][8];
+  __shared__ long held_tile[NR > 0 ? kHeldTiles : 1];
+  __shared__ double scratch[8];
+  __shared__ int s_flag;
+  if (!epi.active()) return;
+  VT* s_val = reinterpret_cast<VT*>(smem);
+  int* s_off = reinterpret_cast<int*>(s_val + (size_t)npat * kPatLen);
+  int* s_len = s_off + npat * kPatLen;
+  const int j = threadIdx.x;
+  for (int q = j; q < npat * kPatLen; q += kLanes) {
+    s_val[q] = rowv[q];
+    s_off[q] = pat[q];
+  }
+  for (int q = j; q < npat; q += kLanes) s_len[q] = plen[q];
+  __syncthreads();
+  const long nvis = red.nvisit >= 0 ? red.nvisit : ((long)n + kTile - 1) / kTile;
+  [[maybe_unused]] int nheld = 0;
+  auto flush = [&]() {
+    __syncthreads();
+    for (int q = j; q < nheld * NR1; q += kLanes) {
+      const int sl = q / NR1, r = q % NR1;
+      double tot = held[sl][r][0];
+#pragma unroll
+      for (int w = 1; w < 8; ++w) tot = dadd(tot, held[sl][r][w]);
+      red.partials[(long)r * red.ntiles + held_tile[sl]] = tot;
+    }
+    __threadfence();
+    __syncthreads();
+    nheld = 0;
+  };
+  Epi ep = epi;
+  int id[4];
+  auto ids = [&](long t) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const long i = t * kTile + (long)q * kLanes + j;
+      id[q] = i < n ? (int)__ldcs(pid + i) : -1;
+    }
+  };
+  if (blockIdx.x < nvis) ids(tile_of(red, blockIdx.x, nvis));
+  RowEntry<VT> e;
+  for (long k = blockIdx.x; k < nvis; k += gridDim.x) {
+    const long t = tile_of(red, k, nvis);
+    int cur[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) cur[q] = id[q];
+    if (k + gridDim.x < nvis) ids(tile_of(red, k + gridDim.x, nvis));
+    double acc[NR1];
+#pragma unroll
+    for (int r = 0; r < NR1; ++r) acc[r] = 0.0;
+    const long row0 = t * kTile + j;
+#pragma unroll
+    for (int q = 0; q < 4; q += kTabRows) {
+      // the rows of a pass all have the entry at hand: their gathers together
+      bool same = true;
+#pragma unroll
+      for (int r = 0; r < kTabRows; ++r) same = same && cur[q + r] == cur[q];
+      if (__all_sync(0xffffffffu, same && cur[q] >= 0)) {
+        e.take(cur[q], s_off, s_val, s_len);
+        VT xv[kTabRows][kPatLen];
+#pragma unroll
+        for (int r = 0; r < kTabRows; ++r) e.gather(x + row0 + (long)(q + r) * kLanes, xv[r]);
+#pragma unroll
+        for (int r = 0; r < kTabRows; ++r)
+          ep.row(row0 + (long)(q + r) * kLanes, pat_dot_len<false>(e.len, e.val, xv[r]), acc);
+      } else {
+#pragma unroll 1
+        for (int r = 0; r < kTabRows; ++r) {
+          const int want = r == 0 ? cur[q] : r == 1 ? cur[q + 1] : r == 2 ? cur[(q + 2) & 3] : cur[(q + 3) & 3];
+          e.take(want, s_off, s_val, s_len);
+          if (want >= 0) {
+            const long row = row0 + (long)(q + r) * kLanes;
+            VT xv[kPatLen];
+            e.gather(x + row, xv);
+            ep.row(row, pat_dot_len<false>(e.len, e.val, xv), acc);
+          }
+        }
+      }
+    }
+    if constexpr (NR > 0) {
+      if (nheld + 1 > kHeldTiles) flush();
+#pragma unroll
+      for (int r = 0; r < NR1; ++r) {
+        const double w = warp_fold(acc[r]);
+        if ((j & 31) == 0) held[nheld][r][j >> 5] = w;
+      }
+      if (j == 0) held_tile[nheld] = t;
+      ++nheld;
+    }
+  }
+  if constexpr (NR > 0) {
+    flush();
+    double tot[NR1];
+    if (red.finish && grid_finish<NR1>(red, tot, scratch, &s_flag, j, 1)) ep.finish(tot);
+  }
+}
+
+// y = A x of a small patterned matrix: one row per thread, so that 32768 rows
+// are 128 CTAs and not 32 tiles, and as few dependent round trips as there
+// can be: the table comes to shared memory while the row's index byte (and
+// row pointer) is on its way, then the gathers and the values together.
+// TAB: values from the row table; else each warp brings the contiguous values
+// of its 32 rows to shared memory, whole lines at a time.
+template <typename VT, class Epi, bool TAB>
+__global__ void __launch_bounds__(kLanes)
+    csr_rows_kernel(const int* __restrict__ rp, const uint8_t* __restrict__ pid, const int* __restrict__ pat,
+                    const int* __restrict__ plen, const VT* __restrict__ vals, int npat, int n,
+                    const VT* __restrict__ x, Epi epi) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  if (!epi.active()) return;
+  constexpr int kStage = TAB ? 0 : kLanes * kPatLen;
+  VT* s_val = reinterpret_cast<VT*>(smem);  // TAB: npat x kPatLen; else kLanes x kPatLen
+  int* s_off = reinterpret_cast<int*>(s_val + (TAB ? npat * kPatLen : kStage));
+  int* s_len = s_off + npat * kPatLen;
+  const int j = threadIdx.x, lane = j & 31;
+  const int row = blockIdx.x * kLanes + j;
+  const bool in = row < n;
+  const int id = in ? (int)__ldg(pid + row) : 0;
+  [[maybe_unused]] int b = 0, len = 0;
+  if constexpr (!TAB) {
+    const int w0 = blockIdx.x * kLanes + (j & ~31);  // the warp's first row
+    b = __ldg(rp + min(row, n));
+    const int e = __ldg(rp + min(row + 1, n));
+    len = e - b;
+    const int base = __shfl_sync(0xffffffffu, b, 0), end = __shfl_sync(0xffffffffu, e, 31);
+    VT* mine = s_val + (j & ~31) * kPatLen;
+    if (w0 < n) {
+#pragma unroll
+      for (int u = 0; u < kPatLen; ++u) {
+        const int k = base + u * 32 + lane;
+        if (k < end) mine[k - base] = __ldg(vals + k);
+      }
+    }
+    b -= base;
+  }
+  for (int q = j; q < npat * kPatLen; q += kLanes) {
+    s_off[q] = __ldg(pat + q);
+    if (TAB) s_val[q] = __ldg(vals + q);
+  }
+  if (TAB)
+    for (int q = j; q < npat; q += kLanes) s_len[q] = __ldg(plen + q);
+  __syncthreads();
+  if (!in) return;
+  const int4* pq = reinterpret_cast<const int4*>(s_off + id * kPatLen);
+  const int4 q0 = pq[0], q1 = pq[1];
+  const int po[kPatLen] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+  VT xv[kPatLen];
+#pragma unroll
+  for (int u = 0; u < kPatLen; ++u) xv[u] = ldg_at(x + row, po[u]);
+  if constexpr (TAB) len = s_len[id];
+  const VT* vs = TAB ? s_val + id * kPatLen : s_val + (j & ~31) * kPatLen + b;
+  epi.row(row, pat_dot_len<false>(len, vs, xv), nullptr);
+}
+
+// Row table sweep with x staged in shared memory.  The column offsets of the
+// table fall into a few clusters (a 3-D grid: the planes below and above, and
+// the row's own plane), so the x a 1024-row tile needs is a few contiguous
+// runs: a producer warp brings them, and the tile's index bytes, in by bulk
+// copies some stages ahead, and the gathers become shared loads at an
+// immediate distance for a lane's four rows.  The gathers from global memory
+// (csr_tab_kernel) waited for L2 most of the time: 97 us for y = A x at
+// 256^3, 68 us staged, where the shared-memory pipe is the limit (0.7 of it
+// for the loads, the rest of its slots for the copies coming in).  Staging
+// two tiles a plane apart, which share a run, took 71 us: fewer bytes from
+// L2, but fewer warps per SM to cover the loads.
+// the table's part of csr_win_kernel's shared memory (values, stage
+// positions, lengths)
+__host__ __device__ inline int win_table_bytes(int npat, int vt_size) {
+  return (npat * (kPatLen * (vt_size + 4) + 4) + 127) & ~127;
+}
+
+// An epilogue with `kTakesX` gets x(row) from the staged window.
+template <class T, class = void>
+struct takes_x : std::false_type {};
+template <class T>
+struct takes_x<T, std::void_t<decltype(T::kTakesX)>> : std::integral_constant<bool, T::kTakesX> {};
+
+template <typename VT, class Epi>
+__device__ __forceinline__ void epi_row(const Epi& ep, long row, VT s, VT xi, double* acc) {
+  if constexpr (takes_x<Epi>::value) ep.row_x(row, s, xi, acc);
+  else ep.row(row, s, acc);
+}
+
+// Sums of Q rows (kLanes apart) of one table entry from the staged x at xs, 0
+// + v0 x0 + ... each.  The padding of a short row is loaded (it is the row's
+// own x) but not added; an eighth entry is loaded when a lane has one.
+template <int Q, typename VT>
+__device__ __forceinline__ void tab_dot(int id, const int* s_off, const VT* s_val, const int* s_len, const VT* xs,
+                                        VT (&s)[Q]) {
+  const int len = s_len[id];
+  const int4* pq = reinterpret_cast<const int4*>(s_off + id * kPatLen);
+  const VT* vs = s_val + id * kPatLen;
+  const bool eight = __any_sync(0xffffffffu, len == kPatLen);
+#pragma unroll
+  for (int q = 0; q < Q; ++q) s[q] = VT(0);
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int4 o = pq[half];
+    VT x[4][Q];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (half == 1 && u == 3 && !eight) continue;
+      const VT* xu = xs + (u == 0 ? o.x : u == 1 ? o.y : u == 2 ? o.z : o.w);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) x[u][q] = xu[q * kLanes];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (half * 4 + u < len) {
+        const VT v = vs[half * 4 + u];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) s[q] = vadd(s[q], vmul(v, x[u][q]));
+      }
+  }
+}
+
+template <typename VT, class Epi>
+__global__ void __launch_bounds__(kCsrThreads, 3)
+    csr_win_kernel(const uint8_t* __restrict__ pid, const int* __restrict__ pat, const int* __restrict__ plen,
+                   const VT* __restrict__ rowv, int npat, int n, int ncols, const VT* __restrict__ x,
+                   const __grid_constant__ WinPlan plan, int stages, Epi epi, RedCtx red, int* err) {
+  constexpr int NR = Epi::NRED;
+  constexpr int NR1 = NR > 0 ? NR : 1;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ double held[NR > 0 ? kHeldTiles : 1][NR1][8];
+  __shared__ long held_tile[NR > 0 ? kHeldTiles : 1];
+  __shared__ double scratch[8];
+  __shared__ int s_flag;
+  __shared__ uint64_t full[kStages], empty[kStages];
+  if (!epi.active()) return;
+  VT* s_val = reinterpret_cast<VT*>(smem);
+  int* s_off = reinterpret_cast<int*>(s_val + (size_t)npat * kPatLen);
+  int* s_len = s_off + npat * kPatLen;
+  const int tab = win_table_bytes(npat, (int)sizeof(VT));
+  const int stage_bytes = plan.total * (int)sizeof(VT) + kTile;
+  unsigned char* stage0 = smem + tab;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = threadIdx.x;
+  if (j == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], kConsumerWarps);
+    }
+    fence_mbar_init();
+  }
+  // position in a stage of x(tile's first row + o)
+  auto staged = [&](int o) {
+    int at = 0;
+    for (int g = 0; g < plan.nseg; ++g)
+      if (o >= plan.start[g] && o <= plan.start[g] + plan.len[g] - kTile) at = plan.base[g] + o - plan.start[g];
+    return at;
+  };
+  for (int q = j; q < npat * kPatLen; q += kCsrThreads) {
+    s_val[q] = rowv[q];
+    s_off[q] = staged(pat[q]);
+  }
+  for (int q = j; q < npat; q += kCsrThreads) s_len[q] = plen[q];
+  __syncthreads();
+  const long nvis = red.nvisit >= 0 ? red.nvisit : ((long)n + kTile - 1) / kTile;
+
+  if (warp == kConsumerWarps) {
+    // ---------------- producer warp (lane 0) ----------------
+    if (lane != 0) return;
+    constexpr int kUnit = 16 / (int)sizeof(VT);  // elements of a 16-byte unit
+    int it = 0;
+    for (long k = blockIdx.x; k < nvis; k += gridDim.x, ++it) {
+      const long row0 = tile_of(red, k, nvis) * kTile;
+      const int st = it % stages;
+      if (it >= stages && !mbar_wait_bounded(&empty[st], (uint32_t)((it / stages - 1) & 1), err)) return;
+      unsigned char* sb = stage0 + (size_t)st * stage_bytes;
+      VT* xs = reinterpret_cast<VT*>(sb + kTile);
+      const uint32_t pb = (uint32_t)((min((long)kTile, (long)n - row0) + 15) & ~15L);
+      uint32_t bytes = pb;
+      for (int g = 0; g < plan.nseg; ++g) {
+        const long g0 = row0 + plan.start[g];
+        const long lo = max(g0, 0L), hi = min(g0 + plan.len[g], (long)ncols);
+        if (hi <= lo) continue;
+        // (lo is a multiple of 4 and x 16-byte aligned; a ragged end of x is
+        // copied by hand)
+        const long whole = lo + (hi - lo) / kUnit * kUnit;
+        bytes += (uint32_t)(whole - lo) * (uint32_t)sizeof(VT);
+        for (long q = whole; q < hi; ++q) xs[plan.base[g] + (q - g0)] = x[q];
+      }
+      mbar_arrive_expect_tx(&full[st], bytes);
+      bulk_g2s(sb, pid + row0, pb, &full[st]);
+      for (int g = 0; g < plan.nseg; ++g) {
+        const long g0 = row0 + plan.start[g];
+        const long lo = max(g0, 0L), hi = min(g0 + plan.len[g], (long)ncols);
+        if (hi <= lo) continue;
+        const uint32_t nb = (uint32_t)((hi - lo) / kUnit * kUnit) * (uint32_t)sizeof(VT);
+        if (nb) bulk_g2s(xs + plan.base[g] + (lo - g0), x + lo, nb, &full[st]);
+      }
+    }
+    return;
+  }
+
+  // ---------------- consumer warps ----------------
+  [[maybe_unused]] int nheld = 0;
+  auto flush = [&]() {
+    named_bar_sync(1, kLanes);
+    for (int q = j; q < nheld * NR1; q += kLanes) {
+      const int sl = q / NR1, r = q % NR1;
+      double tot = held[sl][r][0];
+#pragma unroll
+      for (int w = 1; w < 8; ++w) tot = dadd(tot, held[sl][r][w]);
+      red.partials[(long)r * red.ntiles + held_tile[sl]] = tot;
+    }
+    __threadfence();
+    named_bar_sync(1, kLanes);
+    nheld = 0;
+  };
+  const int centre = staged(0);  // x(row) of a lane's first row in a stage
+  Epi ep = epi;
+  int it = 0;
+  for (long k = blockIdx.x; k < nvis; k += gridDim.x, ++it) {
+    const long t = tile_of(red, k, nvis);
+    const int st = it % stages;
+    if (!mbar_wait_bounded(&full[st], (uint32_t)((it / stages) & 1), err)) return;
+    const unsigned char* sb = stage0 + (size_t)st * stage_bytes;
+    const VT* xs = reinterpret_cast<const VT*>(sb + kTile) + j;
+    const VT* xc = xs + centre;
+    double acc[NR1];
+#pragma unroll
+    for (int r = 0; r < NR1; ++r) acc[r] = 0.0;
+    const long row0 = t * kTile + j;
+    int cur[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) cur[q] = row0 + q * kLanes < n ? (int)sb[j + q * kLanes] : -1;
+    const bool same = cur[0] >= 0 && cur[1] == cur[0] && cur[2] == cur[0] && cur[3] == cur[0];
+    if (__all_sync(0xffffffffu, same)) {
+      // one table entry for the lane's four rows
+      VT s[4];
+      tab_dot<4>(cur[0], s_off, s_val, s_len, xs, s);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) epi_row(ep, row0 + q * kLanes, s[q], xc[q * kLanes], acc);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        VT s[1];
+        tab_dot<1>(max(cur[q], 0), s_off, s_val, s_len, xs + q * kLanes, s);
+        if (cur[q] >= 0) epi_row(ep, row0 + q * kLanes, s[0], xc[q * kLanes], acc);
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[st]);
+    if constexpr (NR > 0) {
+      if (nheld + 1 > kHeldTiles) flush();
+#pragma unroll
+      for (int r = 0; r < NR1; ++r) {
+        const double w = warp_fold(acc[r]);
+        if (lane == 0) held[nheld][r][warp] = w;
+      }
+      if (j == 0) held_tile[nheld] = t;
+      ++nheld;
+    }
+  }
+  if constexpr (NR > 0) {
+    flush();
+    double tot[NR1];
+    if (red.finish && grid_finish<NR1>(red, tot, scratch, &s_flag, j, 1)) ep.finish(tot);
   }
 }
 

@@ -253,11 +253,9 @@ struct TileWindow {
   long partials_cap = 0;
 };
 
-// max_per_sm > 0 caps the resident CTAs per SM (the batched solves' tuner).
-template <typename VT, typename CT, class Epi>
-int launch_csr_ct(celg_handle* h, const CsrDev& A, const VT* vals, const CT* cols, int cap,
-                  const VT* x, const Epi& epi, const TileWindow* win = nullptr, int max_per_sm = 0) {
-  const long nt = ntiles_of(A.n);
+// The tiles a launch of a CSR sweep visits and where its partials go.
+template <class Epi>
+int csr_red_ctx(celg_handle* h, long nt, const TileWindow* win, RedCtx* out, long* visits) {
   RedCtx red{nullptr, h->ticket, nt};
   long nvis = nt;
   if (win) {
@@ -277,12 +275,24 @@ int launch_csr_ct(celg_handle* h, const CsrDev& A, const VT* vals, const CT* col
     }
     red.nvisit = nvis;
     red.partials = win->partials;
-    if (win->inside && nvis == 0) return CELG_OK;
   } else if (Epi::NRED > 0) {
     int st = ensure_partials(h, nt, Epi::NRED);
     if (st) return st;
     red.partials = h->partials;
   }
+  *out = red;
+  *visits = nvis;
+  return CELG_OK;
+}
+
+// max_per_sm > 0 caps the resident CTAs per SM (the batched solves' tuner).
+template <typename VT, typename CT, class Epi>
+int launch_csr_ct(celg_handle* h, const CsrDev& A, const VT* vals, const CT* cols, int cap,
+                  const VT* x, const Epi& epi, const TileWindow* win = nullptr, int max_per_sm = 0) {
+  RedCtx red;
+  long nvis = 0;
+  if (const int st = csr_red_ctx<Epi>(h, ntiles_of(A.n), win, &red, &nvis)) return st;
+  if (win && win->inside && nvis == 0) return CELG_OK;
   if (A.n == 0) return CELG_OK;
   red.sweep = next_sweep(h, true);
   constexpr bool kPat = std::is_same<CT, PatIdx>::value;
@@ -302,13 +312,76 @@ int launch_csr_ct(celg_handle* h, const CsrDev& A, const VT* vals, const CT* col
   return CELG_OK;
 }
 
-// CSR sweep over the row patterns when the matrix has them (same values,
-// same columns, same order: the same sums), else over the 1-byte column
-// offsets, else (fallback false) nothing is launched and 1 is returned.
+template <typename VT>
+const VT* row_values(const CsrDev& A) {
+  if constexpr (sizeof(VT) == 8) return A.rowv;
+  else return A.rowv32;
+}
+
+// CSR sweep over the row table (row_forms.cu).
+template <typename VT, class Epi>
+int launch_csr_tab(celg_handle* h, const CsrDev& A, const VT* x, const Epi& epi, const TileWindow* win) {
+  RedCtx red;
+  long nvis = 0;
+  if (const int st = csr_red_ctx<Epi>(h, ntiles_of(A.n), win, &red, &nvis)) return st;
+  if (A.n == 0 || (win && win->inside && nvis == 0)) return CELG_OK;
+  red.sweep = next_sweep(h, false);
+  const int smem = A.npat * (kPatLen * ((int)sizeof(VT) + 4) + 4);
+  // Staged when two stages fit a third of an SM, x is aligned for bulk copies
+  // and every CTA has a tile (below that the ring only adds latency).
+  const int tab = win_table_bytes(A.npat, (int)sizeof(VT));
+  const int stage = A.win.total * (int)sizeof(VT) + kTile;
+  const int stages = A.win.nseg > 0 ? std::min(kStages, (72 * 1024 - tab) / stage) : 0;
+  if (stages >= 2 && ((uintptr_t)x & 15) == 0 && nvis >= 3L * h->sms) {
+    const int bytes = tab + stages * stage;
+    if (const int st = allow_dynamic_smem<csr_win_kernel<VT, Epi>>(bytes)) return st;
+    csr_win_kernel<VT, Epi><<<(int)std::min(nvis, 3L * h->sms), kCsrThreads, bytes, h->stream>>>(
+        A.pid, A.pat, A.plen, row_values<VT>(A), A.npat, A.n, A.ncols, x, A.win, stages, epi, red, h->err_d);
+    CELG_CUDA(cudaGetLastError());
+    return CELG_OK;
+  }
+  const int grid = (int)std::max(
+      1L, std::min(nvis, (long)h->sms * resident_per_sm<csr_tab_kernel<VT, Epi>>(kLanes, kPatMax * 100)));
+  csr_tab_kernel<VT, Epi><<<grid, kLanes, smem, h->stream>>>(A.pid, A.pat, A.plen, row_values<VT>(A), A.npat, A.n, x,
+                                                             epi, red);
+  CELG_CUDA(cudaGetLastError());
+  return CELG_OK;
+}
+
+// Most rows for csr_rows_kernel.  Row table: 32^3 rows 4.5 us against 6.2 by
+// csr_tab_kernel's tiles, 80^3 6.8 : 8.3, 96^3 10.3 : 10.3, 128^3 16.8 : 12.4.
+// Row patterns against the staged csr_tma_kernel: 32^3 4.6 : 6.2, 80^3 10.0 :
+// 12.3, 96^3 14.4 : 12.9, 128^3 34.9 : 25.0.
+constexpr long kRowsTab = 800000, kRowsPat = 600000;
+
+template <typename VT, class Epi>
+int launch_csr_rows(celg_handle* h, const CsrDev& A, const VT* vals, const VT* x, const Epi& epi) {
+  const int grid = (A.n + kLanes - 1) / kLanes;
+  const int table = A.npat * kPatLen * 4 + A.npat * 4;
+  if (A.rowv)
+    csr_rows_kernel<VT, Epi, true><<<grid, kLanes, A.npat * kPatLen * (int)sizeof(VT) + table, h->stream>>>(
+        A.rp, A.pid, A.pat, A.plen, row_values<VT>(A), A.npat, A.n, x, epi);
+  else
+    csr_rows_kernel<VT, Epi, false><<<grid, kLanes, kLanes * kPatLen * (int)sizeof(VT) + table, h->stream>>>(
+        A.rp, A.pid, A.pat, A.plen, vals, A.npat, A.n, x, epi);
+  CELG_CUDA(cudaGetLastError());
+  return CELG_OK;
+}
+
+// CSR sweep over the row table or the row patterns when the matrix has them
+// (same values, same columns, same order: the same sums), else over the
+// 1-byte column offsets, else nothing is launched and *done is false.
 template <typename VT, class Epi>
 int launch_csr_compact(celg_handle* h, const CsrDev& A, const VT* vals, const VT* x, const Epi& epi,
                        const TileWindow* win, int max_per_sm, bool* done) {
   *done = true;
+  if constexpr (Epi::NRED == 0 && !is_batched<Epi>::value) {
+    if (A.pid && !win && A.n > 0 && A.n <= (A.rowv ? kRowsTab : kRowsPat))
+      return launch_csr_rows<VT>(h, A, vals, x, epi);
+  }
+  if constexpr (!is_batched<Epi>::value) {
+    if (A.rowv) return launch_csr_tab<VT>(h, A, x, epi, win);
+  }
   if (A.pid)
     return launch_csr_ct<VT, PatIdx>(h, A, vals, reinterpret_cast<const PatIdx*>(A.pid), A.cap, x,
                                      epi, win, max_per_sm);
@@ -317,20 +390,23 @@ int launch_csr_compact(celg_handle* h, const CsrDev& A, const VT* vals, const VT
   return CELG_OK;
 }
 
-// CSR sweep with the matrix's own column indices; the FP32 copy uses the
-// row patterns or the 1-byte offset dictionary when the matrix has them.
+// CSR sweep in the matrix's most compact form.
 template <typename VT, class Epi>
 int launch_csr(celg_handle* h, const CsrDev& A, const VT* vals, const VT* x, const Epi& epi) {
-  if constexpr (sizeof(VT) == 4) {
-    bool done = false;
-    const int st = launch_csr_compact<VT>(h, A, vals, x, epi, nullptr, 0, &done);
-    if (done) return st;
-  }
+  bool done = false;
+  const int st = launch_csr_compact<VT>(h, A, vals, x, epi, nullptr, 0, &done);
+  if (done) return st;
   return launch_csr_ct<VT, int>(h, A, vals, A.ci, A.cap, x, epi);
 }
 
 template <class Epi>
 int launch_jad(celg_handle* h, const CsrDev& A, const JadDev& J, const double* x, const Epi& epi) {
+  // A jagged row's diagonals are its entries in stored order, so a sweep that
+  // only stores row sums gives the same bits from the row patterns, which
+  // need no permutation.  (With a reduction the order of the rows counts.)
+  if constexpr (Epi::NRED == 0) {
+    if (A.pid) return launch_csr<double>(h, A, A.v, x, epi);
+  }
   const long nt = ntiles_of(A.n);
   RedCtx red{nullptr, h->ticket, nt};
   if (Epi::NRED > 0) {

@@ -455,6 +455,7 @@ extern "C" int celg_destroy(celg_handle* h) {
   cudaFree(h->oc_slots);
   cudaFree(h->gm_work);
   cudaFree(h->gm_state_d);
+  cudaFree(h->gm_exch);
   cudaFreeHost(h->gm_state_h);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);

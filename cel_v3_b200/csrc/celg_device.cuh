@@ -120,6 +120,18 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
+// Whether the i-th unsuccessful poll of a word in global memory may be
+// followed by another: looks at the clock every 64 polls, and gives up (and
+// makes the CTA's other waiting threads give up) after kWaitLimitNs.
+__device__ __forceinline__ bool poll_more(unsigned i, unsigned long long& t0, int* abort_) {
+  if ((i & 63u) != 63u) return true;
+  const unsigned long long t = global_ns();
+  if (!t0) t0 = t;
+  if (t - t0 <= kWaitLimitNs && !*(volatile int*)abort_) return true;
+  *(volatile int*)abort_ = 1;
+  return false;
+}
+
 // Untiled bulk copy global -> shared, completion signalled on `bar`.
 // dst, src 16-byte aligned and bytes a multiple of 16 (checked by callers).
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes,

@@ -143,6 +143,7 @@ struct celg_handle {
   size_t gm_cap = 0;          // doubles
   void* gm_state_d = nullptr;
   void* gm_state_h = nullptr; // pinned
+  void* gm_exch = nullptr;    // exchange words of its one-kernel orthogonalisation
   // last solve timing
   float last_ms = 0.f;
   int last_iters = 0;

@@ -219,9 +219,8 @@ __global__ void gm_cycle_start_kernel(GmArgs a) {
 // Arnoldi step j after the Gram-Schmidt sweeps left the raw column
 // h(0..j+1, j): the previous rotations, the new rotation, gamma and the
 // convergence test (:722-737), in the host restatement's operation order.
-__global__ void gm_givens_kernel(GmArgs a, int j) {
+__device__ void gm_givens(const GmArgs& a, int j) {
   GmState* s = a.st;
-  if (!s->act) return;
   s->steps += 1;
   for (int i = 0; i < j; ++i) {
     if (a.literal) {
@@ -248,6 +247,292 @@ __global__ void gm_givens_kernel(GmArgs a, int j) {
     s->jdone = j + 1;
     s->conv = 1;
     s->act = 0;
+  }
+}
+
+__global__ void gm_givens_kernel(GmArgs a, int j) {
+  if (a.st->act) gm_givens(a, j);
+}
+
+// ---- one Arnoldi step's orthogonalisation in one cooperative kernel ----------------
+//
+// As one sweep per basis vector, modified Gram-Schmidt reads w, v_i and
+// v_i+1 and writes w, 32 n bytes, for each of the j+1 vectors of step j: at
+// 128^3 and 15 vectors on average 210 us a step, all of it memory time.  Here
+// each CTA keeps its share of w in registers for the whole step and each v_i
+// in shared memory between its use as the next and as the current vector, so
+// that an MGS step reads 8 n bytes, and the vector after next is on its way
+// (bulk copy) while the coefficient is being summed.  The tiles, the order
+// within a tile and the tree over the tile sums are those of tile_kernel.
+//
+// Exchange: a CTA publishes its tile sums, CTA 0 polls and folds them and
+// publishes the coefficient, all as 16-byte words of a value and the number
+// of the exchange, written and read whole, so that a word needs no reset.  A
+// tile's word is not written again before its CTA has the coefficient that
+// was made from it.  (Eight CTAs folding a group each: twice as slow, 148
+// pollers of eight words hold up the writers.)  Waits are bounded.
+//
+// The copies of the vector after next start when the pass over the current
+// one is done, a few at a time: all at once they queue the exchange's words
+// behind 14 MB of data.  (Tile by tile within the pass, with a barrier per
+// tile, the pass took 5800 cycles instead of 2400.)
+constexpr int kGmThreads = 512;            // 128 registers each (a 17th warp would leave 96)
+constexpr int kGmHalf = 7;                 // tiles of w in a thread's registers (4 rows of each)
+constexpr int kGmTiles = 2 * kGmHalf;      // tiles of a CTA, alternating between its two 256-thread halves
+constexpr int kGmStaged = kGmTiles - 2;    // tiles of v that fit shared memory twice; the others come from L2
+constexpr int kGmPolls = 5;                // tile sums a thread of CTA 0 polls
+constexpr int kGmMaxTiles = 2112;
+constexpr int kGmSmem = (2 * kGmStaged * kTile + kGmMaxTiles) * 8;
+
+struct GmExch {
+  ulonglong2* word;           // the coefficient's, then one per tile
+  unsigned long long* count;  // exchanges so far (device)
+};
+
+__device__ __forceinline__ void put_word(ulonglong2* p, double v, unsigned long long tag) {
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+               "l"(__double_as_longlong(v)), "l"(tag)
+               : "memory");
+}
+__device__ __forceinline__ bool get_word(const ulonglong2* p, unsigned long long tag, double* v) {
+  unsigned long long lo, hi;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+  *v = __longlong_as_double((long long)lo);
+  return hi == tag;
+}
+__device__ __forceinline__ double wait_word(const ulonglong2* p, unsigned long long tag, int* abort_) {
+  double v;
+  unsigned long long t0 = 0;
+  for (unsigned i = 0; !get_word(p, tag, &v) && poll_more(i, t0, abort_); ++i) {
+  }
+  return v;
+}
+
+// The butterfly sums (warp_fold) of 8 values per lane at once: at each step
+// the lanes of one half of the butterfly take over one half of the values, so
+// that 9 exchanges do what 40 would.  Every sum adds the same pairs (operands
+// in either order) as warp_fold.  Lane 4 u gets the sum of value u.
+__device__ __forceinline__ double warp_fold8(const double (&v)[8], int lane) {
+  double a[4], b[2], c;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const bool up = lane & 16;
+    const double mine = up ? v[k + 4] : v[k], other = up ? v[k] : v[k + 4];
+    a[k] = dadd(mine, __shfl_xor_sync(0xffffffffu, other, 16));
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const bool up = lane & 8;
+    const double mine = up ? a[k + 2] : a[k], other = up ? a[k] : a[k + 2];
+    b[k] = dadd(mine, __shfl_xor_sync(0xffffffffu, other, 8));
+  }
+  {
+    const bool up = lane & 4;
+    const double mine = up ? b[1] : b[0], other = up ? b[0] : b[1];
+    c = dadd(mine, __shfl_xor_sync(0xffffffffu, other, 4));
+  }
+  c = dadd(c, __shfl_xor_sync(0xffffffffu, c, 2));
+  return dadd(c, __shfl_xor_sync(0xffffffffu, c, 1));
+}
+
+// One pass over the thread's rows: f(value of w, v_i, v_i+1) -> the new w and
+// the term to sum.  FULL: every row exists.
+template <bool FULL, class F>
+__device__ __forceinline__ void gm_pass(double (&wr)[kGmHalf][4], double (&acc)[8], const double* cur, const double* nxt,
+                                        const double* gcur, const double* gnxt, int half, int T, int rows, F f) {
+  constexpr int kLast = kGmHalf - 1;
+  acc[kGmHalf] = 0.0;
+  // the tile that is not staged comes straight from memory
+  double e0[4], e1[4];
+  if (2 * kLast + half < T) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int o = kLast * 2 * kTile + q * kLanes;
+      const bool in = FULL || o < rows;
+      e0[q] = in ? __ldg(gcur + o) : 0.0;
+      e1[q] = in ? __ldg(gnxt + o) : 0.0;
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < kGmHalf; ++s) {
+    double t = 0.0;
+    if (2 * s + half < T) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int o = s * 2 * kTile + q * kLanes;
+        if (FULL || o < rows) {
+          const double a = s == kLast ? e0[q] : cur[o];
+          const double b = s == kLast ? e1[q] : nxt[o];
+          t = dadd(t, f(wr[s][q], a, b));
+        }
+      }
+    }
+    acc[s] = t;
+  }
+}
+
+__global__ void __launch_bounds__(kGmThreads, 1)
+    gm_orth_kernel(GmArgs a, int j, long n, const double* __restrict__ w, double* V, double* Z, size_t nn,
+                   const double* __restrict__ J, GmExch ex, int per_cta, int* err) {
+  extern __shared__ __align__(128) double vbuf[];  // [2][kGmStaged][kTile], then the tile sums (CTA 0)
+  double* tsum = vbuf + 2 * kGmStaged * kTile;
+  __shared__ double part[kGmTiles][8];
+  __shared__ double red[8];
+  __shared__ double s_tot;
+  __shared__ int abort_;
+  __shared__ uint64_t full[2];
+  if (!*(volatile const int*)&a.st->act) return;
+  const int tid = threadIdx.x, half = (tid >> 8) & 1, lane256 = tid & 255;
+  const long ntiles = (n + kTile - 1) / kTile;
+  const long t0 = (long)blockIdx.x * per_cta;
+  const int T = (int)max(0L, min((long)per_cta, ntiles - t0));
+  unsigned long long tag = *(volatile unsigned long long*)ex.count;
+  if (tid == 0) {
+    abort_ = 0;
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    fence_mbar_init();
+  }
+  __syncthreads();
+
+  // offsets of a thread's rows: s 2 kTile + q kLanes from its first
+  const long first = (t0 + half) * kTile + lane256;
+  const long mine = half * kTile + lane256;  // the same within the CTA's share
+  const int rows = (int)min(n - first, 1L << 30);
+  const bool all = (t0 + T) * kTile <= n;
+  // v_i into buffer i & 1, by one thread (vectors start on 128-byte
+  // boundaries and have room to the next 16 bytes)
+  auto fetch = [&](int i, bool spread) {
+    const long bytes = (min((long)min(T, kGmStaged) * kTile, n - t0 * kTile) * 8 + 15) & ~15L;
+    double* dst = vbuf + (size_t)(i & 1) * kGmStaged * kTile;
+    const double* src = V + nn * (size_t)i + t0 * kTile;
+    mbar_arrive_expect_tx(&full[i & 1], (uint32_t)bytes);
+    for (long o = 0; o < bytes; o += 16384) {
+      if (spread && o) __nanosleep(150);
+      bulk_g2s(dst + o / 8, src + o / 8, (uint32_t)min(16384L, bytes - o), &full[i & 1]);
+    }
+  };
+  if (tid == kGmThreads - 1) {
+    fetch(0, false);
+    if (j > 0) fetch(1, false);
+  }
+  auto wait_for = [&](int i) {
+    if (!mbar_wait_bounded(&full[i & 1], (uint32_t)((i >> 1) & 1), err)) *(volatile int*)&abort_ = 1;
+  };
+  auto buf = [&](int i) { return vbuf + (size_t)(i & 1) * kGmStaged * kTile + mine; };
+  auto vec = [&](int i) { return V + nn * (size_t)i + first; };
+  // the sum of the tiles' lane sums acc[s], the same in every thread; after
+  // its first barrier vector `next` is fetched (none: -1)
+  auto total = [&](const double (&acc)[8], int next) -> double {
+    ++tag;
+    const double f = warp_fold8(acc, tid & 31);
+    const int s = (tid & 31) >> 2, l = 2 * s + half;
+    if ((tid & 3) == 0 && s < kGmHalf && l < T) part[l][lane256 >> 5] = f;
+    __syncthreads();
+    if (tid < T) {
+      double g = part[tid][0];
+#pragma unroll
+      for (int k = 1; k < 8; ++k) g = dadd(g, part[tid][k]);
+      put_word(ex.word + 1 + t0 + tid, g, tag);
+    }
+    if (next >= 0 && tid == kGmThreads - 1) fetch(next, true);
+    if (blockIdx.x == 0) {
+      // a thread's words are polled together: one round trip, not one each
+      double v[kGmPolls];
+      unsigned long long t0w = 0;
+      for (unsigned i = 0;; ++i) {
+        bool ok = true;
+#pragma unroll
+        for (int u = 0; u < kGmPolls; ++u) {
+          const int k = tid + u * kGmThreads;
+          if (k < ntiles) ok = get_word(ex.word + 1 + k, tag, &v[u]) && ok;
+        }
+        if (ok || !poll_more(i, t0w, &abort_)) break;
+      }
+#pragma unroll
+      for (int u = 0; u < kGmPolls; ++u)
+        if (tid + u * kGmThreads < ntiles) tsum[tid + u * kGmThreads] = v[u];
+      __syncthreads();
+      if (tid < kLanes) {
+        double g = 0.0;
+        for (int k = tid; k < ntiles; k += kLanes) g = dadd(g, tsum[k]);
+        g = warp_fold(g);
+        if ((tid & 31) == 0) red[tid >> 5] = g;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        double g = red[0];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) g = dadd(g, red[k]);
+        put_word(ex.word, g, tag);
+        s_tot = g;
+      }
+    } else if (tid == 0) {
+      s_tot = wait_word(ex.word, tag, &abort_);
+    }
+    __syncthreads();
+    return s_tot;
+  };
+
+  double wr[kGmHalf][4], acc[8];
+#pragma unroll
+  for (int s = 0; s < kGmHalf; ++s)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int o = s * 2 * kTile + q * kLanes;
+      wr[s][q] = 2 * s + half < T && o < rows ? __ldg(w + first + o) : 0.0;
+    }
+  wait_for(0);
+  const auto dot = [](double x, double v, double) { return dmul(v, x); };
+  if (all) gm_pass<true>(wr, acc, buf(0), buf(0), vec(0), vec(0), half, T, rows, dot);
+  else gm_pass<false>(wr, acc, buf(0), buf(0), vec(0), vec(0), half, T, rows, dot);
+  double h = total(acc, -1);
+  if (blockIdx.x == 0 && tid == 0) a.h(0, j) = h;
+  for (int i = 0; i < j; ++i) {
+    wait_for(i + 1);
+    const auto step = [h](double& x, double v, double vn) {
+      x = __dsub_rn(x, dmul(h, v));
+      return dmul(vn, x);
+    };
+    if (all) gm_pass<true>(wr, acc, buf(i), buf(i + 1), vec(i), vec(i + 1), half, T, rows, step);
+    else gm_pass<false>(wr, acc, buf(i), buf(i + 1), vec(i), vec(i + 1), half, T, rows, step);
+    h = total(acc, i + 2 <= j ? i + 2 : -1);
+    if (blockIdx.x == 0 && tid == 0) a.h(i + 1, j) = h;
+    if (*(volatile int*)&abort_) break;
+  }
+  const auto last = [h](double& x, double v, double) {
+    x = __dsub_rn(x, dmul(h, v));
+    return dmul(x, x);
+  };
+  if (all) gm_pass<true>(wr, acc, buf(j), buf(j), vec(j), vec(j), half, T, rows, last);
+  else gm_pass<false>(wr, acc, buf(j), buf(j), vec(j), vec(j), half, T, rows, last);
+  h = sqrt(total(acc, -1));
+  if (blockIdx.x == 0 && tid == 0) a.h(j + 1, j) = h;
+  // v_{j+1} = w / h(j+1, j), z_{j+1} = J v_{j+1}: not read when the cycle ends here
+  if (j + 1 < a.M) {
+    double* v = V + nn * (size_t)(j + 1) + first;
+    double* z = Z + nn * (size_t)(j + 1) + first;
+#pragma unroll
+    for (int s = 0; s < kGmHalf; ++s)
+      if (2 * s + half < T)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int o = s * 2 * kTile + q * kLanes;
+          if (o < rows) {
+            const double x = __ddiv_rn(wr[s][q], h);
+            v[o] = x;
+            z[o] = dmul(x, __ldg(J + first + o));
+          }
+        }
+  }
+  if (tid == 0 && *(volatile int*)&abort_) atomicExch(err, kErrTimeout);
+  if (blockIdx.x == 0 && tid == 0) {
+    *ex.count = tag;
+    gm_givens(a, j);
+    if (*(volatile int*)&abort_) a.st->act = 0;
   }
 }
 
@@ -443,6 +728,8 @@ struct GmPlan {
   double* r;
   double* w;
   GmArgs a;
+  GmExch ex;      // exchange words of gm_orth_kernel
+  int per_cta;    // its tiles per CTA; 0: the graph of sweeps
   double* Vp(int i) const { return V + nn * (size_t)i; }
   double* Zp(int i) const { return Z + nn * (size_t)i; }
   double* Hp(int i, int j) const { return a.H + (size_t)j * (a.M + 1) + i; }
@@ -473,6 +760,43 @@ static int gm_record_setup(celg_handle* h, const GmPlan& g) {
   return CELG_OK;
 }
 
+static int gm_orth(celg_handle* h, const GmPlan& g, int j) {
+  GmArgs a = g.a;
+  long n = g.n;
+  const double* w = g.w;
+  double *V = g.V, *Z = g.Z;
+  size_t nn = g.nn;
+  const double* J = g.m->jacobi;
+  GmExch ex = g.ex;
+  int per = g.per_cta;
+  int* err = h->err_d;
+  void* params[] = {&a, &j, &n, &w, &V, &Z, &nn, &J, &ex, &per, &err};
+  const int grid = (int)((ntiles_of(n) + per - 1) / per);
+  CELG_CUDA(cudaLaunchCooperativeKernel((const void*)gm_orth_kernel, dim3(grid), dim3(kGmThreads), params, kGmSmem,
+                                        h->stream));
+  return CELG_OK;
+}
+
+// Tiles per CTA of gm_orth_kernel, 0 when w does not fit the registers of the
+// resident CTAs (then the graph of sweeps runs; CELG_ONCHIP_ROWS as for PCG).
+static int gm_plan_orth(celg_handle* h, GmPlan* g) {
+  g->per_cta = 0;
+  const long nt = ntiles_of(g->n);
+  const char* e = std::getenv("CELG_ONCHIP_ROWS");
+  if (g->n < 1 || nt > std::min((long)kGmTiles * h->sms, (long)kGmMaxTiles) || (e && g->n > std::atol(e))) return CELG_OK;
+  if (const int st = allow_dynamic_smem<gm_orth_kernel>(kGmSmem)) return st;
+  int per_sm = 0;
+  CELG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gm_orth_kernel, kGmThreads, kGmSmem));
+  if (per_sm < 1) return CELG_OK;
+  const size_t bytes = 256 + sizeof(ulonglong2) * (size_t)(kGmMaxTiles + 1);
+  if (!h->gm_exch) CELG_CUDA(cudaMalloc(&h->gm_exch, bytes));
+  CELG_CUDA(cudaMemsetAsync(h->gm_exch, 0, bytes, h->stream));
+  g->ex.count = static_cast<unsigned long long*>(h->gm_exch);
+  g->ex.word = static_cast<ulonglong2*>(h->gm_exch) + 15;
+  g->per_cta = (int)((nt + h->sms - 1) / h->sms);
+  return CELG_OK;
+}
+
 // One restart cycle: M Arnoldi steps (the kernels of the steps after
 // convergence return at once), back substitution, x update, the new
 // residual and the loop decision.
@@ -487,6 +811,11 @@ static int gm_record_cycle(celg_handle* h, const GmPlan& g) {
   for (int j = 0; !st && j < M; ++j) {
     // w = 0 + A z_j (:680-697)
     st = gm_spmv(h, g, g.Zp(j), g.w);
+    if (!st && g.per_cta > 0) {
+      st = gm_orth(h, g, j);
+      if (st) break;
+      continue;
+    }
     // h_0j = v_0 . w, then modified Gram-Schmidt with the next coefficient fused
     if (!st) st = launch_tile(h, g.n, OpDotIf{g.Vp(0), g.w, g.Hp(0, j), act});
     for (int i = 0; !st && i <= j; ++i) {
@@ -526,7 +855,8 @@ int gmres_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const c
   if (p->iter_max < 0) return CELG_ERR_ARG;
   if (!m->jacobi) return CELG_ERR_STATE;
   if (fmt == CELG_FMT_JAD && m->jad.mmax < 0) return CELG_ERR_STATE;
-  const size_t nn = (size_t)std::max(1L, n);
+  // distance of the basis vectors: each starts on a 128-byte boundary
+  const size_t nn = ((size_t)std::max(1L, n) + 15) & ~(size_t)15;
   int st = ensure_work(h, (size_t)n);
   if (!st) st = ensure_offset_dict(h, m);
   if (!st) st = ensure_gmres_work(h, nn, M);
@@ -551,6 +881,7 @@ int gmres_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const c
   g.a = GmArgs{sd, g.Z + nn * (size_t)M, M, hist_cap ? h->hist_d : nullptr, hist_cap, p->iter_max,
                p->literal_ref_bugs, 0, h->err_d};
   CELG_CUDA(cudaMemsetAsync(h->err_d, 0, sizeof(int), h->stream));
+  if ((st = gm_plan_orth(h, &g))) return st;
   if (!graphs_enabled()) {
     // host-driven (profiling): one poll of the loop flag per restart cycle
     CELG_CUDA(cudaEventRecord(h->ev0, h->stream));
@@ -567,9 +898,9 @@ int gmres_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const c
     CELG_CUDA(cudaEventRecord(h->ev1, h->stream));
   } else {
     char kb[512];
-    std::snprintf(kb, sizeof(kb), "gmres|%p|%d|%d|%p|%p|%d|%d|%d|%.17g|%.17g|%d|%d", (const void*)m,
+    std::snprintf(kb, sizeof(kb), "gmres|%p|%d|%d|%p|%p|%d|%d|%d|%.17g|%.17g|%d|%d|%d", (const void*)m,
                   m->csr.n, fmt, (const void*)b, (const void*)x, M, p->x0_mode, p->literal_ref_bugs,
-                  p->eps_abs, p->eps_rel, p->iter_max, hist_cap);
+                  p->eps_abs, p->eps_rel, p->iter_max, hist_cap, g.per_cta);
     const std::string key(kb);
     GraphEntry* ge = graph_cache_find(h, key);
     if (!ge) {

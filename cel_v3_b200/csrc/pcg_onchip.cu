@@ -96,15 +96,6 @@ __device__ __forceinline__ void load2(const double* q, unsigned long long& a, un
   asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(q) : "memory");
 }
 
-__device__ __forceinline__ bool poll_more(unsigned i, unsigned long long& t0, int* abort_) {
-  if ((i & 63u) != 63u) return true;
-  const unsigned long long t = global_ns();
-  if (!t0) t0 = t;
-  if (t - t0 <= kWaitLimitNs && !*(volatile int*)abort_) return true;
-  *(volatile int*)abort_ = 1;
-  return false;
-}
-
 // The eight warp sums of a tile, waited for, added in warp order.
 __device__ __forceinline__ double tile_sum(const double* q, int* abort_) {
   unsigned long long w[8];

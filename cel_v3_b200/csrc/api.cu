@@ -21,6 +21,58 @@ int cuda_status(cudaError_t e, const char* what) {
   return CELG_ERR_CUDA;
 }
 
+// ---- device blocks of a handle ------------------------------------------------
+
+cudaError_t dev_alloc_bytes(celg_handle* h, void** p, size_t bytes) {
+  *p = nullptr;
+  bytes = std::max<size_t>((bytes + 511) & ~(size_t)511, 512);
+  // the smallest spare block that fits without wasting more than it holds
+  size_t best = h->spare.size();
+  for (size_t k = 0; k < h->spare.size(); ++k)
+    if (h->spare[k].bytes >= bytes && h->spare[k].bytes <= 2 * bytes + 65536 &&
+        (best == h->spare.size() || h->spare[k].bytes < h->spare[best].bytes))
+      best = k;
+  if (best < h->spare.size()) {
+    h->blocks.push_back(h->spare[best]);
+    h->spare_bytes -= h->spare[best].bytes;
+    h->spare.erase(h->spare.begin() + (long)best);
+    *p = h->blocks.back().p;
+    return cudaSuccess;
+  }
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && !h->spare.empty()) {
+    (void)cudaGetLastError();
+    dev_free_spare(h);
+    e = cudaMalloc(p, bytes);
+  }
+  if (e == cudaSuccess) h->blocks.push_back({*p, bytes});
+  return e;
+}
+
+void dev_free(celg_handle* h, void* p) {
+  if (!p) return;
+  for (size_t k = h->blocks.size(); k-- > 0;)
+    if (h->blocks[k].p == p) {
+      const celg_handle::DevBlock b = h->blocks[k];
+      h->blocks.erase(h->blocks.begin() + (long)k);
+      if (b.bytes <= kSpareBlock && h->spare_bytes + b.bytes <= kSpareBytes) {
+        h->spare.push_back(b);
+        h->spare_bytes += b.bytes;
+      } else {
+        cudaFree(p);
+      }
+      return;
+    }
+  cudaFree(p);
+}
+
+void dev_free_spare(celg_handle* h) {
+  cudaStreamSynchronize(h->stream);
+  for (const celg_handle::DevBlock& b : h->spare) cudaFree(b.p);
+  h->spare.clear();
+  h->spare_bytes = 0;
+}
+
 // ---- matrix set-up kernels ---------------------------------------------------
 
 // 0-based conversion, padding of the row-pointer tail and validation.
@@ -207,23 +259,21 @@ int ensure_offset_dict(celg_handle* h, celg_mat* m) {
 }
 
 void free_mat_arrays(celg_mat* m) {
-  cudaFree(m->csr.rp);
-  cudaFree(m->csr.ci);
-  cudaFree(m->csr.v);
-  cudaFree(m->csr.v32);
+  celg_handle* h = m->h;
+  dev_free(h, m->csr.rp);  // ci and v are parts of its block
+  dev_free(h, m->csr.v32);
   cudaFree(m->csr.ci8);
   cudaFree(m->csr.dict);
-  row_forms_free(m->csr);
-  sell_free(m->csr);
+  row_forms_free(h, m->csr);
+  sell_free(h, m->csr);
   cudaFree(m->jad.begin);
   cudaFree(m->jad.ci);
   cudaFree(m->jad.v);
   cudaFree(m->jad.perm);
   cudaFree(m->jad.pid);
-  cudaFree(m->diag);
-  cudaFree(m->jacobi);
-  cudaFree(m->jacobi32);
-  cudaFree(m->scale);
+  dev_free(h, m->diag);  // jacobi is a part of its block
+  dev_free(h, m->jacobi32);
+  dev_free(h, m->scale);
   cudaFree(m->bjinv);
 }
 
@@ -231,17 +281,34 @@ void free_mat_arrays(celg_mat* m) {
 // SpMV's bulk copies round a sub-tile's entry range out to 16-byte units of
 // the narrowest column array: up to 3 entries past nnz with int32 columns,
 // up to 15 with the 1-byte offsets, so ci and v carry 32 zeroed entries.
+// The three arrays are one allocation: each costs its 0.1-0.2 ms to get and
+// again to give back.
 constexpr int kCsrPad = 32;
-int alloc_csr(celg_mat* m, int n, int nnz, int ncols) {
+static size_t block(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+
+// room for nnz_cap entries; the entry count and the padding are set later
+int alloc_csr_room(celg_mat* m, int n, size_t nnz_cap, int ncols) {
   m->csr.n = n;
-  m->csr.nnz = nnz;
   m->csr.ncols = ncols;
-  CELG_CUDA(cudaMalloc(&m->csr.rp, sizeof(int) * ((size_t)n + 1 + 8)));
-  CELG_CUDA(cudaMalloc(&m->csr.ci, sizeof(int) * ((size_t)nnz + kCsrPad)));
-  CELG_CUDA(cudaMalloc(&m->csr.v, sizeof(double) * ((size_t)nnz + kCsrPad)));
+  const size_t rp = block(sizeof(int) * ((size_t)n + 1 + 8)), ci = block(sizeof(int) * (nnz_cap + kCsrPad));
+  unsigned char* p = nullptr;
+  CELG_CUDA(dev_alloc(m->h, &p, rp + ci + sizeof(double) * (nnz_cap + kCsrPad)));
+  m->csr.rp = reinterpret_cast<int*>(p);
+  m->csr.ci = reinterpret_cast<int*>(p + rp);
+  m->csr.v = reinterpret_cast<double*>(p + rp + ci);
+  return CELG_OK;
+}
+
+int set_csr_entries(celg_mat* m, int nnz) {
+  m->csr.nnz = nnz;
   CELG_CUDA(cudaMemsetAsync(m->csr.ci + nnz, 0, sizeof(int) * kCsrPad, m->h->stream));
   CELG_CUDA(cudaMemsetAsync(m->csr.v + nnz, 0, sizeof(double) * kCsrPad, m->h->stream));
   return CELG_OK;
+}
+
+int alloc_csr(celg_mat* m, int n, int nnz, int ncols) {
+  const int st = alloc_csr_room(m, n, (size_t)nnz, ncols);
+  return st ? st : set_csr_entries(m, nnz);
 }
 
 int finish_csr(celg_handle* h, celg_mat* m, int base) {
@@ -433,6 +500,7 @@ extern "C" int celg_destroy(celg_handle* h) {
   multi_free(h->multi);
   h->multi = nullptr;
   graph_cache_clear(h);
+  dev_free_spare(h);
   cudaFree(h->partials);
   cudaFree(h->sb);
   cudaFree(h->sx);
@@ -648,7 +716,7 @@ extern "C" int celg_mat_scale_diagonal(celg_mat* m) {
   CELG_CUDA(cudaStreamSynchronize(m->h->stream));
   graph_cache_clear(m->h);
   multi_forget_matrix(m->h->multi, m);
-  sell_free(m->csr);
+  sell_free(m->h, m->csr);
   st = row_forms_search(m->h, m->csr, true, nullptr);
   if (st) return st;
   CELG_CUDA(cudaStreamSynchronize(m->h->stream));
@@ -666,13 +734,13 @@ extern "C" int celg_mat_make_fp32(celg_mat* m) {
   if (!m || m->csr.ncols != m->csr.n) return CELG_ERR_ARG;
   CELG_CUDA(cudaSetDevice(m->h->device));
   if (!m->csr.v32) {
-    CELG_CUDA(cudaMalloc(&m->csr.v32, sizeof(float) * ((size_t)m->csr.nnz + 32)));
+    CELG_CUDA(dev_alloc(m->h, &m->csr.v32, sizeof(float) * ((size_t)m->csr.nnz + 32)));
     CELG_CUDA(cudaMemsetAsync(m->csr.v32 + m->csr.nnz, 0, sizeof(float) * 32, m->h->stream));
   }
   int st = launch_to_f32(m->h, m->csr.nnz, m->csr.v, m->csr.v32);
   if (!st) st = ensure_offset_dict(m->h, m);
   if (!st && m->jacobi) {
-    if (!m->jacobi32) CELG_CUDA(cudaMalloc(&m->jacobi32, sizeof(float) * std::max(1, m->csr.n)));
+    if (!m->jacobi32) CELG_CUDA(dev_alloc(m->h, &m->jacobi32, sizeof(float) * std::max(1, m->csr.n)));
     st = launch_to_f32(m->h, m->csr.n, m->jacobi, m->jacobi32);
   }
   if (st) return st;

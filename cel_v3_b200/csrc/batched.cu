@@ -787,6 +787,7 @@ struct Batch {
   int nlive = 0;               // systems with at least one row
   // launch shape picked by batch_tune (index into kBatchShapes, -1: not tuned)
   int shape = -1;
+  celg_handle* h = nullptr;  // whose blocks the row patterns are
   std::vector<long> row_off;
   std::vector<int> n;
   // FP32 refinement (allocated on first use): A.v32 holds the FP32 values
@@ -810,7 +811,7 @@ void batch_free(Batch* b) {
   cudaFree(b->A.ci);
   cudaFree(b->A.v);
   cudaFree(b->A.ci8);
-  row_forms_free(b->A);
+  if (b->h) row_forms_free(b->h, b->A);
   cudaFree(b->A.dict);
   cudaFree(b->J);
   cudaFree(b->B);
@@ -837,6 +838,7 @@ static int ew(celg_handle* h, long n) {
 static int batch_build(celg_handle* h, int count, celg_mat* const* mats, const std::string& key,
                        Batch** out) {
   Batch* bt = new Batch();
+  bt->h = h;
   bt->key = key;
   bt->nsys = count;
   bt->row_off.resize(count);

@@ -135,8 +135,11 @@ int launch_scale_vec(celg_handle* h, long n, const double* a, const double* s, d
 
 int launch_jacobi_setup(celg_handle* h, celg_mat* m) {
   const int n = m->csr.n;
-  if (!m->diag) CELG_CUDA(cudaMalloc(&m->diag, sizeof(double) * std::max(1, n)));
-  if (!m->jacobi) CELG_CUDA(cudaMalloc(&m->jacobi, sizeof(double) * std::max(1, n)));
+  if (!m->diag) {
+    const size_t nn = ((size_t)std::max(1, n) + 31) & ~(size_t)31;
+    CELG_CUDA(dev_alloc(h, &m->diag, sizeof(double) * 2 * nn));
+    m->jacobi = m->diag + nn;
+  }
   if (n <= 0) return CELG_OK;
   jacobi_setup_kernel<<<ew_grid(h, n), 256, 0, h->stream>>>(n, m->csr.rp, m->csr.ci, m->csr.v,
                                                              m->scaled ? m->scale : nullptr,
@@ -147,7 +150,7 @@ int launch_jacobi_setup(celg_handle* h, celg_mat* m) {
 
 int launch_row_scale(celg_handle* h, celg_mat* m) {
   const int n = m->csr.n;
-  if (!m->scale) CELG_CUDA(cudaMalloc(&m->scale, sizeof(double) * std::max(1, n)));
+  if (!m->scale) CELG_CUDA(dev_alloc(h, &m->scale, sizeof(double) * std::max(1, n)));
   if (n <= 0) return CELG_OK;
   row_scale_kernel<<<ew_grid(h, n), 256, 0, h->stream>>>(n, m->csr.rp, m->csr.v, m->diag, m->scale);
   CELG_CUDA(cudaGetLastError());

@@ -151,6 +151,13 @@ struct celg_handle {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // tile order of the next sweep (RedCtx::sweep bit 0)
   int sweep_rev = 0;
+  // blocks of dev_alloc in use, and given back ones kept for the next request
+  struct DevBlock {
+    void* p;
+    size_t bytes;
+  };
+  std::vector<DevBlock> blocks, spare;
+  size_t spare_bytes = 0;
 };
 
 struct celg_mat {
@@ -176,6 +183,21 @@ int cuda_status(cudaError_t e, const char* what);
     if (e_ != cudaSuccess) return ::celg::cuda_status(e_, #call); \
   } while (0)
 
+// Device memory of the handle's matrices.  Blocks given back are kept for
+// later requests on the handle, in the order of its stream, up to
+// kSpareBytes in all (getting and returning a block costs 0.1-0.2 ms each,
+// at times milliseconds); celg_destroy frees them.
+constexpr size_t kSpareBlock = (size_t)32 << 20, kSpareBytes = (size_t)96 << 20;
+cudaError_t dev_alloc_bytes(celg_handle* h, void** p, size_t bytes);
+void dev_free(celg_handle* h, void* p);
+void dev_free_spare(celg_handle* h);
+template <typename T>
+cudaError_t dev_alloc(celg_handle* h, T** p, size_t bytes) {
+  void* q = nullptr;
+  const cudaError_t e = dev_alloc_bytes(h, &q, bytes);
+  *p = static_cast<T*>(q);
+  return e;
+}
 int ensure_partials(celg_handle* h, long ntiles, int nred);
 void graph_cache_clear(celg_handle* h);
 void graph_cache_drop_matrix(celg_handle* h, const void* m);
@@ -223,14 +245,16 @@ int ensure_offset_dict(celg_handle* h, celg_mat* m);
 // the same for any CSR array set (left unset beyond 256 distinct offsets)
 int build_offset_dict_csr(celg_handle* h, CsrDev& A);
 // pcg_onchip.cu: drop the sliced copy (the values changed, or the matrix goes)
-void sell_free(CsrDev& A);
+void sell_free(celg_handle* h, CsrDev& A);
 // row_forms.cu
 size_t row_sets_bytes();
 int row_forms_search(celg_handle* h, const CsrDev& A, bool with_values, const int* bad);
 int row_forms_build(celg_handle* h, CsrDev& A, bool with_values);
 int row_forms_jacobi(celg_handle* h, CsrDev& A, const double* J);
-void row_forms_free(CsrDev& A);
+void row_forms_free(celg_handle* h, CsrDev& A);
 int alloc_csr(celg_mat* m, int n, int nnz, int ncols);
+int alloc_csr_room(celg_mat* m, int n, size_t nnz_cap, int ncols);
+int set_csr_entries(celg_mat* m, int nnz);
 int finish_csr(celg_handle* h, celg_mat* m, int base);
 void free_mat_arrays(celg_mat* m);
 // assemble.cu: COO (device arrays, row and column bases) -> CSR matrix

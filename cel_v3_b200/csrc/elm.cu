@@ -17,6 +17,17 @@ struct Elm {
   std::vector<double> vals;
   std::vector<long long> diag_idx;
   int cur_row = -1;
+  // Rows that arrive whole, in order and with ascending columns need no sort:
+  // as long as all do (direct), celg_elm_insert_rows copies the caller's
+  // columns and values straight into the arrays of the matrix to be (dmat,
+  // columns 1-based until it is completed) and keeps the row pointer here.
+  // Any other insertion moves the entries to rows/cols/vals above.
+  bool direct = true;
+  bool lost = false;       // completing them failed: nothing is left to retry with
+  std::vector<int> rp;     // one entry per row begun, and the end
+  celg_mat* dmat = nullptr;
+  size_t dcap = 0;         // entries dmat has room for
+  size_t hint = 0;
   celg_mat* mat = nullptr;
   bool completed = false;
   int solver = CELG_SOLVER_GMRES;
@@ -35,8 +46,8 @@ extern "C" int celg_elm_destroy(celg_handle* h) {
   cudaSetDevice(h->device);
   cudaStreamSynchronize(h->stream);
   if (e->mat) celg_mat_destroy(e->mat);
-  cudaFree(e->b_d);
-  cudaFree(e->x_d);
+  if (e->dmat) celg_mat_destroy(e->dmat);
+  dev_free(h, e->b_d);  // x_d is a part of its block
   delete e;
   h->elm = nullptr;
   return CELG_OK;
@@ -55,11 +66,7 @@ extern "C" int celg_elm_init(celg_handle* h, int n_total, int n_local, int row_l
   e->n_local = n_local;
   e->row_low = row_low;
   long long hint = nnz_hint ? (long long)(nnz_hint[0] + nnz_hint[1]) * n_local : 0;
-  if (hint > 0 && hint < (1LL << 31)) {
-    e->rows.reserve((size_t)hint);
-    e->cols.reserve((size_t)hint);
-    e->vals.reserve((size_t)hint);
-  }
+  if (hint > 0 && hint < (1LL << 31)) e->hint = (size_t)hint;
   e->diag_idx.assign((size_t)n_local, -1);
   celg_params_default(&e->params);
   e->params.x0_mode = CELG_X0_REF_ONES;
@@ -94,11 +101,93 @@ extern "C" int celg_elm_row_start(celg_handle* h, int row) {
   return CELG_OK;
 }
 
+// Leaves the direct mode: the entries so far become triplets on the host, in
+// the order they were inserted.
+static int elm_undirect(celg_handle* h, Elm* e) {
+  if (!e->direct) return CELG_OK;
+  const size_t nnz = e->rp.empty() ? 0 : (size_t)e->rp.back();
+  const size_t room = std::max(nnz, e->hint);
+  e->rows.reserve(room);
+  e->cols.reserve(room);
+  e->vals.reserve(room);
+  if (nnz) {
+    e->cols.resize(nnz);
+    e->vals.resize(nnz);
+    CELG_CUDA(cudaMemcpyAsync(e->cols.data(), e->dmat->csr.ci, sizeof(int) * nnz, cudaMemcpyDeviceToHost, h->stream));
+    CELG_CUDA(cudaMemcpyAsync(e->vals.data(), e->dmat->csr.v, sizeof(double) * nnz, cudaMemcpyDeviceToHost, h->stream));
+    CELG_CUDA(cudaStreamSynchronize(h->stream));
+    for (size_t r = 0; r + 1 < e->rp.size(); ++r) {
+      const int row = e->row_low + (int)r;
+      e->rows.insert(e->rows.end(), (size_t)(e->rp[r + 1] - e->rp[r]), row);
+      for (int k = e->rp[r]; k < e->rp[r + 1]; ++k)
+        if (e->cols[(size_t)k] == row) e->diag_idx[r] = k;
+    }
+  }
+  if (e->dmat) celg_mat_destroy(e->dmat);
+  e->dmat = nullptr;
+  e->direct = false;
+  return CELG_OK;
+}
+
+// Whole rows in order with ascending columns, appended to dmat; *taken is
+// false (and nothing done) when the rows are not of that kind, or so few that
+// copies of their own (about 25 us a call) cost more than keeping them on the
+// host until the matrix is complete.
+static int elm_append_rows(celg_handle* h, Elm* e, int first_row, int nrows, const int* row_ptr, const int* cols,
+                           const double* vals, bool* taken) {
+  *taken = false;
+  const int base = row_ptr[0];
+  const size_t total = (size_t)(row_ptr[nrows] - base);
+  const int r0 = first_row - e->row_low;
+  const size_t done = e->rp.empty() ? 0 : e->rp.size() - 1;  // rows begun so far
+  const size_t at = e->rp.empty() ? 0 : (size_t)e->rp.back();
+  if (total < 4096 && nrows < e->n_local) return CELG_OK;
+  if (r0 < (int)done || at + total >= (size_t)1 << 31 || (total > 0 && (!cols || !vals))) return CELG_OK;
+  for (int i = 0; i < nrows; ++i)
+    if (row_ptr[i + 1] < row_ptr[i]) return CELG_OK;
+  bool bad = false;
+  for (int i = 0; i < nrows; ++i) {
+    const int b = row_ptr[i] - base, end = row_ptr[i + 1] - base;
+    if (b == end) continue;
+    bad |= cols[b] < 1 || cols[end - 1] > e->n_total;
+    for (int k = b + 1; k < end; ++k) bad |= cols[k] < cols[k - 1];
+  }
+  if (bad) return CELG_OK;
+  if (at + total > e->dcap || !e->dmat) {
+    celg_mat* m = new celg_mat();
+    m->h = h;
+    const size_t cap = std::max(std::max(at + total, e->hint), e->dmat ? 2 * e->dcap : 0);
+    if (const int st = alloc_csr_room(m, e->n_local, std::min(cap, ((size_t)1 << 31) - 1), e->n_local)) {
+      delete m;
+      return st;
+    }
+    if (at) {
+      CELG_CUDA(cudaMemcpyAsync(m->csr.ci, e->dmat->csr.ci, sizeof(int) * at, cudaMemcpyDeviceToDevice, h->stream));
+      CELG_CUDA(cudaMemcpyAsync(m->csr.v, e->dmat->csr.v, sizeof(double) * at, cudaMemcpyDeviceToDevice, h->stream));
+    }
+    if (e->dmat) celg_mat_destroy(e->dmat);
+    e->dmat = m;
+    e->dcap = std::min(cap, ((size_t)1 << 31) - 1);
+  }
+  if (total) {
+    // (from pageable memory these return when the caller's arrays are read)
+    CELG_CUDA(cudaMemcpyAsync(e->dmat->csr.ci + at, cols, sizeof(int) * total, cudaMemcpyHostToDevice, h->stream));
+    CELG_CUDA(cudaMemcpyAsync(e->dmat->csr.v + at, vals, sizeof(double) * total, cudaMemcpyHostToDevice, h->stream));
+    CELG_CUDA(cudaStreamSynchronize(h->stream));
+  }
+  if (e->rp.empty()) e->rp.push_back(0);
+  e->rp.resize((size_t)r0 + 1, (int)at);  // rows left out are empty
+  for (int i = 0; i < nrows; ++i) e->rp.push_back((int)at + row_ptr[i + 1] - base);
+  *taken = true;
+  return CELG_OK;
+}
+
 extern "C" int celg_elm_insert(celg_handle* h, int col, double value) {
   if (!h || !h->elm) return CELG_ERR_STATE;
   Elm* e = h->elm;
   if (e->completed || e->cur_row < 0) return CELG_ERR_STATE;
   if (col < 1 || col > e->n_total) return CELG_ERR_ARG;
+  if (const int st = elm_undirect(h, e)) return st;
   e->rows.push_back(e->cur_row);
   e->cols.push_back(col);
   e->vals.push_back(value);
@@ -113,6 +202,7 @@ extern "C" int celg_elm_reinsert(celg_handle* h, int col, double value) {
   Elm* e = h->elm;
   if (e->completed || e->cur_row < 0) return CELG_ERR_STATE;
   if (col != e->cur_row) return CELG_ERR_ARG;
+  if (const int st = elm_undirect(h, e)) return st;
   const long long k = e->diag_idx[(size_t)(e->cur_row - e->row_low)];
   if (k < 0) return CELG_ERR_ARG;
   e->vals[(size_t)k] = value;
@@ -135,6 +225,16 @@ extern "C" int celg_elm_insert_rows(celg_handle* h, int first_row, int nrows, co
   const int base = row_ptr[0];
   const long long total = (long long)row_ptr[nrows] - base;
   if (total < 0) return CELG_ERR_ARG;
+  if (e->direct) {
+    cudaSetDevice(h->device);
+    bool taken = false;
+    if (const int st = elm_append_rows(h, e, first_row, nrows, row_ptr, cols, vals, &taken)) return st;
+    if (taken) {
+      e->cur_row = first_row + nrows - 1;
+      return CELG_OK;
+    }
+    if (const int st = elm_undirect(h, e)) return st;
+  }
   e->rows.reserve(e->rows.size() + (size_t)total);
   e->cols.reserve(e->cols.size() + (size_t)total);
   e->vals.reserve(e->vals.size() + (size_t)total);
@@ -154,20 +254,11 @@ extern "C" int celg_elm_insert_rows(celg_handle* h, int first_row, int nrows, co
   return CELG_OK;
 }
 
-// cel_elmSolverMatrixCompleted (:193-439) for one rank: entries sorted by
-// row, then column (cel_sp_mat_format_sparse_31_sort,
-// src/fspmt/cel_sp_mat_module.f90:518-585; equal keys keep insertion order)
-// and the CSR row pointer (cel_sp_mat_to_csr, :430-456), both on the device;
-// then Jacobi, optional diagonal scaling (:375-388 of the ELM module), JAD
-// when selected.
-extern "C" int celg_elm_matrix_completed(celg_handle* h) {
-  if (!h || !h->elm) return CELG_ERR_STATE;
-  Elm* e = h->elm;
-  if (e->completed) return CELG_ERR_STATE;
+// the triplets go to the device as inserted; the stable (row, column) sort
+// and the row pointer are built there (assemble.cu)
+static int elm_complete_triplets(celg_handle* h, Elm* e, celg_mat** m) {
   const size_t nnz = e->vals.size();
   if (nnz >= (size_t)1 << 31) return CELG_ERR_ARG;
-  // the triplets go to the device as inserted; the stable (row, column) sort
-  // and the row pointer are built there (assemble.cu)
   const size_t nz = std::max<size_t>(nnz, 1);
   int *r_d = nullptr, *c_d = nullptr;
   double* v_d = nullptr;
@@ -180,14 +271,48 @@ extern "C" int celg_elm_matrix_completed(celg_handle* h) {
     ce = cudaMemcpyAsync(c_d, e->cols.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice, h->stream);
   if (ce == cudaSuccess && nnz)
     ce = cudaMemcpyAsync(v_d, e->vals.data(), sizeof(double) * nnz, cudaMemcpyHostToDevice, h->stream);
-  celg_mat* m = nullptr;
   int st = ce == cudaSuccess ? coo_to_mat_device(h, e->n_local, e->n_local, (int)nnz, r_d, c_d, v_d,
-                                                 e->row_low, 1, &m)
+                                                 e->row_low, 1, m)
                              : cuda_status(ce, "ELM triplet upload");
   cudaStreamSynchronize(h->stream);
   cudaFree(r_d);
   cudaFree(c_d);
   cudaFree(v_d);
+  return st;
+}
+
+// the rows are in place: their pointer follows
+static int elm_complete_direct(celg_handle* h, Elm* e, celg_mat** m) {
+  const int nnz = e->rp.back();
+  e->rp.resize((size_t)e->n_local + 1, nnz);
+  celg_mat* d = e->dmat;
+  int st = set_csr_entries(d, nnz);
+  if (st) return st;
+  // (the row pointer is 1-based like the columns, for one conversion)
+  for (int& v : e->rp) v += 1;
+  const cudaError_t ce =
+      cudaMemcpyAsync(d->csr.rp, e->rp.data(), sizeof(int) * e->rp.size(), cudaMemcpyHostToDevice, h->stream);
+  st = ce == cudaSuccess ? finish_csr(h, d, 1) : cuda_status(ce, "ELM row pointer");
+  for (int& v : e->rp) v -= 1;
+  if (st) return st;
+  *m = d;
+  e->dmat = nullptr;
+  return CELG_OK;
+}
+
+// cel_elmSolverMatrixCompleted (:193-439) for one rank: entries sorted by
+// row, then column (cel_sp_mat_format_sparse_31_sort,
+// src/fspmt/cel_sp_mat_module.f90:518-585; equal keys keep insertion order)
+// and the CSR row pointer (cel_sp_mat_to_csr, :430-456), both on the device;
+// then Jacobi, optional diagonal scaling (:375-388 of the ELM module), JAD
+// when selected.
+extern "C" int celg_elm_matrix_completed(celg_handle* h) {
+  if (!h || !h->elm) return CELG_ERR_STATE;
+  Elm* e = h->elm;
+  if (e->completed || e->lost) return CELG_ERR_STATE;
+  celg_mat* m = nullptr;
+  e->lost = e->direct && e->dmat;
+  int st = e->lost ? elm_complete_direct(h, e, &m) : elm_complete_triplets(h, e, &m);
   if (st) return st;
   st = celg_mat_jacobi(m);
   if (!st && e->diag_scaling) st = celg_mat_scale_diagonal(m);
@@ -198,11 +323,12 @@ extern "C" int celg_elm_matrix_completed(celg_handle* h) {
     return st;
   }
   e->mat = m;
-  const size_t n = (size_t)std::max(1, e->n_local);
-  if (cudaMalloc(&e->b_d, sizeof(double) * n) != cudaSuccess ||
-      cudaMalloc(&e->x_d, sizeof(double) * n) != cudaSuccess)
-    return CELG_ERR_CUDA;
+  const size_t n = ((size_t)std::max(1, e->n_local) + 31) & ~(size_t)31;
+  if (dev_alloc(h, &e->b_d, sizeof(double) * 2 * n) != cudaSuccess) return CELG_ERR_CUDA;
+  e->x_d = e->b_d + n;
   e->completed = true;
+  e->lost = false;
+  std::vector<int>().swap(e->rp);
   std::vector<int>().swap(e->rows);
   std::vector<int>().swap(e->cols);
   std::vector<double>().swap(e->vals);

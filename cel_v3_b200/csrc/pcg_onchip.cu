@@ -563,11 +563,11 @@ __global__ void slice_fill_kernel(int n, const int* __restrict__ rp, const int* 
   }
 }
 
-void sell_free(CsrDev& A) {
-  cudaFree(A.sell_v);
-  cudaFree(A.sell_v32);
-  cudaFree(A.sell_c);
-  cudaFree(A.sell_base);
+void sell_free(celg_handle* h, CsrDev& A) {
+  dev_free(h, A.sell_v);
+  dev_free(h, A.sell_v32);
+  dev_free(h, A.sell_c);
+  dev_free(h, A.sell_base);
   A.sell_v = nullptr;
   A.sell_v32 = nullptr;
   A.sell_c = A.sell_base = nullptr;
@@ -593,9 +593,9 @@ static int ensure_sell(celg_handle* h, CsrDev& A, const VT* vals, bool* ok) {
       void* tmp = nullptr;
       size_t tmp_bytes = 0;
       cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, width, base, (int)nslices + 1, h->stream);
-      cudaError_t e = cudaMalloc(&width, sizeof(int) * (nslices + 1));
-      if (e == cudaSuccess) e = cudaMalloc(&base, sizeof(int) * (nslices + 1));
-      if (e == cudaSuccess) e = cudaMalloc(&tmp, std::max<size_t>(tmp_bytes, 16));
+      cudaError_t e = dev_alloc(h, &width, sizeof(int) * (nslices + 1));
+      if (e == cudaSuccess) e = dev_alloc(h, &base, sizeof(int) * (nslices + 1));
+      if (e == cudaSuccess) e = dev_alloc(h, &tmp, std::max<size_t>(tmp_bytes, 16));
       if (e == cudaSuccess) e = cudaMemsetAsync(width + nslices, 0, sizeof(int), h->stream);
       int total = 0, longest = 0;
       int* longest_d = h->err_d + 5;
@@ -610,10 +610,10 @@ static int ensure_sell(celg_handle* h, CsrDev& A, const VT* vals, bool* ok) {
       if (e == cudaSuccess)
         e = cudaMemcpyAsync(&longest, longest_d, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
       if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-      cudaFree(width);
-      cudaFree(tmp);
+      dev_free(h, width);
+      dev_free(h, tmp);
       if (e != cudaSuccess || longest > kMaxWidth || 32L * total > 2L * A.nnz + 32 * nslices) {
-        cudaFree(base);
+        dev_free(h, base);
         A.sell_total = 0;
         return e != cudaSuccess ? cuda_status(e, "sliced matrix") : CELG_OK;
       }
@@ -625,15 +625,15 @@ static int ensure_sell(celg_handle* h, CsrDev& A, const VT* vals, bool* ok) {
   VT*& sv = sell_vals(A, vals);
   const bool need_c = !pat && !A.sell_c;
   if (!sv) {
-    cudaError_t e = cudaMalloc(&sv, sizeof(VT) * (size_t)A.sell_total);
-    if (e == cudaSuccess && need_c) e = cudaMalloc(&A.sell_c, sizeof(int) * (size_t)A.sell_total);
+    cudaError_t e = dev_alloc(h, &sv, sizeof(VT) * (size_t)A.sell_total);
+    if (e == cudaSuccess && need_c) e = dev_alloc(h, &A.sell_c, sizeof(int) * (size_t)A.sell_total);
     if (e == cudaSuccess) {
       slice_fill_kernel<VT><<<(int)std::min(((long)A.n + 255) / 256, (long)h->sms * 8), 256, 0, h->stream>>>(
           A.n, A.rp, A.ci, vals, pat ? nullptr : A.sell_base, sv, need_c ? A.sell_c : nullptr);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
-      sell_free(A);
+      sell_free(h, A);
       return cuda_status(e, "sliced matrix");
     }
   }

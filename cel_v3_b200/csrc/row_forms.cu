@@ -198,9 +198,8 @@ static WinPlan plan_window(const int* pat, int count) {
   return w;
 }
 
-void row_forms_free(CsrDev& A) {
-  cudaFree(A.pid);
-  cudaFree(A.pat);
+void row_forms_free(celg_handle* h, CsrDev& A) {
+  dev_free(h, A.pat);  // the other arrays are parts of its block
   A.pid = nullptr;
   A.pat = nullptr;
   A.npat = 0;
@@ -230,7 +229,7 @@ int row_forms_search(celg_handle* h, const CsrDev& A, bool with_values, const in
 // Builds the forms the search found (the stream has been waited for).  On a
 // failed allocation the matrix keeps its plain columns.
 int row_forms_build(celg_handle* h, CsrDev& A, bool with_values) {
-  row_forms_free(A);
+  row_forms_free(h, A);
   if (A.n == 0 || A.nnz == 0) return CELG_OK;
   const RowSets* found = static_cast<const RowSets*>(h->rows_h);
   std::vector<RowSets> keep(1, *found);
@@ -242,16 +241,12 @@ int row_forms_build(celg_handle* h, CsrDev& A, bool with_values) {
       if (s.key[w][q]) rows.emplace_back(s.key[w][q], s.rep[w][q]);
     std::sort(rows.begin(), rows.end());
     const int np = (int)rows.size();
-    // one block: pat, plen, reps (ints), then the tables of 8-byte values
+    // one block: pat, plen, reps (ints), the tables of 8-byte values, the bytes
     const size_t ints = (size_t)np * (kPatLen + 2);
     const size_t tab = ((ints * sizeof(int) + 15) & ~(size_t)15);
-    const size_t bytes = tab + (size_t)np * (kPatLen * 12) + kPatMax * 12 + (size_t)np * 8 + 64;
-    CELG_CUDA(cudaMalloc(&A.pat, bytes));
-    if (cudaMalloc(&A.pid, (size_t)A.n + 16) != cudaSuccess) {
-      (void)cudaGetLastError();
-      row_forms_free(A);
-      return CELG_ERR_CUDA;
-    }
+    const size_t bytes = (tab + (size_t)np * (kPatLen * 12) + kPatMax * 12 + (size_t)np * 8 + 64 + 255) & ~(size_t)255;
+    CELG_CUDA(dev_alloc(h, &A.pat, bytes + (size_t)A.n + 16));
+    A.pid = reinterpret_cast<uint8_t*>(A.pat) + bytes;
     A.npat = np;
     A.plen = A.pat + (size_t)np * kPatLen;
     A.prep = A.plen + np;
@@ -290,11 +285,11 @@ int row_forms_build(celg_handle* h, CsrDev& A, bool with_values) {
       e = cudaMemcpyAsync(pat_h, A.pat, sizeof(int) * (size_t)np * kPatLen, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) {
-      row_forms_free(A);
+      row_forms_free(h, A);
       return cuda_status(e, "row forms");
     }
     if (*mis_h) {  // two different rows with one hash
-      row_forms_free(A);
+      row_forms_free(h, A);
       continue;
     }
     if (w) {

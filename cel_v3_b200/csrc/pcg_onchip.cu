@@ -57,10 +57,10 @@ constexpr int kOcTail = 64;  // doubles after the slots: the totals (kSlotSets),
 // slot sets: p.v, (r.z, r.r) twice, ||b||^2, set-up (r.z, r.r), verification
 // (pairs at even positions)
 enum OcSlot { kSlotUpd0 = 0, kSlotUpd1 = 2, kSlotInit = 4, kSlotPv = 6, kSlotB = 7, kSlotVer = 8, kSlotSets = 9 };
-// longest row of a sliced matrix: with at most 2^16 slices (kOcMaxUnits) the
-// sum of the slice widths stays within an int
-constexpr int kMaxWidth = 32767;
-constexpr long kOcMaxUnits = 1L << 14;
+// longest row of a sliced matrix: with at most 4 kOcMaxUnits slices the sum of
+// the slice widths stays within an int
+constexpr int kMaxWidth = 31000;
+constexpr long kOcMaxUnits = 8 * 2112;
 constexpr unsigned long long kSentinel = ~0ull;
 
 template <typename VT>
@@ -73,6 +73,10 @@ struct OcArgs {
   const uint8_t* pid;
   const int* pat;
   int pat_ints;
+  const int* plen;
+  const VT* rowv;     // row table (then no sliced values), or null
+  int juni;           // one Jacobi value, jval, for all rows
+  VT jval;
   const VT* b;
   VT* x;
   const VT* J;
@@ -530,6 +534,407 @@ __global__ void __launch_bounds__(kOcThreads, 1) pcg_onchip_kernel(OcArgs<VT> a)
   }
 }
 
+// ---- systems of 0.7 to 2.1 million rows ------------------------------------------
+//
+// The same loop where only r and p fit on the chip.  As three sweeps a 128^3
+// system took 60 us an iteration: 140 bytes a row cross from L2 to the SMs,
+// at about 7 TB/s, plus three launches.  With r and p in shared memory it is
+// the values, the gathers, v, J (twice) and x.  A CTA has whole tiles, its
+// two halves alternate between them (warp w of a half has the tile's rows 32
+// w + lane + 256 k), and it publishes tile sums; CTA 0, which folds them all,
+// has kWideLess tiles less and their room for the sums.
+// us an iteration, sweeps : this kernel (variable coefficients, FP64): 90^3
+// 34.8 : 21.9, 104^3 41.3 : 27.0, 120^3 54.8 : 38.4, 128^3 61.3 : 51.5 (the
+// working set leaves L2); constant coefficients 128^3 43.8 : 32.9.
+constexpr int kWideTiles = 14;  // r and p of 14 tiles: 224 of 227 KB
+constexpr int kWideLess = 4;    // 64 KB: two sums of up to 2112 tiles
+constexpr int kWidePolls = 9;
+constexpr int kWideStatic = (2 * kWideTiles * 8 + 16) * 8 + 64;  // its static shared memory
+
+struct WideArgs {
+  OcArgs<double> o;  // slot: kSlotSets x ntiles
+  double* v;
+  int per;           // tiles of a CTA
+};
+
+__host__ __device__ inline int wide_table_bytes(int pat_ints) {
+  return ((pat_ints + pat_ints / kPatLen) * 4 + 127) & ~127;
+}
+
+// the matrix: int32 columns, row patterns, row table
+enum { kFormCols, kFormPat, kFormTable };
+
+// row sum as row_sum, the row's length and pattern from memory
+template <int FORM>
+__device__ __forceinline__ double wide_row_sum(const OcArgs<double>& a, const int* s_pat, const int* s_len,
+                                               const double* src, int row, int lane, int id) {
+  double t = 0.0;
+  if constexpr (FORM != kFormCols) {
+    const int len = s_len[id];
+    const double* xr = src + row;
+    const int4* pq = reinterpret_cast<const int4*>(s_pat + id * kPatLen);
+    double xv[kPatLen], vv[kPatLen];
+    if constexpr (FORM == kFormTable) {
+      // (the lanes of one pattern share the loads; the table stays in L1)
+      const double2* tv = reinterpret_cast<const double2*>(a.rowv + id * kPatLen);
+#pragma unroll
+      for (int e = 0; e < kPatLen; e += 2) {
+        const double2 t2 = __ldg(tv + e / 2);
+        vv[e] = t2.x;
+        vv[e + 1] = t2.y;
+      }
+    } else {
+      const double* gv = a.sv + (size_t)(row >> 5) * (kPatLen * 32) + lane;
+#pragma unroll
+      for (int e = 0; e < kPatLen; ++e)
+        if (e < len) vv[e] = ld_stream(gv + e * 32);
+    }
+    const int4 q0 = pq[0], q1 = pq[1];
+    xv[0] = xr[q0.x];
+    xv[1] = xr[q0.y];
+    xv[2] = xr[q0.z];
+    xv[3] = xr[q0.w];
+    xv[4] = xr[q1.x];
+    xv[5] = xr[q1.y];
+    xv[6] = xr[q1.z];
+    if (len == kPatLen) xv[7] = xr[q1.w];
+#pragma unroll
+    for (int e = 0; e < kPatLen; ++e)
+      if (e < len) t = dadd(t, dmul(vv[e], xv[e]));
+  } else {
+    constexpr int C = 8;
+    const int len = __ldg(a.rp + row + 1) - __ldg(a.rp + row);
+    const size_t at = (size_t)__ldg(a.sbase + (row >> 5)) * 32 + lane;
+    for (int e0 = 0; e0 < len; e0 += C) {
+      int c[C];
+      double xv[C], vv[C];
+#pragma unroll
+      for (int e = 0; e < C; ++e)
+        if (e0 + e < len) {
+          c[e] = ld_stream(a.sc + at + (e0 + e) * 32);
+          vv[e] = ld_stream(a.sv + at + (e0 + e) * 32);
+        }
+#pragma unroll
+      for (int e = 0; e < C; ++e)
+        if (e0 + e < len) xv[e] = src[c[e]];
+#pragma unroll
+      for (int e = 0; e < C; ++e)
+        if (e0 + e < len) t = dadd(t, dmul(vv[e], xv[e]));
+    }
+  }
+  return t;
+}
+
+template <int FORM>
+__device__ __forceinline__ double wide_J(const OcArgs<double>& a, int row) {
+  if constexpr (FORM == kFormTable)
+    if (a.juni) return a.jval;
+  return __ldg(a.J + row);
+}
+
+template <int FORM>
+__global__ void __launch_bounds__(kOcThreads, 1) pcg_wide_kernel(WideArgs wa) {
+  const OcArgs<double>& a = wa.o;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ double part[2][kWideTiles][8];
+  __shared__ double red[16];
+  __shared__ int abort_;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = tid >> 8, w = warp & 7;
+  const int nt = a.ntiles, per = wa.per;
+  const int t0 = blockIdx.x == 0 ? 0 : (int)blockIdx.x * per - kWideLess;
+  const int T = max(0, min(blockIdx.x == 0 ? per - kWideLess : per, nt - t0));
+  int* s_pat = reinterpret_cast<int*>(smem);
+  int* s_len = s_pat + a.pat_ints;
+  double* s_r = reinterpret_cast<double*>(smem + wide_table_bytes(a.pat_ints));
+  double* s_p = s_r + (size_t)(blockIdx.x == 0 ? per - kWideLess : per) * kTile;
+  double* s_tp = s_r + (size_t)2 * (per - kWideLess) * kTile;  // CTA 0
+  if (tid == 0) abort_ = 0;
+  for (int q = tid; q < a.pat_ints; q += kOcThreads) s_pat[q] = a.pat[q];
+  for (int q = tid; q < a.pat_ints / kPatLen; q += kOcThreads) s_len[q] = a.plen[q];
+  __syncthreads();
+  auto slots = [&](int set) { return a.slot + (size_t)set * nt; };
+  OcSmem<double> ex(nullptr, 0, 0, 0, 0);  // grid_exchange wants the flag only
+  ex.abort_ = &abort_;
+  unsigned epoch = 1;
+
+  // the tile sums of NR warp sums per tile in part[], published
+  auto publish_tiles = [&](auto nr, int set) {
+    constexpr int NR = decltype(nr)::value;
+    __syncthreads();
+    for (int q = tid; q < NR * T; q += kOcThreads) {
+      const int r = q / T, l = q % T;
+      double f = part[r][l][0];
+#pragma unroll
+      for (int g = 1; g < 8; ++g) f = dadd(f, part[r][l][g]);
+      publish(slots(set + r) + t0 + l, f);
+    }
+  };
+  // grid_sum over tile sums
+  auto sum = [&](auto nr, int set, double* tot) {
+    constexpr int NR = decltype(nr)::value;
+    if (blockIdx.x == 0) {
+      const double* q = slots(set);
+      unsigned long long v[kWidePolls], c0 = 0;
+      for (unsigned i = 0;; ++i) {
+        bool ok = true;
+#pragma unroll
+        for (int u = 0; u < kWidePolls; ++u) {
+          const int k = tid + u * kOcThreads;
+          if (k < NR * nt) {
+            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v[u]) : "l"(q + k) : "memory");
+            ok = ok && v[u] != kSentinel;
+          }
+        }
+        if (ok || !poll_more(i, c0, &abort_)) break;
+      }
+#pragma unroll
+      for (int u = 0; u < kWidePolls; ++u)
+        if (tid + u * kOcThreads < NR * nt) s_tp[tid + u * kOcThreads] = __longlong_as_double((long long)v[u]);
+      __syncthreads();
+      if (warp < 8 * NR) {
+        const double* tp = s_tp + (warp >> 3) * nt;
+        double s = 0.0;
+        for (int k = (warp & 7) * 32 + lane; k < nt; k += kLanes) s = dadd(s, tp[k]);
+        s = warp_fold(s);
+        if (lane == 0) red[warp] = s;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        tot[r] = red[8 * r];
+#pragma unroll
+        for (int g = 1; g < 8; ++g) tot[r] = dadd(tot[r], red[8 * r + g]);
+      }
+      if (tid < NR) publish(a.total + set + tid, tid ? tot[NR - 1] : tot[0]);
+      __syncthreads();
+    } else {
+      if (tid == 0) {
+        unsigned long long c0 = 0, w0, w1 = 0;
+        for (unsigned i = 0;; ++i) {
+          if constexpr (NR == 2) load2(a.total + set, w0, w1);
+          else asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w0) : "l"(a.total + set) : "memory");
+          if ((w0 != kSentinel && w1 != kSentinel) || !poll_more(i, c0, &abort_)) break;
+        }
+        red[0] = __longlong_as_double((long long)w0);
+        red[1] = __longlong_as_double((long long)w1);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < NR; ++r) tot[r] = red[r];
+      __syncthreads();
+    }
+  };
+  using One = std::integral_constant<int, 1>;
+  using Two = std::integral_constant<int, 2>;
+  double tot[2];
+
+  // ---- x0, ||b|| ------------------------------------------------------------
+  for (int l = half; l < T; l += 2) {
+    double acc = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int row = (t0 + l) * kTile + k * kLanes + w * 32 + lane;
+      const int i = l * kTile + k * kLanes + w * 32 + lane;
+      s_r[i] = s_p[i] = 0.0;
+      if (row < a.n) {
+        const double bi = a.b[row];
+        acc = dadd(acc, dmul(bi, bi));
+        if (a.x0_mode != CELG_X0_USER) a.x[row] = a.x0_mode == CELG_X0_REF_ONES ? 1.0 : 0.0;
+      }
+    }
+    acc = warp_fold(acc);
+    if (lane == 0) part[0][l][w] = acc;
+  }
+  publish_tiles(One(), kSlotB);
+  grid_exchange(a, ex, epoch++);
+  sum(One(), kSlotB, tot);
+  const double bnorm = sqrt(tot[0]);
+  double eps = a.eps_abs;
+  if (a.eps_rel > 0.0 && a.eps_rel * bnorm > eps) eps = a.eps_rel * bnorm;
+
+  // ---- r = b - A x, p = J r -------------------------------------------------
+  for (int l = half; l < T; l += 2) {
+    double rp = 0.0, rr = 0.0;
+    for (int k = 0; k < 4; ++k) {
+      const int row = (t0 + l) * kTile + k * kLanes + w * 32 + lane;
+      const int i = l * kTile + k * kLanes + w * 32 + lane;
+      if (row < a.n) {
+        const double s = wide_row_sum<FORM>(a, s_pat, s_len, a.x, row, lane, FORM == kFormCols ? 0 : (int)__ldg(a.pid + row));
+        const double ri = __dsub_rn(a.b[row], dadd(0.0, s));
+        const double z = dmul(ri, wide_J<FORM>(a, row));
+        s_r[i] = ri;
+        s_p[i] = z;
+        a.p[row] = z;
+        rp = dadd(rp, dmul(ri, z));
+        rr = dadd(rr, dmul(ri, ri));
+      }
+    }
+    rp = warp_fold(rp);
+    rr = warp_fold(rr);
+    if (lane == 0) {
+      part[0][l][w] = rp;
+      part[1][l][w] = rr;
+    }
+  }
+  publish_tiles(Two(), kSlotInit);
+  grid_exchange(a, ex, epoch++);
+  sum(Two(), kSlotInit, tot);
+  double alpha = tot[0], norm = sqrt(tot[1]), sigma = 0.0, beta = 0.0, pvd = 0.0, rz = 0.0;
+  int iter = 0, err = 0;
+  const bool scribe = blockIdx.x == 0 && tid == 0;
+  if (scribe && a.hist && a.hist_cap > 0) a.hist[0] = norm;
+  bool act = iter < a.iter_max && fabs(alpha) > kRealSmall && norm > eps;
+  int stop = *(volatile int*)&abort_;
+
+  while (act && !stop) {
+    // v = A p, p.v; the pattern bytes come a tile ahead
+    int id[4];
+    auto ids = [&](int l) {
+      if constexpr (FORM != kFormCols)
+        if (l < T)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            id[k] = (int)__ldg(a.pid + min((t0 + l) * kTile + k * kLanes + w * 32 + lane, a.n - 1));
+    };
+    ids(half);
+    for (int l = half; l < T; l += 2) {
+      double acc = 0.0;
+      const int now[4] = {id[0], id[1], id[2], id[3]};
+      ids(l + 2);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int row = (t0 + l) * kTile + k * kLanes + w * 32 + lane;
+        if (row < a.n) {
+          const double vi = dadd(0.0, wide_row_sum<FORM>(a, s_pat, s_len, a.p, row, lane, now[k]));
+          wa.v[row] = vi;
+          acc = dadd(acc, dmul(vi, s_p[l * kTile + k * kLanes + w * 32 + lane]));
+        }
+      }
+      acc = warp_fold(acc);
+      if (lane == 0) part[0][l][w] = acc;
+    }
+    publish_tiles(One(), kSlotPv);
+    sum(One(), kSlotPv, tot);
+    pvd = tot[0];
+    sigma = alpha / pvd;
+    if (!isfinite(sigma)) {
+      err = kErrBreakdown;
+      act = false;
+      break;
+    }
+    // r += (-sigma) v, r.z, r.r
+    const int us = (iter & 1) ? kSlotUpd1 : kSlotUpd0, uo = (iter & 1) ? kSlotUpd0 : kSlotUpd1;
+    for (int l = half; l < T; l += 2) {
+      double f0 = 0.0, f1 = 0.0, v[4], J[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int row = (t0 + l) * kTile + k * kLanes + w * 32 + lane;
+        v[k] = row < a.n ? wa.v[row] : 0.0;
+        J[k] = row < a.n ? wide_J<FORM>(a, row) : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int i = l * kTile + k * kLanes + w * 32 + lane;
+        const double ri = dadd(s_r[i], dmul(-sigma, v[k]));
+        s_r[i] = ri;
+        const double z = dmul(ri, J[k]);
+        f0 = dadd(f0, dmul(ri, z));
+        f1 = dadd(f1, dmul(ri, ri));
+      }
+      f0 = warp_fold(f0);
+      f1 = warp_fold(f1);
+      if (lane == 0) {
+        part[0][l][w] = f0;
+        part[1][l][w] = f1;
+      }
+    }
+    publish_tiles(Two(), us);
+    sum(Two(), us, tot);
+    rz = tot[0];
+    beta = rz / alpha;
+    alpha = rz;
+    norm = sqrt(tot[1]);
+    ++iter;
+    if (scribe && a.hist && iter < a.hist_cap) a.hist[iter] = norm;
+    act = iter < a.iter_max && fabs(alpha) > kRealSmall && norm > eps;
+    // x += sigma p, p = beta p + J r; slots back to the sentinel as in
+    // pcg_onchip_kernel
+    for (int l = half; l < T; l += 2) {
+      double x[4], J[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int row = (t0 + l) * kTile + k * kLanes + w * 32 + lane;
+        x[k] = row < a.n ? a.x[row] : 0.0;
+        J[k] = row < a.n ? wide_J<FORM>(a, row) : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int row = (t0 + l) * kTile + k * kLanes + w * 32 + lane;
+        const int i = l * kTile + k * kLanes + w * 32 + lane;
+        if (row < a.n) {
+          const double pi = s_p[i];
+          a.x[row] = dadd(x[k], dmul(sigma, pi));
+          if (act) {
+            const double pn = dadd(dmul(beta, pi), dmul(s_r[i], J[k]));
+            s_p[i] = pn;
+            a.p[row] = pn;
+          }
+        }
+      }
+    }
+    for (int q = tid; q < 3 * T; q += kOcThreads) {
+      const int r = q / T;
+      *reinterpret_cast<unsigned long long*>(slots(r == 0 ? kSlotPv : uo + r - 1) + t0 + q % T) = kSentinel;
+    }
+    if (blockIdx.x == 0 && tid < 3)
+      *reinterpret_cast<unsigned long long*>(a.total + (tid == 0 ? kSlotPv : uo + tid - 1)) = kSentinel;
+    stop = *(volatile int*)&abort_;
+    if (act) {
+      grid_exchange(a, ex, epoch++);
+      stop = *(volatile int*)&abort_;
+    }
+  }
+
+  // ---- ||b - A x|| -------------------------------------------------------------
+  double vres = 0.0;
+  if (a.verify && !stop) {
+    grid_exchange(a, ex, epoch++);
+    for (int l = half; l < T; l += 2) {
+      double acc = 0.0;
+      for (int k = 0; k < 4; ++k) {
+        const int row = (t0 + l) * kTile + k * kLanes + w * 32 + lane;
+        if (row < a.n) {
+          const double ri = __dsub_rn(a.b[row], dadd(0.0, wide_row_sum<FORM>(a, s_pat, s_len, a.x, row, lane, FORM == kFormCols ? 0 : (int)__ldg(a.pid + row))));
+          acc = dadd(acc, dmul(ri, ri));
+        }
+      }
+      acc = warp_fold(acc);
+      if (lane == 0) part[0][l][w] = acc;
+    }
+    publish_tiles(One(), kSlotVer);
+    sum(One(), kSlotVer, tot);
+    vres = bnorm > 0.0 ? sqrt(tot[0]) / bnorm : sqrt(tot[0]);
+  }
+  if (scribe) {
+    PcgState* o = a.out;
+    o->alpha = alpha;
+    o->sigma = sigma;
+    o->beta = beta;
+    o->norm = norm;
+    o->bnorm = bnorm;
+    o->eps = eps;
+    o->pvd = pvd;
+    o->rz = rz;
+    o->vres = vres;
+    o->iter = iter;
+    o->active = act ? 1 : 0;
+    o->err = *(volatile int*)&abort_ ? kErrTimeout : err;
+    o->hist_len = iter + 1;
+    o->xpend = o->xprev = 0;
+    o->sigprev = 0.0;
+  }
+}
+
 // ---- sliced matrix copy -----------------------------------------------------------
 
 // longest row of each slice of 32 rows, and of the matrix
@@ -666,6 +1071,22 @@ static int launch_onchip(celg_handle* h, const OcArgs<VT>& a, int grid, size_t s
   return CELG_OK;
 }
 
+template <int FORM>
+static int launch_wide(celg_handle* h, const OcArgs<double>& o, double* v, int per, int grid, size_t smem, bool* done) {
+  if (const int st = allow_dynamic_smem<pcg_wide_kernel<FORM>>((int)smem)) return st;
+  WideArgs arg{o, v, per};
+  void* params[] = {&arg};
+  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)pcg_wide_kernel<FORM>, dim3(grid), dim3(kOcThreads),
+                                                    params, smem, h->stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    (void)cudaGetLastError();
+    return CELG_OK;
+  }
+  CELG_CUDA(e);
+  *done = true;
+  return CELG_OK;
+}
+
 template <typename VT>
 int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_params* p, int hist_cap, bool* done) {
   *done = false;
@@ -678,14 +1099,24 @@ int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_param
   const bool pat = A.pid != nullptr;
   const int pat_ints = pat ? A.npat * kPatLen : 0;
   const size_t base = OcSmem<VT>(nullptr, (int)nt, pat_ints, slots, 0).bytes;
-  if (base > (size_t)kOcMaxSmem) return CELG_OK;
+  // the wide form, where r and p fit
+  const int per = (int)((nt + kWideLess + h->sms - 1) / h->sms);
+  const bool wide = base > (size_t)kOcMaxSmem;
+  if (wide && (sizeof(VT) != 8 || per > kWideTiles || per <= kWideLess || 2 * nt > kWidePolls * kOcThreads ||
+               2 * nt * 8 > 2 * kWideLess * kTile * 8 ||
+               wide_table_bytes(pat_ints) + 2 * per * kTile * 8 + kWideStatic > kOcMaxSmem))
+    return CELG_OK;
   const size_t per_cached = sizeof(VT) * kUnitRows * kPatLen;
-  const int ncache = pat ? (int)std::min<size_t>((size_t)slots, (kOcMaxSmem - base) / per_cached) : 0;
-  const size_t smem = OcSmem<VT>(nullptr, (int)nt, pat_ints, slots, ncache).bytes;
-  bool ok = false;
-  int st = ensure_sell<VT>(h, A, B.vals, &ok);
-  if (st || !ok) return st;
-  const size_t nslot = (size_t)kSlotSets * nunits;
+  const int ncache = pat && !wide ? (int)std::min<size_t>((size_t)slots, (kOcMaxSmem - base) / per_cached) : 0;
+  const size_t smem = wide ? wide_table_bytes(pat_ints) + (size_t)2 * per * kTile * 8
+                           : OcSmem<VT>(nullptr, (int)nt, pat_ints, slots, ncache).bytes;
+  const VT* rowv = wide ? row_values<VT>(A) : nullptr;
+  if (!rowv) {
+    bool ok = false;
+    const int st = ensure_sell<VT>(h, A, B.vals, &ok);
+    if (st || !ok) return st;
+  }
+  const size_t nslot = (size_t)kSlotSets * (wide ? nt + (nt & 1) : nunits);
   if (nslot > h->oc_cap) {
     CELG_CUDA(cudaStreamSynchronize(h->stream));
     cudaFree(h->oc_slots);
@@ -706,6 +1137,10 @@ int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_param
   a.pid = A.pid;
   a.pat = A.pat;
   a.pat_ints = pat_ints;
+  a.plen = A.plen;
+  a.rowv = rowv;
+  a.juni = B.juni;
+  a.jval = B.jval;
   a.b = B.b;
   a.x = B.x;
   a.J = B.J;
@@ -722,6 +1157,14 @@ int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_param
   a.eps_abs = p->eps_abs;
   a.eps_rel = p->eps_rel;
   CELG_CUDA(cudaMemsetAsync(h->oc_slots, 0xff, sizeof(double) * (nslot + kOcTail), h->stream));
+  if constexpr (sizeof(VT) == 8) {
+    if (wide) {
+      const int wgrid = (int)((nt + kWideLess + per - 1) / per);
+      if (rowv) return launch_wide<kFormTable>(h, a, B.v, per, wgrid, smem, done);
+      return pat ? launch_wide<kFormPat>(h, a, B.v, per, wgrid, smem, done)
+                 : launch_wide<kFormCols>(h, a, B.v, per, wgrid, smem, done);
+    }
+  }
   return pat ? launch_onchip<VT, true>(h, a, grid, smem, done) : launch_onchip<VT, false>(h, a, grid, smem, done);
 }
 

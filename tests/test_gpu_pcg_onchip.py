@@ -22,6 +22,20 @@ def rand(n, **kw):
     return spd_from_pattern(*random_csr(n, np.random.default_rng(n), **kw))
 
 
+def wide_band(n):
+    """Symmetric, diagonally dominant, 1 to 5 entries a row, no row patterns."""
+    i = np.arange(n - 700)
+    i = i[np.random.default_rng(1).random(i.size) < 0.8]
+    j = i + 1 + (i * 2654435761) % 600
+    u = 0.5 + np.random.default_rng(2).random(i.size)
+    import scipy.sparse as sp
+    A = sp.coo_matrix((u, (i, j)), shape=(n, n))
+    A = A + A.T
+    A = (sp.diags(np.asarray(A.sum(axis=1)).ravel() + 0.1) - A).tocsr()
+    A.sort_indices()
+    return A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
+
+
 CASES = {
     "one_row": lambda: grid(1, 1, 1),
     "31_rows": lambda: grid(31, 1, 1),
@@ -29,6 +43,11 @@ CASES = {
     "one_tile": lambda: grid(16, 8, 8),
     "tile_and_a_row": lambda: grid(41, 25, 1),
     "values_partly_cached": lambda: grid(75, 70, 64),
+    "wide_few_tiles": lambda: grid(95, 90, 89),
+    "wide_ragged": lambda: grid(113, 112, 111),
+    "wide_most_tiles": lambda: grid(128, 128, 128),
+    "wide_uneven_rows": lambda: wide_band(760003),
+    "too_many_rows": lambda: grid(131, 129, 127),
     "uneven_rows": lambda: rand(1023, max_len=9),
     "uneven_rows_many_units": lambda: rand(20011, max_len=12),
     "some_long_rows": lambda: rand(4099, max_len=5, long_rows=40, long_len=300),
@@ -52,8 +71,9 @@ def test_onchip_equals_graph_and_oracle(gpu, name, monkeypatch):
     b, x0 = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
     bd = torch.from_numpy(b).cuda()
     m = h.matrix_from_csr(rp, ci, v).jacobi()
-    runs = [dict(x0_mode=celgpu.X0_ZERO, eps_rel=1e-9, iter_max=2000), dict(x0_mode=celgpu.X0_USER, iter_max=3),
-            dict(x0_mode=celgpu.X0_REF_ONES, eps_rel=0.0, eps_abs=1e-3, iter_max=2000), dict(iter_max=0)]
+    cap = 2000 if n < 500000 else 25
+    runs = [dict(x0_mode=celgpu.X0_ZERO, eps_rel=1e-9, iter_max=cap), dict(x0_mode=celgpu.X0_USER, iter_max=3),
+            dict(x0_mode=celgpu.X0_REF_ONES, eps_rel=0.0, eps_abs=1e-3, iter_max=cap), dict(iter_max=0)]
     if n < 5000:
         runs.append(dict(precision=celgpu.PREC_FP32_IR, eps_rel=1e-9, inner_eps_rel=1e-3))
     for kw in runs:
@@ -65,7 +85,7 @@ def test_onchip_equals_graph_and_oracle(gpu, name, monkeypatch):
             assert np.array_equal(xg, xo) and np.array_equal(ig.history, io.history)
             for f in ("iter_done", "status", "final_norm2", "bnorm", "verified_relres", "arnoldi_steps"):
                 assert io[f] == ig[f], f
-    xr, ir = R.pcg_jacobi(R.Matrix(rp, ci, v), R.jacobi(R.diag(rp, ci, v)), b, eps_rel=1e-9, iter_max=2000,
+    xr, ir = R.pcg_jacobi(R.Matrix(rp, ci, v), R.jacobi(R.diag(rp, ci, v)), b, eps_rel=1e-9, iter_max=cap,
                           red=R.RED_TREE)
     x, i = solve(celgpu, h, torch, m, bd, x0, **runs[0])
     assert i.iter_done == ir["iter_done"] and np.array_equal(x, xr)

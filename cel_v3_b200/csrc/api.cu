@@ -521,6 +521,12 @@ extern "C" int celg_destroy(celg_handle* h) {
   cudaFreeHost(h->ru_state_h);
   cudaFree(h->hist_d);
   cudaFree(h->oc_slots);
+  cudaFree(h->oc_work);
+  cudaFreeHost(h->oc_states);
+  for (int l = 0; l < 8; ++l) {
+    if (h->oc_lane[l]) cudaStreamDestroy(h->oc_lane[l]);
+    if (h->oc_event[l]) cudaEventDestroy(h->oc_event[l]);
+  }
   cudaFree(h->gm_work);
   cudaFree(h->gm_state_d);
   cudaFree(h->gm_exch);

@@ -1177,11 +1177,64 @@ static int pcg_batched_ir(celg_handle* h, int count, celg_mat* const* mats, cons
 static int pcg_batched_ru(celg_handle* h, int count, celg_mat* const* mats, const double* const* b_d,
                           double* const* x_d, const celg_params* p, celg_result* res);
 
+// Every system in a kernel of its own (pcg_onchip.cu); *done is false when
+// one of them does not fit, the caller asked for a launch shape of the common
+// sweeps, or graphs are off.
+static int pcg_batched_onchip(celg_handle* h, int count, celg_mat* const* mats, const double* const* b_d,
+                              double* const* x_d, const celg_params* p, celg_result* res, bool* done) {
+  *done = false;
+  if (!graphs_enabled() || std::getenv("CELG_BATCH_SHAPE") || p->iter_max < 0) return CELG_OK;
+  for (int s = 0; s < count; ++s) {
+    if (!mats[s] || !mats[s]->jacobi || mats[s]->h != h) return CELG_ERR_ARG;
+    if (mats[s]->csr.n > 0 && (!b_d[s] || !x_d[s])) return CELG_ERR_ARG;
+  }
+  const PcgState* states = nullptr;
+  CELG_CUDA(cudaEventRecord(h->ev0, h->stream));
+  const int st = pcg_onchip_many(h, count, mats, b_d, x_d, p, &states, done);
+  if (st || !*done) return st;
+  CELG_CUDA(cudaEventRecord(h->ev1, h->stream));
+  CELG_CUDA(cudaStreamSynchronize(h->stream));
+  cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1);
+  int ret = CELG_OK, iters = 0;
+  for (int s = 0; s < count; ++s) {
+    if (mats[s]->csr.n == 0) {
+      if (res) {
+        std::memset(&res[s], 0, offsetof(celg_result, history));
+        res[s].history_len = 0;
+      }
+      continue;
+    }
+    const PcgState& q = states[s];
+    int rs = CELG_OK;
+    if (q.err) rs = q.err;
+    else if (!(q.norm <= q.eps) && q.iter >= p->iter_max && std::fabs(q.alpha) > kRealSmall) rs = CELG_ERR_NOCONV;
+    if (rs && !ret) ret = rs;
+    iters = std::max(iters, q.iter);
+    if (res) {
+      res[s].iter_done = q.iter;
+      res[s].final_norm2 = q.norm;
+      res[s].bnorm = q.bnorm;
+      res[s].verified_relres = q.vres;
+      res[s].err = rs;
+      res[s].arnoldi_steps = 0;
+      res[s].history_len = 0;
+    }
+  }
+  h->last_iters = iters;
+  return ret;
+}
+
 int pcg_batched(celg_handle* h, int count, celg_mat* const* mats, const double* const* b_d,
                 double* const* x_d, const celg_params* p, celg_result* res) {
   if (p->precision == CELG_PREC_FP32_IR) return pcg_batched_ir(h, count, mats, b_d, x_d, p, res);
   if (p->precision == CELG_PREC_FP32_RU) return pcg_batched_ru(h, count, mats, b_d, x_d, p, res);
   if (p->precision != CELG_PREC_FP64) return CELG_ERR_ARG;
+  {
+    bool done = false;
+    const int ret = pcg_batched_onchip(h, count, mats, b_d, x_d, p, res, &done);
+    h->batch_onchip = done;
+    if (ret || done) return ret;
+  }
   Batch* bt = nullptr;
   int st = batch_for(h, count, mats, b_d, x_d, &bt);
   if (st) return st;
@@ -1644,8 +1697,9 @@ extern "C" int celg_tuned_config(celg_handle* h, int what, int out[2]) {
   if (!h || !out) return CELG_ERR_ARG;
   out[0] = out[1] = -1;
   if (what == CELG_TUNE_BATCH) {
-    if (!h->batch || h->batch->shape < 0) return CELG_ERR_STATE;
-    const celg::BatchShape sh = celg::kBatchShapes[h->batch->shape];
+    if (!h->batch_onchip && (!h->batch || h->batch->shape < 0)) return CELG_ERR_STATE;
+    // (systems solved in kernels of their own leave the first shape: nothing to tune)
+    const celg::BatchShape sh = celg::kBatchShapes[h->batch_onchip ? 0 : h->batch->shape];
     out[0] = sh.csr_per_sm;
     out[1] = sh.tile_per_sm;
     return CELG_OK;

@@ -120,9 +120,18 @@ struct celg_handle {
   std::vector<celg::GraphEntry> graphs;
   double* hist_d = nullptr;
   int hist_cap = 0;
-  // exchange slots of the one-kernel solve (oc_cap doubles and a tail)
+  // exchange slots of the one-kernel solve (oc_cap doubles)
   double* oc_slots = nullptr;
   size_t oc_cap = 0;
+  // the same for many systems side by side: work vectors, pinned states, and
+  // the streams and events of its lanes (lane 0 is the handle's stream)
+  double* oc_work = nullptr;
+  size_t oc_work_cap = 0;
+  celg::PcgState* oc_states = nullptr;
+  int oc_states_cap = 0;
+  cudaStream_t oc_lane[8] = {};
+  cudaEvent_t oc_event[8] = {};
+  bool batch_onchip = false;  // the last batched FP64 solve ran that way
   // host-buffer solve staging (stable pointers keep cached graphs valid)
   double* sb = nullptr;
   double* sx = nullptr;

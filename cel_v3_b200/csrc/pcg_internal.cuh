@@ -92,6 +92,10 @@ int pcg_run(celg_handle* h, const PcgBind<VT>& B, const celg_params* p, const vo
 template <typename VT>
 int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_params* p, int hist_cap,
                bool* done);
+// the same for `count` systems at once (each its own kernel, empty ones left
+// out); their states, in pinned memory, are complete once h->stream is
+int pcg_onchip_many(celg_handle* h, int count, celg_mat* const* mats, const double* const* b, double* const* x,
+                    const celg_params* p, const PcgState** states, bool* done);
 int copy_history(celg_handle* h, int len, celg_result* res);
 
 template <typename VT>

@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(kOcThreads, 1) pcg_onchip_kernel(OcArgs<VT> a)
 // the values, the gathers, v, J (twice) and x.  A CTA has whole tiles, its
 // two halves alternate between them (warp w of a half has the tile's rows 32
 // w + lane + 256 k), and it publishes tile sums; CTA 0, which folds them all,
-// has kWideLess tiles less and their room for the sums.
+// has kWideLess tiles less and their room for the sums where both do not fit.
 // us an iteration, sweeps : this kernel (variable coefficients, FP64): 90^3
 // 34.8 : 21.9, 104^3 41.3 : 27.0, 120^3 54.8 : 38.4, 128^3 61.3 : 51.5 (the
 // working set leaves L2); constant coefficients 128^3 43.8 : 32.9.
@@ -555,6 +555,7 @@ struct WideArgs {
   OcArgs<double> o;  // slot: kSlotSets x ntiles
   double* v;
   int per;           // tiles of a CTA
+  int less;          // of them CTA 0 has not: 0 or kWideLess
 };
 
 __host__ __device__ inline int wide_table_bytes(int pat_ints) {
@@ -641,13 +642,14 @@ __global__ void __launch_bounds__(kOcThreads, 1) pcg_wide_kernel(WideArgs wa) {
   __shared__ int abort_;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = tid >> 8, w = warp & 7;
   const int nt = a.ntiles, per = wa.per;
-  const int t0 = blockIdx.x == 0 ? 0 : (int)blockIdx.x * per - kWideLess;
-  const int T = max(0, min(blockIdx.x == 0 ? per - kWideLess : per, nt - t0));
+  const int own = blockIdx.x == 0 ? per - wa.less : per;
+  const int t0 = blockIdx.x == 0 ? 0 : (int)blockIdx.x * per - wa.less;
+  const int T = max(0, min(own, nt - t0));
   int* s_pat = reinterpret_cast<int*>(smem);
   int* s_len = s_pat + a.pat_ints;
   double* s_r = reinterpret_cast<double*>(smem + wide_table_bytes(a.pat_ints));
-  double* s_p = s_r + (size_t)(blockIdx.x == 0 ? per - kWideLess : per) * kTile;
-  double* s_tp = s_r + (size_t)2 * (per - kWideLess) * kTile;  // CTA 0
+  double* s_p = s_r + (size_t)own * kTile;
+  double* s_tp = s_r + (size_t)2 * own * kTile;  // CTA 0
   if (tid == 0) abort_ = 0;
   for (int q = tid; q < a.pat_ints; q += kOcThreads) s_pat[q] = a.pat[q];
   for (int q = tid; q < a.pat_ints / kPatLen; q += kOcThreads) s_len[q] = a.plen[q];
@@ -1056,12 +1058,12 @@ static long onchip_max_rows() {
 // *done stays false when the device cannot hold the grid at once (fewer SMs
 // at this process's disposal than the device has).
 template <typename VT, bool PAT>
-static int launch_onchip(celg_handle* h, const OcArgs<VT>& a, int grid, size_t smem, bool* done) {
+static int launch_onchip(cudaStream_t stream, const OcArgs<VT>& a, int grid, size_t smem, bool* done) {
   if (const int st = allow_dynamic_smem<pcg_onchip_kernel<VT, PAT>>((int)smem)) return st;
   OcArgs<VT> arg = a;
   void* params[] = {&arg};
   const cudaError_t e = cudaLaunchCooperativeKernel((const void*)pcg_onchip_kernel<VT, PAT>, dim3(grid),
-                                                    dim3(kOcThreads), params, smem, h->stream);
+                                                    dim3(kOcThreads), params, smem, stream);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     (void)cudaGetLastError();
     return CELG_OK;
@@ -1072,12 +1074,13 @@ static int launch_onchip(celg_handle* h, const OcArgs<VT>& a, int grid, size_t s
 }
 
 template <int FORM>
-static int launch_wide(celg_handle* h, const OcArgs<double>& o, double* v, int per, int grid, size_t smem, bool* done) {
+static int launch_wide(cudaStream_t stream, const OcArgs<double>& o, double* v, int per, int less, int grid, size_t smem,
+                       bool* done) {
   if (const int st = allow_dynamic_smem<pcg_wide_kernel<FORM>>((int)smem)) return st;
-  WideArgs arg{o, v, per};
+  WideArgs arg{o, v, per, less};
   void* params[] = {&arg};
   const cudaError_t e = cudaLaunchCooperativeKernel((const void*)pcg_wide_kernel<FORM>, dim3(grid), dim3(kOcThreads),
-                                                    params, smem, h->stream);
+                                                    params, smem, stream);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     (void)cudaGetLastError();
     return CELG_OK;
@@ -1087,85 +1090,259 @@ static int launch_wide(celg_handle* h, const OcArgs<double>& o, double* v, int p
   return CELG_OK;
 }
 
+// How a system runs on `sms` SMs, and the doubles of exchange words it needs.
+struct OnchipPlan {
+  bool wide = false;
+  int slots = 0, grid = 0, per = 0, less = 0, ncache = 0;
+  size_t smem = 0, nslot = 0;
+  size_t words() const { return nslot + (nslot & 1) + kOcTail; }
+};
+
+// false: the system does not fit
 template <typename VT>
-int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_params* p, int hist_cap, bool* done) {
-  *done = false;
+static bool onchip_plan(const CsrDev& A, int sms, OnchipPlan* out) {
   const long n = A.n;
-  if (n < 1 || n > onchip_max_rows()) return CELG_OK;
+  if (n < 1 || n > onchip_max_rows()) return false;
   const long nt = ntiles_of(n), nunits = nt * 8;
-  if (nunits > kOcMaxUnits) return CELG_OK;
-  const int slots = (int)((nunits + h->sms - 1) / h->sms);
-  const int grid = (int)((nunits + slots - 1) / slots);
+  if (nunits > kOcMaxUnits) return false;
+  OnchipPlan q;
+  q.slots = (int)((nunits + sms - 1) / sms);
+  q.grid = (int)((nunits + q.slots - 1) / q.slots);
   const bool pat = A.pid != nullptr;
   const int pat_ints = pat ? A.npat * kPatLen : 0;
-  const size_t base = OcSmem<VT>(nullptr, (int)nt, pat_ints, slots, 0).bytes;
+  const size_t base = OcSmem<VT>(nullptr, (int)nt, pat_ints, q.slots, 0).bytes;
   // the wide form, where r and p fit
-  const int per = (int)((nt + kWideLess + h->sms - 1) / h->sms);
-  const bool wide = base > (size_t)kOcMaxSmem;
-  if (wide && (sizeof(VT) != 8 || per > kWideTiles || per <= kWideLess || 2 * nt > kWidePolls * kOcThreads ||
-               2 * nt * 8 > 2 * kWideLess * kTile * 8 ||
-               wide_table_bytes(pat_ints) + 2 * per * kTile * 8 + kWideStatic > kOcMaxSmem))
-    return CELG_OK;
-  const size_t per_cached = sizeof(VT) * kUnitRows * kPatLen;
-  const int ncache = pat && !wide ? (int)std::min<size_t>((size_t)slots, (kOcMaxSmem - base) / per_cached) : 0;
-  const size_t smem = wide ? wide_table_bytes(pat_ints) + (size_t)2 * per * kTile * 8
-                           : OcSmem<VT>(nullptr, (int)nt, pat_ints, slots, ncache).bytes;
-  const VT* rowv = wide ? row_values<VT>(A) : nullptr;
-  if (!rowv) {
-    bool ok = false;
-    const int st = ensure_sell<VT>(h, A, B.vals, &ok);
-    if (st || !ok) return st;
+  q.wide = base > (size_t)kOcMaxSmem;
+  if (q.wide) {
+    if (sizeof(VT) != 8 || 2 * nt > kWidePolls * kOcThreads) return false;
+    // CTA 0's room for the sums: beside its tiles, else in place of some
+    for (q.less = 0;; q.less = kWideLess) {
+      q.per = (int)((nt + q.less + sms - 1) / sms);
+      q.smem = wide_table_bytes(pat_ints) + (size_t)2 * q.per * kTile * 8 + (q.less ? 0 : 2 * nt * 8);
+      if (q.per <= kWideTiles && q.per > q.less && q.smem + kWideStatic <= (size_t)kOcMaxSmem) break;
+      if (q.less) return false;
+    }
+    q.grid = (int)((nt + q.less + q.per - 1) / q.per);
+    q.nslot = (size_t)kSlotSets * (nt + (nt & 1));
+  } else {
+    const size_t per_cached = sizeof(VT) * kUnitRows * kPatLen;
+    q.ncache = pat ? (int)std::min<size_t>((size_t)q.slots, (kOcMaxSmem - base) / per_cached) : 0;
+    q.smem = OcSmem<VT>(nullptr, (int)nt, pat_ints, q.slots, q.ncache).bytes;
+    q.nslot = (size_t)kSlotSets * nunits;
   }
-  const size_t nslot = (size_t)kSlotSets * (wide ? nt + (nt & 1) : nunits);
-  if (nslot > h->oc_cap) {
-    CELG_CUDA(cudaStreamSynchronize(h->stream));
-    cudaFree(h->oc_slots);
-    h->oc_slots = nullptr;
-    h->oc_cap = 0;
-    CELG_CUDA(cudaMalloc(&h->oc_slots, sizeof(double) * (nslot + kOcTail)));
-    h->oc_cap = nslot;
-  }
+  *out = q;
+  return true;
+}
+
+// the sliced values, where the kernel reads them
+template <typename VT>
+static int onchip_matrix(celg_handle* h, CsrDev& A, const VT* vals, const OnchipPlan& q, bool* ok) {
+  *ok = q.wide && row_values<VT>(A);
+  return *ok ? CELG_OK : ensure_sell<VT>(h, A, vals, ok);
+}
+
+// words: q.words() doubles set to 0xff
+template <typename VT>
+static int onchip_launch(cudaStream_t stream, CsrDev& A, const PcgBind<VT>& B, const celg_params* p, const OnchipPlan& q,
+                         double* words, PcgState* out, double* hist, int hist_cap, bool* done) {
   OcArgs<VT> a;
-  a.n = (int)n;
-  a.ntiles = (int)nt;
-  a.slots = slots;
-  a.ncache = ncache;
+  a.n = A.n;
+  a.ntiles = (int)ntiles_of(A.n);
+  a.slots = q.slots;
+  a.ncache = q.ncache;
   a.sv = sell_vals(A, B.vals);
   a.sc = A.sell_c;
   a.sbase = A.sell_base;
   a.rp = A.rp;
   a.pid = A.pid;
   a.pat = A.pat;
-  a.pat_ints = pat_ints;
+  a.pat_ints = A.pid ? A.npat * kPatLen : 0;
   a.plen = A.plen;
-  a.rowv = rowv;
+  a.rowv = q.wide ? row_values<VT>(A) : nullptr;
   a.juni = B.juni;
   a.jval = B.jval;
   a.b = B.b;
   a.x = B.x;
   a.J = B.J;
   a.p = B.p;
-  a.slot = h->oc_slots;
-  a.total = h->oc_slots + (nslot + (nslot & 1));
+  a.slot = words;
+  a.total = words + (q.nslot + (q.nslot & 1));
   a.arrive = reinterpret_cast<unsigned*>(a.total + kSlotSets + 7);
-  a.out = h->state_h;
-  a.hist = h->hist_d;
+  a.out = out;
+  a.hist = hist;
   a.hist_cap = hist_cap;
   a.iter_max = p->iter_max;
   a.x0_mode = p->x0_mode;
   a.verify = B.verify_vals != nullptr;
   a.eps_abs = p->eps_abs;
   a.eps_rel = p->eps_rel;
-  CELG_CUDA(cudaMemsetAsync(h->oc_slots, 0xff, sizeof(double) * (nslot + kOcTail), h->stream));
   if constexpr (sizeof(VT) == 8) {
-    if (wide) {
-      const int wgrid = (int)((nt + kWideLess + per - 1) / per);
-      if (rowv) return launch_wide<kFormTable>(h, a, B.v, per, wgrid, smem, done);
-      return pat ? launch_wide<kFormPat>(h, a, B.v, per, wgrid, smem, done)
-                 : launch_wide<kFormCols>(h, a, B.v, per, wgrid, smem, done);
+    if (q.wide) {
+      if (a.rowv) return launch_wide<kFormTable>(stream, a, B.v, q.per, q.less, q.grid, q.smem, done);
+      return A.pid ? launch_wide<kFormPat>(stream, a, B.v, q.per, q.less, q.grid, q.smem, done)
+                   : launch_wide<kFormCols>(stream, a, B.v, q.per, q.less, q.grid, q.smem, done);
     }
   }
-  return pat ? launch_onchip<VT, true>(h, a, grid, smem, done) : launch_onchip<VT, false>(h, a, grid, smem, done);
+  return A.pid ? launch_onchip<VT, true>(stream, a, q.grid, q.smem, done)
+               : launch_onchip<VT, false>(stream, a, q.grid, q.smem, done);
+}
+
+static int onchip_words(celg_handle* h, size_t words) {
+  if (words > h->oc_cap) {
+    CELG_CUDA(cudaStreamSynchronize(h->stream));
+    cudaFree(h->oc_slots);
+    h->oc_slots = nullptr;
+    h->oc_cap = 0;
+    CELG_CUDA(cudaMalloc(&h->oc_slots, sizeof(double) * words));
+    h->oc_cap = words;
+  }
+  CELG_CUDA(cudaMemsetAsync(h->oc_slots, 0xff, sizeof(double) * words, h->stream));
+  return CELG_OK;
+}
+
+template <typename VT>
+int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_params* p, int hist_cap, bool* done) {
+  *done = false;
+  OnchipPlan q;
+  if (!onchip_plan<VT>(A, h->sms, &q)) return CELG_OK;
+  bool ok = false;
+  int st = onchip_matrix<VT>(h, A, B.vals, q, &ok);
+  if (st || !ok) return st;
+  st = onchip_words(h, q.words());
+  if (st) return st;
+  return onchip_launch<VT>(h->stream, A, B, p, q, h->oc_slots, h->state_h, h->hist_d, hist_cap, done);
+}
+
+// ---- many systems ------------------------------------------------------------------
+//
+// Independent systems as such kernels side by side, each on a share of the
+// SMs: the SMs' time goes into exchanges when one small system has them all,
+// and about 1.3 million rows at once keep their working set in L2.  1, 2, 4
+// or 8 lanes (streams) share the SMs; the largest systems come first, and
+// when a lane is through with its class it divides into two of the next, so
+// that no lane waits for another.  64 systems of sides 16..96: 155 ms in
+// common sweeps (batched.cu), 160 with classes of 303k, 151k and 74k rows,
+// 124 with these.
+constexpr int kOcLanes = 8;
+static long lane_rows(int lanes) { return lanes == 1 ? 1L << 30 : lanes == 2 ? 900000 : lanes == 4 ? 500000 : 200000; }
+
+int pcg_onchip_many(celg_handle* h, int count, celg_mat* const* mats, const double* const* b, double* const* x,
+                    const celg_params* p, const PcgState** states, bool* done) {
+  *done = false;
+  struct Job {
+    int sys, lanes;
+    OnchipPlan q;
+    size_t words;
+  };
+  std::vector<Job> jobs;
+  size_t words = 0;
+  for (int s = 0; s < count; ++s) {
+    CsrDev& A = mats[s]->csr;
+    if (A.n == 0) continue;
+    Job j;
+    j.sys = s;
+    j.lanes = 0;
+    for (int lanes = kOcLanes; lanes >= 1 && !j.lanes; lanes /= 2)
+      if (A.n <= lane_rows(lanes) && onchip_plan<double>(A, std::max(1, h->sms / lanes), &j.q)) j.lanes = lanes;
+    if (!j.lanes) return CELG_OK;
+    j.words = words;
+    words += j.q.words();
+    jobs.push_back(j);
+  }
+  // Which way is faster, from us an iteration of each and iterations that grow
+  // with the side: the sweeps take 24 us and the rows of all live systems at
+  // 26k a us for as many iterations as the slowest needs; a kernel takes 7 us
+  // and its rows at its lane's share of 36k a us.  (64 systems of sides 8..16:
+  // 2.2 : 3.1 ms, the sweeps; 8..40 8.9 : 8.1, 16..60 32 : 26.)
+  double sweeps = 0.0, slowest = 0.0, kernels = 0.0, longest = 0.0;
+  for (const Job& j : jobs) {
+    const double n = (double)mats[j.sys]->csr.n, its = std::cbrt(n), t = its * (7.0 + n * j.lanes / 36000.0);
+    slowest = std::max(slowest, its);
+    sweeps += its * n / 26000.0;
+    kernels += t / j.lanes;
+    longest = std::max(longest, t);
+  }
+  if (std::max(kernels, longest) >= sweeps + 24.0 * slowest) return CELG_OK;
+  for (const Job& j : jobs) {
+    bool ok = false;
+    CsrDev& A = mats[j.sys]->csr;
+    const int st = onchip_matrix<double>(h, A, A.v, j.q, &ok);
+    if (st || !ok) return st;
+  }
+  // work vectors p and v of every lane, as long as the largest system
+  size_t room = 32;
+  for (const Job& j : jobs) room = std::max(room, ((size_t)mats[j.sys]->csr.n + 31) & ~(size_t)31);
+  const size_t work = 2 * kOcLanes * room;
+  if (work > h->oc_work_cap) {
+    CELG_CUDA(cudaStreamSynchronize(h->stream));
+    cudaFree(h->oc_work);
+    h->oc_work = nullptr;
+    h->oc_work_cap = 0;
+    CELG_CUDA(cudaMalloc(&h->oc_work, sizeof(double) * work));
+    h->oc_work_cap = work;
+  }
+  if (count > h->oc_states_cap) {
+    cudaFreeHost(h->oc_states);
+    h->oc_states = nullptr;
+    h->oc_states_cap = 0;
+    CELG_CUDA(cudaMallocHost(&h->oc_states, sizeof(PcgState) * (size_t)count));
+    h->oc_states_cap = count;
+  }
+  for (int l = 0; l < kOcLanes; ++l) {
+    if (l && !h->oc_lane[l]) CELG_CUDA(cudaStreamCreateWithFlags(&h->oc_lane[l], cudaStreamNonBlocking));
+    if (!h->oc_event[l]) CELG_CUDA(cudaEventCreateWithFlags(&h->oc_event[l], cudaEventDisableTiming));
+  }
+  int st = onchip_words(h, std::max<size_t>(words, 1));
+  if (st) return st;
+  std::stable_sort(jobs.begin(), jobs.end(),
+                   [&](const Job& a, const Job& c) { return mats[a.sys]->csr.n > mats[c.sys]->csr.n; });
+  const Job* first = nullptr;
+  for (const Job& j : jobs)
+    if (!first || j.lanes < first->lanes) first = &j;
+  double load[kOcLanes] = {};
+  auto stream_of = [&](int l) { return l ? h->oc_lane[l] : h->stream; };
+  for (int lanes = 1; lanes <= kOcLanes && !st; lanes *= 2) {
+    // lane l of the upper half starts where lane l - lanes / 2 is now
+    for (int l = lanes / 2; l < lanes && lanes > 1; ++l) {
+      const int from = l - lanes / 2;
+      CELG_CUDA(cudaEventRecord(h->oc_event[l], stream_of(from)));
+      CELG_CUDA(cudaStreamWaitEvent(stream_of(l), h->oc_event[l], 0));
+      load[l] = load[from];
+    }
+    for (const Job& j : jobs) {
+      if (j.lanes != lanes || st) continue;
+      celg_mat* m = mats[j.sys];
+      int l = 0;
+      for (int k = 1; k < lanes; ++k)
+        if (load[k] < load[l]) l = k;
+      // (iterations grow with the side; an iteration is a fixed part and the
+      // rows' share of the memory)
+      load[l] += std::cbrt((double)m->csr.n) * (200000.0 + (double)lanes * m->csr.n);
+      PcgBind<double> B;
+      B.A = &m->csr;
+      B.vals = B.verify_vals = m->csr.v;
+      B.b = b[j.sys];
+      B.x = x[j.sys];
+      B.p = h->oc_work + (size_t)(2 * l) * room;
+      B.v = h->oc_work + (size_t)(2 * l + 1) * room;
+      B.J = m->jacobi;
+      B.juni = m->csr.juni;
+      B.jval = m->csr.jval;
+      bool launched = false;
+      st = onchip_launch<double>(stream_of(l), m->csr, B, p, j.q, h->oc_slots + j.words, h->oc_states + j.sys, nullptr,
+                                 0, &launched);
+      // (the largest shares come first: if the first is refused, nothing has run)
+      if (!st && !launched && &j == first) return CELG_OK;
+      if (!st && !launched) st = CELG_ERR_CUDA;
+    }
+  }
+  for (int l = 1; l < kOcLanes; ++l) {
+    CELG_CUDA(cudaEventRecord(h->oc_event[l], h->oc_lane[l]));
+    CELG_CUDA(cudaStreamWaitEvent(h->stream, h->oc_event[l], 0));
+  }
+  *states = h->oc_states;
+  *done = !st;
+  return st;
 }
 
 template int pcg_onchip<double>(celg_handle*, CsrDev&, const PcgBind<double>&, const celg_params*, int, bool*);

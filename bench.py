@@ -9,8 +9,9 @@ and b stay resident in HBM (1.9 GB, far above the 126 MB L2, so no L2 flush
 is needed between steps).
 
 Also reported on the same line:
-  roofline      the dominant kernel (the CSR SpMV), timed alone with CUDA
-                events, algorithmic bytes 12 nnz + 4 (n+1) + 16 n per launch
+  roofline      the CSR SpMV, timed alone with CUDA events, over the bytes of
+                the form it reads: 17 n per launch, since the rows of this
+                matrix repeat and it is read as one index byte per row
   e2e           the same solves through the reference-facing ELM interface
                 (celg_elm_doit + celg_elm_collect_solution: b copied from
                 pinned host memory, x copied back) inside the timed region
@@ -175,13 +176,12 @@ def plain_large_form(h, celgpu, torch, stream, m, b, x, iters_csr):
         xs = torch.from_numpy(np.random.default_rng(1).random(n)).cuda()
         ys = torch.zeros(n, dtype=torch.float64, device="cuda")
         row = {}
-        # JAD reads no column data when the matrix has row patterns: 8 bytes
-        # per non-zero and one pattern byte per row instead of 12
+        # the Poisson rows repeat: both formats are swept over the row table,
+        # one index byte per row, x and y
         pat = mm.column_form() == celgpu.COLS_PATTERN
-        jad_bytes = (8 * nnz + n if pat else 12 * nnz) + 4 * 8 + 20 * n
-        row["jad_columns"] = "row patterns" if pat else "int32"
-        for name, fmt, nbytes in (("csr", celgpu.FMT_CSR, 12 * nnz + 4 * (n + 1) + 16 * n),
-                                  ("jad", celgpu.FMT_JAD, jad_bytes)):
+        row["matrix_form"] = "row table" if pat else "int32 columns"
+        for name, fmt, nbytes in (("csr", celgpu.FMT_CSR, 17 * n if pat else 12 * nnz + 4 * (n + 1) + 16 * n),
+                                  ("jad", celgpu.FMT_JAD, 17 * n if pat else 12 * nnz + 4 * 8 + 20 * n)):
             ms, _ = time_it(lambda: h.spmv(mm, xs.data_ptr(), ys.data_ptr(), fmt=fmt), 50)
             gbs = nbytes / (ms / 1e3) / 1e9
             row[name] = {"ms": ms, "gbs": gbs, "frac_of_measured": gbs / peak, "bytes": nbytes}
@@ -718,8 +718,8 @@ def run_gpu(args):
     ms_per_step = ms / args.steps
     # algorithmic bytes of one iteration, as the library accounts them for the
     # solve it ran: K1 (matrix, p gathered, v stored), K2 (r, v, J read, r
-    # stored), K3 (p, r, J, x read, p, x stored); the matrix is 9 bytes per
-    # non-zero with 1-byte column offsets, else 12
+    # stored), K3 (p, r, J, x read, p, x stored); this matrix is one byte per
+    # row (the row table) and its J, the same for all rows, is not read
     pcg_bytes = int(h.elm_performance()[2])
 
     # ---- roofline: the CSR SpMV kernel alone ----
@@ -734,10 +734,11 @@ def run_gpu(args):
     e1.record(stream)
     torch.cuda.synchronize()
     spmv_ms = e0.elapsed_time(e1) / reps
-    spmv_bytes = 12 * nnz + 4 * (n + 1) + 16 * n
+    # one index byte of the row table, x and y per row
+    spmv_bytes = 17 * n
     peak, peak_kind = measured_peaks()
     achieved = spmv_bytes / (spmv_ms / 1e3) / 1e9
-    traffic, traffic_src = ncu_traffic("spmv_csr_256")
+    traffic, traffic_src = ncu_traffic("spmv_row_table_256")
 
     # ---- other precision forms on the same system (reported, not the value) ----
     forms = {}
@@ -799,7 +800,7 @@ def run_gpu(args):
                 "bytes_per_iteration": pcg_bytes,
                 "achieved_gbs": pcg_bytes * iters / (ms_per_step / 1e3) / 1e9,
                 "frac_of_peak": pcg_bytes * iters / (ms_per_step / 1e3) / 1e9 / peak},
-        "roofline": {"kernel": "csr_tma_kernel<double, EpiStore> (SpMV 256^3)", "bound": "hbm",
+        "roofline": {"kernel": "csr_win_kernel<double, EpiStore> (SpMV 256^3)", "bound": "hbm",
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": f"{peak_kind} hbm_gbs (copy, burst)",
                      "bytes_per_launch": spmv_bytes, "ms_per_launch": spmv_ms,

@@ -1,5 +1,6 @@
 // batched.cu -- Jacobi-PCG on many independent systems of uneven size in one
-// device-driven loop.
+// device-driven loop (FP64 batches run as one kernel per system instead where
+// that is faster: pcg_onchip_many, pcg_onchip.cu).
 //
 // The systems are concatenated into one block-diagonal CSR matrix, each
 // system's rows padded to whole 1024-row tiles (padding rows are empty, with

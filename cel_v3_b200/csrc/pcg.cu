@@ -20,11 +20,13 @@
 // vector update is computed in double from the float operands and rounded
 // once, reductions and scalars are double.  For VT = double the arithmetic
 // is exactly the reference's.
-// Algorithmic bytes per FP64 CSR iteration: 12 nnz + 4 (n+1) + 96 n (K1
-// 12 nnz + 4 (n+1) + 16 n, p gathered and v stored, the p of p.v coming
-// from L1/L2; K2 32 n; K3 48 n).  When the matrix has at most 256 column
-// offsets the CSR sweeps read 1-byte column codes instead of int32 columns:
-// 9 nnz instead of 12 nnz.
+// Algorithmic bytes per FP64 CSR iteration: the matrix, and 92 n (K1 16 n, p
+// gathered and v stored, the p of p.v coming from L1/L2; K2 32 n; K3 44 n,
+// paired).  The matrix is 12 nnz + 4 (n+1) with int32 columns, 9 nnz + 4 (n+1)
+// with 1-byte offsets, 8 nnz + n + 4 (n+1) with row patterns and n with the
+// row table, whose Jacobi values save 14 n or 16 n more.
+//
+// Systems that fit are solved by one kernel instead (pcg_onchip.cu).
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

@@ -243,13 +243,14 @@ int celg_solve_host(celg_handle* h, celg_mat* m, int solver, const double* b_hos
                     double* x_host, const celg_params* p, celg_result* res);
 
 /* ---- batched form -------------------------------------------------------------- */
-/* Jacobi-PCG on `count` independent systems of uneven size in one device-driven
- * loop (one CUDA graph launch for the whole batch).  mats[k] must have Jacobi
- * set; b_d[k], x_d[k] are device vectors of mats[k]'s size.  p applies to every
+/* Jacobi-PCG on `count` independent systems of uneven size: in FP64, systems
+ * of up to 2.1 million rows as one kernel each, side by side on the GPU, or
+ * (many tiny systems, larger ones, the FP32 forms) all in one device-driven
+ * loop of common sweeps, one CUDA graph launch.  mats[k] must have Jacobi set; b_d[k], x_d[k] are device vectors of mats[k]'s size.  p applies to every
  * system (eps_rel relative to each system's own ||b||).  res (count entries,
  * nullable) receives the per-system reports; history is not recorded.  Each
  * system's result is bit-identical to celg_pcg_jacobi on it alone.  The
- * concatenated copy of the matrices is cached on the handle until another
+ * concatenated copy of the matrices that the common sweeps read is cached on the handle until another
  * batch or a celg_mat_destroy.  precision CELG_PREC_FP64, CELG_PREC_FP32_IR
  * (FP32 inner solves inside FP64 refinement of every system: iter_done is
  * then the outer step count, arnoldi_steps the inner iterations, as for

@@ -480,6 +480,9 @@ __device__ __forceinline__ void vacc(float4& s, float v, const float4& x) {
   s.w = vadd(s.w, vmul(v, x.w));
 }
 
+// Forms of the matrix that the 16-byte-gather SpMM reads.
+constexpr int kSpmmStored = 0, kSpmmPattern = 1, kSpmmTable = 2;
+
 // The same SpMM with 16-byte gathers and rows spread over lanes: a warp
 // works on RS = 4 RP rows per step, lanes 8g..8g+7 on rows g, g+4, ... of
 // the step (RP rows each, whose gathers are all in flight together).  Lane l
@@ -498,7 +501,15 @@ __device__ __forceinline__ void vacc(float4& s, float v, const float4& x) {
 // use by all CTAs together within L2.
 // PAT: the matrix's row patterns (pid, pat; spmv_kernels.cuh) give each
 // entry's column as row + offset, so the X gathers need no column load.
-template <class Epi, int MINB, int U, int RP, bool PAT>
+// TAB: the row table gives the values too.  A lane then reads its row's
+// pattern byte from a register (the warp's 32 bytes are loaded a row group
+// ahead) and offsets, values and length from shared memory: no load stands
+// before the X gathers, and a third of the global loads go.  128^3, k = 32:
+// a whole solve 395 -> 380 ms (two boxes 1.035x); what is left is the gathers
+// themselves, 1 KB a row from L2 and 26 L1 wavefronts a row.  Handing the
+// CTAs of an SM tiles a plane apart, so that they meet in L1: 375 ms on a box
+// where the patterns took 382, no better than the table alone.
+template <class Epi, int MINB, int U, int RP, int FORM>
 __global__ void __launch_bounds__(kLanes, MINB) spmm_vec_kernel(const int* __restrict__ rp,
                                                                const int* __restrict__ ci,
                                                                const typename Epi::VT* __restrict__ v,
@@ -507,7 +518,8 @@ __global__ void __launch_bounds__(kLanes, MINB) spmm_vec_kernel(const int* __res
                                                                Epi epi, RedCtx red,
                                                                const uint8_t* __restrict__ pid,
                                                                const int* __restrict__ pat,
-                                                               int pat_ints) {
+                                                               const int* __restrict__ plen, int npat) {
+  constexpr bool PAT = FORM != kSpmmStored, TAB = FORM == kSpmmTable;
   using VT = typename Epi::VT;
   using V16 = typename Vec16<VT>::T;
   constexpr int NR = Epi::NRED;
@@ -541,11 +553,24 @@ __global__ void __launch_bounds__(kLanes, MINB) spmm_vec_kernel(const int* __res
   VT* sw = reinterpret_cast<VT*>(s_dyn + (long)warp * kWarpDoubles);
   double* sp = s_dyn + (long)warp * kWarpDoubles + RS * 32 * (int)sizeof(VT) / 8;
   [[maybe_unused]] int* s_pat = reinterpret_cast<int*>(s_dyn + 8L * kWarpDoubles);
+  [[maybe_unused]] VT* s_val = reinterpret_cast<VT*>(s_pat + npat * kPatLen);
+  [[maybe_unused]] int* s_len = reinterpret_cast<int*>(s_val + npat * kPatLen);
   if constexpr (PAT) {
-    for (int q = threadIdx.x; q < pat_ints; q += blockDim.x) s_pat[q] = pat[q];
+    for (int q = threadIdx.x; q < npat * kPatLen; q += blockDim.x) {
+      s_pat[q] = pat[q];
+      if constexpr (TAB) s_val[q] = v[q];
+    }
+    if constexpr (TAB)
+      for (int q = threadIdx.x; q < npat; q += blockDim.x) s_len[q] = plen[q];
     __syncthreads();
   }
   const long ntiles = ((long)n + kTile - 1) / kTile;
+  // TAB: the pattern bytes of the warp's 32 rows, a row group ahead
+  [[maybe_unused]] int id_next = 0;
+  if constexpr (TAB) {
+    const long i = tile_at(blockIdx.x, ntiles, red.sweep) * kTile + threadIdx.x;
+    if (blockIdx.x < ntiles && i < n) id_next = __ldg(pid + i);
+  }
   for (long kt = blockIdx.x; kt < ntiles; kt += gridDim.x) {
     const long t = tile_at(kt, ntiles, red.sweep);
     double acc[NR1];
@@ -553,6 +578,13 @@ __global__ void __launch_bounds__(kLanes, MINB) spmm_vec_kernel(const int* __res
     for (int r = 0; r < NR1; ++r) acc[r] = 0.0;
     for (int q = 0; q < 4; ++q) {
       const long row0 = t * kTile + q * kSub + warp * 32;
+      [[maybe_unused]] const int ids = id_next;
+      if constexpr (TAB) {
+        long i = row0 + kSub + lane;
+        if (q == 3 || row0 + kSub >= n)
+          i = kt + gridDim.x < ntiles ? tile_at(kt + gridDim.x, ntiles, red.sweep) * kTile + threadIdx.x : n;
+        id_next = i < n ? (int)__ldg(pid + i) : 0;
+      }
       if (row0 >= n) break;
       const int nrows = (int)min(32L, (long)n - row0);
       for (int s0 = 0; s0 < nrows; s0 += RS) {
@@ -569,10 +601,20 @@ __global__ void __launch_bounds__(kLanes, MINB) spmm_vec_kernel(const int* __res
         }
         int b[RP], e[RP];
         [[maybe_unused]] const int* po[RP];
+        [[maybe_unused]] const VT* pv[RP];
         int lmax = 0;
 #pragma unroll
         for (int j = 0; j < RP; ++j) {
           const int r = s0 + g + 4 * j;
+          if constexpr (TAB) {
+            const int id = __shfl_sync(0xffffffffu, ids, r);
+            b[j] = 0;
+            e[j] = r < nrows ? s_len[id] : 0;
+            po[j] = s_pat + id * kPatLen;
+            pv[j] = s_val + id * kPatLen;
+            lmax = max(lmax, e[j]);
+            continue;
+          }
           b[j] = r < nrows ? __ldg(rp + row0 + r) : 0;
           e[j] = r < nrows ? __ldg(rp + row0 + r + 1) : 0;
           if constexpr (PAT) po[j] = s_pat + (r < nrows ? (int)__ldg(pid + row0 + r) : 0) * kPatLen;
@@ -595,7 +637,10 @@ __global__ void __launch_bounds__(kLanes, MINB) spmm_vec_kernel(const int* __res
                 cc[j][u] = kk < e[j] ? (int)(row0 + s0 + g + 4 * j) + po[j][c0 + u] : 0;
               else
                 cc[j][u] = kk < e[j] ? __ldg(ci + kk) : 0;
-              vv[j][u] = kk < e[j] ? __ldg(v + kk) : VT(0);
+              if constexpr (TAB)
+                vv[j][u] = kk < e[j] ? pv[j][kk] : VT(0);
+              else
+                vv[j][u] = kk < e[j] ? __ldg(v + kk) : VT(0);
             }
           V16 xg[RP][U][NV];
 #pragma unroll
@@ -1677,7 +1722,7 @@ static int launch_spmm_cfg(celg_handle* h, const CsrDev& A, const typename Epi::
   return CELG_OK;
 }
 
-template <class Epi, int MINB, int U, int RP, bool PAT>
+template <class Epi, int MINB, int U, int RP, int FORM>
 static int launch_spmm_vec_p(celg_handle* h, const CsrDev& A, const typename Epi::VT* vals, int k,
                              const typename Epi::VT* X, const Epi& epi) {
   using VT = typename Epi::VT;
@@ -1685,28 +1730,31 @@ static int launch_spmm_vec_p(celg_handle* h, const CsrDev& A, const typename Epi
   RedCtx red{h->partials, h->ticket, nt};
   if (A.n == 0) return CELG_OK;
   red.sweep = next_sweep(h, false);
-  auto kern = spmm_vec_kernel<Epi, MINB, U, RP, PAT>;
+  auto kern = spmm_vec_kernel<Epi, MINB, U, RP, FORM>;
   const int rs = 4 * RP;
-  const int pat_ints = PAT ? A.npat * kPatLen : 0;
-  const int smem =
-      8 * (rs * 32 * (int)sizeof(VT) + (sizeof(VT) == 8 ? rs * 64 * 8 : 0)) + pat_ints * 4;
-  if (const int st = allow_dynamic_smem<spmm_vec_kernel<Epi, MINB, U, RP, PAT>>(smem)) return st;
+  const int npat = FORM != kSpmmStored ? A.npat : 0;
+  const int smem = 8 * (rs * 32 * (int)sizeof(VT) + (sizeof(VT) == 8 ? rs * 64 * 8 : 0)) +
+                   npat * (kPatLen * 4 + (FORM == kSpmmTable ? kPatLen * (int)sizeof(VT) + 4 : 0));
+  if (const int st = allow_dynamic_smem<spmm_vec_kernel<Epi, MINB, U, RP, FORM>>(smem)) return st;
   int per_sm = 0;
   CELG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLanes, smem));
   const int grid = grid_for_tiles(h, nt, std::max(1, per_sm));
   kern<<<grid, kLanes, smem, h->stream>>>(A.rp, A.ci, vals, A.n, k, X, epi, red, A.pid, A.pat,
-                                          pat_ints);
+                                          A.plen, npat);
   CELG_CUDA(cudaGetLastError());
   return CELG_OK;
 }
 
-// The 16-byte-gather SpMM, on the row patterns when the matrix has them
-// (same columns in the same order: the same sums).
+// The 16-byte-gather SpMM, on the most compact form that the matrix has: the
+// row table, the row patterns or the entries as stored (same columns and
+// values in the same order: the same sums).
 template <class Epi, int MINB, int U, int RP>
 static int launch_spmm_vec(celg_handle* h, const CsrDev& A, const typename Epi::VT* vals, int k,
                            const typename Epi::VT* X, const Epi& epi) {
-  if (A.pid) return launch_spmm_vec_p<Epi, MINB, U, RP, true>(h, A, vals, k, X, epi);
-  return launch_spmm_vec_p<Epi, MINB, U, RP, false>(h, A, vals, k, X, epi);
+  if (A.rowv)
+    return launch_spmm_vec_p<Epi, MINB, U, RP, kSpmmTable>(h, A, row_values<typename Epi::VT>(A), k, X, epi);
+  if (A.pid) return launch_spmm_vec_p<Epi, MINB, U, RP, kSpmmPattern>(h, A, vals, k, X, epi);
+  return launch_spmm_vec_p<Epi, MINB, U, RP, kSpmmStored>(h, A, vals, k, X, epi);
 }
 
 // SpMM of the FP32 solves: the 16-byte-gather kernel when k is a multiple

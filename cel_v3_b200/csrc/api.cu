@@ -730,7 +730,9 @@ extern "C" int celg_mat_scale_diagonal(celg_mat* m) {
   if (!st) st = launch_jacobi_setup(m->h, m);  // jacobi = sqrt|d| / d
   if (st) return st;
   if (m->jad.mmax >= 0) st = build_jad(m);
+  // the FP32 copies follow, the Jacobi values too: their table has the new ones
   if (!st && m->csr.v32) st = launch_to_f32(m->h, m->csr.nnz, m->csr.v, m->csr.v32);
+  if (!st && m->jacobi32) st = launch_to_f32(m->h, m->csr.n, m->jacobi, m->jacobi32);
   if (st) return st;
   CELG_CUDA(cudaStreamSynchronize(m->h->stream));
   return CELG_OK;

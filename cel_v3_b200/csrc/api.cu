@@ -635,6 +635,14 @@ extern "C" int celg_mat_from_csr_device(celg_handle* h, int n, int nnz, const in
   return CELG_OK;
 }
 
+// The cached batch, which holds copies of its matrices, and the graphs on it.
+static void drop_batch(celg_handle* h) {
+  if (!h->batch) return;
+  graph_cache_clear(h);
+  batch_free(h->batch);
+  h->batch = nullptr;
+}
+
 extern "C" int celg_mat_destroy(celg_mat* m) {
   if (!m) return CELG_OK;
   celg_handle* h = m->h;
@@ -643,11 +651,7 @@ extern "C" int celg_mat_destroy(celg_mat* m) {
   // cached solve graphs (and a cached batch) may reference this matrix
   graph_cache_drop_matrix(h, m);
   multi_forget_matrix(h->multi, m);
-  if (h->batch) {
-    graph_cache_clear(h);
-    batch_free(h->batch);
-    h->batch = nullptr;
-  }
+  drop_batch(h);
   free_mat_arrays(m);
   delete m;
   return CELG_OK;
@@ -717,10 +721,11 @@ extern "C" int celg_mat_scale_diagonal(celg_mat* m) {
   if (!st) st = launch_row_scale(m->h, m);
   if (st) return st;
   m->scaled = true;
-  // the values changed: what was derived from them goes, and with it the
-  // cached graphs that hold its addresses
+  // the values changed: what was derived from them goes (a cached batch's
+  // copies too), and with it the cached graphs that hold its addresses
   CELG_CUDA(cudaStreamSynchronize(m->h->stream));
   graph_cache_clear(m->h);
+  drop_batch(m->h);
   multi_forget_matrix(m->h->multi, m);
   sell_free(m->h, m->csr);
   st = row_forms_search(m->h, m->csr, true, nullptr);

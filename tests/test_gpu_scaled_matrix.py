@@ -47,3 +47,31 @@ def test_scaled_after_a_solve(gpu, kind, precision, columns):
     assert got[1] == want[1] and np.array_equal(got[0], want[0])
     m.destroy()
     fresh.destroy()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_ru", "fp32_ir"])
+def test_scaled_between_batches(gpu, precision, monkeypatch):
+    """The common sweeps read concatenated copies of the systems."""
+    celgpu, h, torch = gpu
+    prec = {"fp64": celgpu.PREC_FP64, "fp32_ru": celgpu.PREC_FP32_RU, "fp32_ir": celgpu.PREC_FP32_IR}[precision]
+    kw = dict(eps_rel=1e-9, iter_max=2000, x0_mode=celgpu.X0_ZERO, precision=prec, inner_eps_rel=1e-2)
+    monkeypatch.setenv("CELG_ONCHIP_ROWS", "0")
+    mats = [h.matrix_from_csr(*variable(q)).jacobi() for q in (9, 14, 11)]
+    b = [torch.from_numpy(np.random.default_rng(m.n).uniform(-1, 1, m.n)).cuda() for m in mats]
+    x = [torch.zeros_like(t) for t in b]
+
+    def batch():
+        i = h.pcg_batched(mats, [t.data_ptr() for t in b], [t.data_ptr() for t in x], **kw)
+        torch.cuda.synchronize()
+        return [t.cpu().numpy() for t in x], i
+
+    batch()
+    mats[1].scale_diagonal()
+    got, info = batch()
+    for k, m in enumerate(mats):
+        y = torch.zeros_like(b[k])
+        one = h.pcg_jacobi(m, b[k].data_ptr(), y.data_ptr(), **kw)
+        torch.cuda.synchronize()
+        assert info[k].iter_done == one.iter_done and np.array_equal(got[k], y.cpu().numpy()), k
+    for m in mats:
+        m.destroy()

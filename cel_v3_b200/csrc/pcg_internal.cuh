@@ -212,8 +212,14 @@ struct EpiAp {
   PcgArgs a;
   __device__ bool active() const { return *(volatile int*)&a.st->active != 0; }
   // p(i) is loaded after the row's gathers: issued before them it cost 23 us
-  // per 256^3 sweep (290 -> 267 us)
-  __device__ void row(long i, VT s, double* acc) const { row_x(i, s, __ldg(p + i), acc); }
+  // per 256^3 sweep (290 -> 267 us).  After the store too: loaded before it,
+  // the FP64 pattern sweep spills a register (a solve of variable coefficients
+  // at 131^3 24.26 against 24.03 ms, at 150^3 37.54 : 37.32).
+  __device__ void row(long i, VT s, double* acc) const {
+    const VT vi = vadd(VT(0), s);
+    v[i] = vi;
+    acc[0] = dacc_prod(acc[0], vi, __ldg(p + i));
+  }
   // p is the sweep's x: taken from the staged window where there is one
   static constexpr bool kTakesX = true;
   __device__ void row_x(long i, VT s, VT pi, double* acc) const {

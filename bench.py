@@ -349,6 +349,9 @@ def batch_form(h, celgpu, torch, stream):
                      "sum_iters": sum(i.iter_done for i in infos),
                      "worst_verified_relres": max(i.verified_relres for i in infos),
                      "all_ok": all(i.status == celgpu.OK for i in infos)}
+        if name != "one_by_one":
+            kernels = h.tuned_config(celgpu.TUNE_BATCH_PATH)[0] == celgpu.BATCH_KERNELS
+            out[name]["path"] = "one kernel per system" if kernels else "common sweeps"
         if name == "batched":
             x64 = [x.clone() for x in xs]
         elif name in ("batched_fp32_ir", "batched_fp32_ru"):
@@ -360,6 +363,7 @@ def batch_form(h, celgpu, torch, stream):
                                                     out["one_by_one"]["solves_per_s"])
     out["systems"] = len(mats)
     out["rows"] = int(sum(s ** 3 for s, *_ in probs))
+    # the shape that the last form's common sweeps were tuned to
     csr_ctas, sweep_ctas = h.tuned_config(celgpu.TUNE_BATCH)
     out["tuned_launch"] = {"spmv_ctas_per_sm": csr_ctas or "max resident",
                            "vector_sweep_ctas_per_sm": sweep_ctas}

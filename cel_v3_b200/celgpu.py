@@ -43,6 +43,9 @@ FMT_JAD = 1
 COLS_INT32, COLS_OFFSET8, COLS_PATTERN = 0, 1, 2
 TUNE_BATCH = 0
 TUNE_SPMM = 1
+TUNE_BATCH_PATH = 2
+BATCH_SWEEPS = 0
+BATCH_KERNELS = 1
 PRECOND_JACOBI = 0
 PRECOND_BLOCK_JACOBI = 1
 
@@ -696,7 +699,8 @@ class Handle:
     def tuned_config(self, what):
         """celg_tuned_config: the autotuner's pick for the last batched
         (TUNE_BATCH: (SpMV CTAs per SM, vector-sweep CTAs per SM)) or
-        multi-RHS (TUNE_SPMM: (FP64 variant, FP32 shape or -1)) solve."""
+        multi-RHS (TUNE_SPMM: (FP64 variant, FP32 shape or -1)) solve, or the
+        last batch's path (TUNE_BATCH_PATH: (BATCH_SWEEPS or BATCH_KERNELS, 0))."""
         out = (ctypes.c_int * 2)()
         _check(lib.celg_tuned_config(self.ptr, int(what), out), "celg_tuned_config")
         return out[0], out[1]

@@ -1225,17 +1225,9 @@ static int pcg_batched_onchip(celg_handle* h, int count, celg_mat* const* mats, 
   return ret;
 }
 
-int pcg_batched(celg_handle* h, int count, celg_mat* const* mats, const double* const* b_d,
-                double* const* x_d, const celg_params* p, celg_result* res) {
-  if (p->precision == CELG_PREC_FP32_IR) return pcg_batched_ir(h, count, mats, b_d, x_d, p, res);
-  if (p->precision == CELG_PREC_FP32_RU) return pcg_batched_ru(h, count, mats, b_d, x_d, p, res);
-  if (p->precision != CELG_PREC_FP64) return CELG_ERR_ARG;
-  {
-    bool done = false;
-    const int ret = pcg_batched_onchip(h, count, mats, b_d, x_d, p, res, &done);
-    h->batch_onchip = done;
-    if (ret || done) return ret;
-  }
+// FP64 in common sweeps over all systems.
+static int pcg_batched_sweeps(celg_handle* h, int count, celg_mat* const* mats, const double* const* b_d,
+                              double* const* x_d, const celg_params* p, celg_result* res) {
   Batch* bt = nullptr;
   int st = batch_for(h, count, mats, b_d, x_d, &bt);
   if (st) return st;
@@ -1680,6 +1672,25 @@ static int pcg_batched_ru(celg_handle* h, int count, celg_mat* const* mats, cons
   return ret;
 }
 
+int pcg_batched(celg_handle* h, int count, celg_mat* const* mats, const double* const* b_d,
+                double* const* x_d, const celg_params* p, celg_result* res) {
+  int path = CELG_BATCH_SWEEPS, st;
+  if (p->precision == CELG_PREC_FP32_IR) {
+    st = pcg_batched_ir(h, count, mats, b_d, x_d, p, res);
+  } else if (p->precision == CELG_PREC_FP32_RU) {
+    st = pcg_batched_ru(h, count, mats, b_d, x_d, p, res);
+  } else if (p->precision == CELG_PREC_FP64) {
+    bool done = false;
+    st = pcg_batched_onchip(h, count, mats, b_d, x_d, p, res, &done);
+    if (done) path = CELG_BATCH_KERNELS;
+    else if (!st) st = pcg_batched_sweeps(h, count, mats, b_d, x_d, p, res);
+  } else {
+    return CELG_ERR_ARG;
+  }
+  if (st == CELG_OK || st == CELG_ERR_NOCONV || st == CELG_ERR_BREAKDOWN) h->batch_path = path;
+  return st;
+}
+
 }  // namespace celg
 
 extern "C" int celg_pcg_batched(celg_handle* h, int count, celg_mat* const* mats,
@@ -1697,10 +1708,17 @@ extern "C" int celg_pcg_batched(celg_handle* h, int count, celg_mat* const* mats
 extern "C" int celg_tuned_config(celg_handle* h, int what, int out[2]) {
   if (!h || !out) return CELG_ERR_ARG;
   out[0] = out[1] = -1;
+  if (what == CELG_TUNE_BATCH_PATH) {
+    if (h->batch_path < 0) return CELG_ERR_STATE;
+    out[0] = h->batch_path;
+    out[1] = 0;
+    return CELG_OK;
+  }
   if (what == CELG_TUNE_BATCH) {
-    if (!h->batch_onchip && (!h->batch || h->batch->shape < 0)) return CELG_ERR_STATE;
     // (systems solved in kernels of their own leave the first shape: nothing to tune)
-    const celg::BatchShape sh = celg::kBatchShapes[h->batch_onchip ? 0 : h->batch->shape];
+    const bool kernels = h->batch_path == CELG_BATCH_KERNELS;
+    if (!kernels && (!h->batch || h->batch->shape < 0)) return CELG_ERR_STATE;
+    const celg::BatchShape sh = celg::kBatchShapes[kernels ? 0 : h->batch->shape];
     out[0] = sh.csr_per_sm;
     out[1] = sh.tile_per_sm;
     return CELG_OK;

@@ -131,7 +131,7 @@ struct celg_handle {
   int oc_states_cap = 0;
   cudaStream_t oc_lane[8] = {};
   cudaEvent_t oc_event[8] = {};
-  bool batch_onchip = false;  // the last batched FP64 solve ran that way
+  int batch_path = -1;  // of the last batched solve: CELG_BATCH_SWEEPS or CELG_BATCH_KERNELS, -1 before the first
   // host-buffer solve staging (stable pointers keep cached graphs valid)
   double* sb = nullptr;
   double* sx = nullptr;

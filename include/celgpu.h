@@ -292,9 +292,16 @@ int celg_pcg_multirhs(celg_handle* h, celg_mat* m, int k, const double* B_d, dou
  * out[0] = the FP64 SpMM variant, 0..14; out[1] = the FP32 SpMM shape of
  * the FP32 forms, 0..4, or -1 before the first of them).  No counterpart in
  * the reference, which has no autotuner.  CELG_ERR_STATE before the first
- * such solve. */
+ * such solve.  what = CELG_TUNE_BATCH_PATH: out[0] = how the last batched
+ * solve ran, CELG_BATCH_SWEEPS (common sweeps over all systems, the form that
+ * has a launch shape) or CELG_BATCH_KERNELS (every system in a kernel of its
+ * own, nothing to tune: CELG_TUNE_BATCH then gives the first of the tuner's
+ * shapes, 0 and 8); out[1] = 0. */
 #define CELG_TUNE_BATCH 0
 #define CELG_TUNE_SPMM 1
+#define CELG_TUNE_BATCH_PATH 2
+#define CELG_BATCH_SWEEPS 0
+#define CELG_BATCH_KERNELS 1
 int celg_tuned_config(celg_handle* h, int what, int out[2]);
 
 /* ---- differentiation --------------------------------------------------------- */

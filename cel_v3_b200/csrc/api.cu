@@ -49,13 +49,13 @@ cudaError_t dev_alloc_bytes(celg_handle* h, void** p, size_t bytes) {
   return e;
 }
 
-void dev_free(celg_handle* h, void* p) {
+void dev_free(celg_handle* h, void* p, bool keep) {
   if (!p) return;
   for (size_t k = h->blocks.size(); k-- > 0;)
     if (h->blocks[k].p == p) {
       const celg_handle::DevBlock b = h->blocks[k];
       h->blocks.erase(h->blocks.begin() + (long)k);
-      if (b.bytes <= kSpareBlock && h->spare_bytes + b.bytes <= kSpareBytes) {
+      if (keep && b.bytes <= kSpareBlock && h->spare_bytes + b.bytes <= kSpareBytes) {
         h->spare.push_back(b);
         h->spare_bytes += b.bytes;
       } else {
@@ -71,6 +71,14 @@ void dev_free_spare(celg_handle* h) {
   for (const celg_handle::DevBlock& b : h->spare) cudaFree(b.p);
   h->spare.clear();
   h->spare_bytes = 0;
+}
+
+void note_use(celg_handle* h, const celg_mat* m) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(h->stream, &cs);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  if (m->h != h || e != cudaSuccess || cs != cudaStreamCaptureStatusNone)
+    __atomic_store_n(&m->elsewhere, 1, __ATOMIC_RELAXED);
 }
 
 // ---- matrix set-up kernels ---------------------------------------------------
@@ -260,18 +268,19 @@ int ensure_offset_dict(celg_handle* h, celg_mat* m) {
 
 void free_mat_arrays(celg_mat* m) {
   celg_handle* h = m->h;
-  dev_free(h, m->csr.rp);  // ci and v are parts of its block
-  dev_free(h, m->csr.v32);
+  const bool keep = !__atomic_load_n(&m->elsewhere, __ATOMIC_RELAXED);
+  dev_free(h, m->csr.rp, keep);  // ci and v are parts of its block
+  dev_free(h, m->csr.v32, keep);
   cudaFree(m->csr.ci8);
   cudaFree(m->csr.dict);
-  row_forms_free(h, m->csr);
+  row_forms_free(h, m->csr, keep);
   sell_free(h, m->csr);
   cudaFree(m->jad.begin);
   cudaFree(m->jad.ci);
   cudaFree(m->jad.v);
   cudaFree(m->jad.perm);
   cudaFree(m->jad.pid);
-  dev_free(h, m->diag);  // jacobi is a part of its block
+  dev_free(h, m->diag, keep);  // jacobi is a part of its block
   dev_free(h, m->jacobi32);
   dev_free(h, m->scale);
   cudaFree(m->bjinv);
@@ -728,6 +737,7 @@ extern "C" int celg_mat_scale_diagonal(celg_mat* m) {
   drop_batch(m->h);
   multi_forget_matrix(m->h->multi, m);
   sell_free(m->h, m->csr);
+  row_forms_free(m->h, m->csr, !__atomic_load_n(&m->elsewhere, __ATOMIC_RELAXED));
   st = row_forms_search(m->h, m->csr, true, nullptr);
   if (st) return st;
   CELG_CUDA(cudaStreamSynchronize(m->h->stream));
@@ -768,6 +778,7 @@ extern "C" int celg_mat_make_fp32(celg_mat* m) {
 extern "C" int celg_spmv(celg_handle* h, const celg_mat* m, int fmt, const double* x_d, double* y_d,
                          int accumulate) {
   if (!h || !m || (m->csr.n > 0 && (!x_d || !y_d))) return CELG_ERR_ARG;
+  note_use(h, m);
   if (fmt == CELG_FMT_JAD) {
     if (accumulate) return CELG_ERR_ARG;  // the reference's JAD kernel overwrites y
     return launch_spmv_jad(h, m->csr, m->jad, x_d, y_d);
@@ -779,6 +790,7 @@ extern "C" int celg_spmv(celg_handle* h, const celg_mat* m, int fmt, const doubl
 extern "C" int celg_spmv_f32(celg_handle* h, const celg_mat* m, const float* x_d, float* y_d,
                              int accumulate) {
   if (!h || !m || (m->csr.n > 0 && (!x_d || !y_d))) return CELG_ERR_ARG;
+  note_use(h, m);
   return launch_spmv_csr_f32(h, m->csr, x_d, y_d, accumulate);
 }
 
@@ -815,6 +827,7 @@ extern "C" int celg_xpby(celg_handle* h, int n, const double* x_d, double beta, 
 extern "C" int celg_jacobi_apply(celg_handle* h, const celg_mat* m, const double* r_d, double* z_d) {
   if (!h || !m) return CELG_ERR_ARG;
   if (!m->jacobi) return CELG_ERR_STATE;
+  note_use(h, m);
   return launch_mul(h, m->csr.n, r_d, m->jacobi, z_d);
 }
 

@@ -181,6 +181,10 @@ struct celg_mat {
   bool dict_tried = false;    // the offset dictionary was attempted (csr.ci8 set if it fits)
   int bj_bs = 0;
   bool scaled = false;
+  // 1 when a stream that is not its handle's may hold work on the arrays:
+  // another handle multiplied with it, or a call was captured into a graph
+  // that runs wherever the caller launches it (note_use)
+  mutable int elsewhere = 0;
 };
 
 namespace celg {
@@ -195,10 +199,11 @@ int cuda_status(cudaError_t e, const char* what);
 // Device memory of the handle's matrices.  Blocks given back are kept for
 // later requests on the handle, in the order of its stream, up to
 // kSpareBytes in all (getting and returning a block costs 0.1-0.2 ms each,
-// at times milliseconds); celg_destroy frees them.
+// at times milliseconds); celg_destroy frees them.  keep = false: the block
+// goes back to the device, which waits for all work on it, on every stream.
 constexpr size_t kSpareBlock = (size_t)32 << 20, kSpareBytes = (size_t)96 << 20;
 cudaError_t dev_alloc_bytes(celg_handle* h, void** p, size_t bytes);
-void dev_free(celg_handle* h, void* p);
+void dev_free(celg_handle* h, void* p, bool keep = true);
 void dev_free_spare(celg_handle* h);
 template <typename T>
 cudaError_t dev_alloc(celg_handle* h, T** p, size_t bytes) {
@@ -260,12 +265,14 @@ size_t row_sets_bytes();
 int row_forms_search(celg_handle* h, const CsrDev& A, bool with_values, const int* bad);
 int row_forms_build(celg_handle* h, CsrDev& A, bool with_values);
 int row_forms_jacobi(celg_handle* h, CsrDev& A, const double* J);
-void row_forms_free(celg_handle* h, CsrDev& A);
+void row_forms_free(celg_handle* h, CsrDev& A, bool keep = true);
 int alloc_csr(celg_mat* m, int n, int nnz, int ncols);
 int alloc_csr_room(celg_mat* m, int n, size_t nnz_cap, int ncols);
 int set_csr_entries(celg_mat* m, int nnz);
 int finish_csr(celg_handle* h, celg_mat* m, int base);
 void free_mat_arrays(celg_mat* m);
+// An operator that queues work on m and returns, on h's stream.
+void note_use(celg_handle* h, const celg_mat* m);
 // assemble.cu: COO (device arrays, row and column bases) -> CSR matrix
 int coo_to_mat_device(celg_handle* h, int n, int ncols, int nnz, const int* rows_d,
                       const int* cols_d, const double* vals_d, int row_base, int col_base,

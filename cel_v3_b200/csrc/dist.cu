@@ -365,6 +365,8 @@ extern "C" int celg_dist_create(celg_handle* h, celg_mat* m, const celg_params* 
   celg_dist* d = new celg_dist();
   d->h = h;
   d->m = m;
+  // its phases only queue work, and may run in the caller's graphs
+  __atomic_store_n(&m->elsewhere, 1, __ATOMIC_RELAXED);
   d->p = *p;
   d->hist = hist_cap > 0 ? hist_d : nullptr;
   d->hist_cap = hist_cap;

@@ -198,8 +198,8 @@ static WinPlan plan_window(const int* pat, int count) {
   return w;
 }
 
-void row_forms_free(celg_handle* h, CsrDev& A) {
-  dev_free(h, A.pat);  // the other arrays are parts of its block
+void row_forms_free(celg_handle* h, CsrDev& A, bool keep) {
+  dev_free(h, A.pat, keep);  // the other arrays are parts of its block
   A.pid = nullptr;
   A.pat = nullptr;
   A.npat = 0;

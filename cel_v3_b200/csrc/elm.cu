@@ -20,13 +20,17 @@ struct Elm {
   // Rows that arrive whole, in order and with ascending columns need no sort:
   // as long as all do (direct), celg_elm_insert_rows copies the caller's
   // columns and values straight into the arrays of the matrix to be (dmat,
-  // columns 1-based until it is completed) and keeps the row pointer here.
+  // columns 1-based until it is completed) and keeps the row pointer here;
+  // pieces of a few rows are held here until there are enough for a copy.
   // Any other insertion moves the entries to rows/cols/vals above.
   bool direct = true;
   bool lost = false;       // completing them failed: nothing is left to retry with
   std::vector<int> rp;     // one entry per row begun, and the end
   celg_mat* dmat = nullptr;
   size_t dcap = 0;         // entries dmat has room for
+  size_t sent = 0;         // entries it has; the held ones follow
+  std::vector<int> held_cols;
+  std::vector<double> held_vals;
   size_t hint = 0;
   celg_mat* mat = nullptr;
   bool completed = false;
@@ -113,9 +117,13 @@ static int elm_undirect(celg_handle* h, Elm* e) {
   if (nnz) {
     e->cols.resize(nnz);
     e->vals.resize(nnz);
-    CELG_CUDA(cudaMemcpyAsync(e->cols.data(), e->dmat->csr.ci, sizeof(int) * nnz, cudaMemcpyDeviceToHost, h->stream));
-    CELG_CUDA(cudaMemcpyAsync(e->vals.data(), e->dmat->csr.v, sizeof(double) * nnz, cudaMemcpyDeviceToHost, h->stream));
-    CELG_CUDA(cudaStreamSynchronize(h->stream));
+    if (e->sent) {
+      CELG_CUDA(cudaMemcpyAsync(e->cols.data(), e->dmat->csr.ci, sizeof(int) * e->sent, cudaMemcpyDeviceToHost, h->stream));
+      CELG_CUDA(cudaMemcpyAsync(e->vals.data(), e->dmat->csr.v, sizeof(double) * e->sent, cudaMemcpyDeviceToHost, h->stream));
+      CELG_CUDA(cudaStreamSynchronize(h->stream));
+    }
+    std::copy(e->held_cols.begin(), e->held_cols.end(), e->cols.begin() + (long)e->sent);
+    std::copy(e->held_vals.begin(), e->held_vals.end(), e->vals.begin() + (long)e->sent);
     for (size_t r = 0; r + 1 < e->rp.size(); ++r) {
       const int row = e->row_low + (int)r;
       e->rows.insert(e->rows.end(), (size_t)(e->rp[r + 1] - e->rp[r]), row);
@@ -125,23 +133,64 @@ static int elm_undirect(celg_handle* h, Elm* e) {
   }
   if (e->dmat) celg_mat_destroy(e->dmat);
   e->dmat = nullptr;
+  e->held_cols.clear();
+  e->held_vals.clear();
   e->direct = false;
   return CELG_OK;
 }
 
+// Copies total entries (columns, values) behind those that dmat has.
+static int elm_send(celg_handle* h, Elm* e, const int* cols, const double* vals, size_t total) {
+  const size_t need = e->sent + total;
+  if (need > e->dcap || !e->dmat) {
+    celg_mat* m = new celg_mat();
+    m->h = h;
+    const size_t cap =
+        std::min(std::max(std::max(need, e->hint), e->dmat ? 2 * e->dcap : 0), ((size_t)1 << 31) - 1);
+    if (const int st = alloc_csr_room(m, e->n_local, cap, e->n_local)) {
+      delete m;
+      return st;
+    }
+    if (e->sent) {
+      CELG_CUDA(cudaMemcpyAsync(m->csr.ci, e->dmat->csr.ci, sizeof(int) * e->sent, cudaMemcpyDeviceToDevice, h->stream));
+      CELG_CUDA(cudaMemcpyAsync(m->csr.v, e->dmat->csr.v, sizeof(double) * e->sent, cudaMemcpyDeviceToDevice, h->stream));
+    }
+    if (e->dmat) celg_mat_destroy(e->dmat);
+    e->dmat = m;
+    e->dcap = cap;
+  }
+  if (total) {
+    // (from pageable memory these return when the caller's arrays are read)
+    CELG_CUDA(cudaMemcpyAsync(e->dmat->csr.ci + e->sent, cols, sizeof(int) * total, cudaMemcpyHostToDevice, h->stream));
+    CELG_CUDA(cudaMemcpyAsync(e->dmat->csr.v + e->sent, vals, sizeof(double) * total, cudaMemcpyHostToDevice, h->stream));
+    CELG_CUDA(cudaStreamSynchronize(h->stream));
+  }
+  e->sent = need;
+  return CELG_OK;
+}
+
+static int elm_send_held(celg_handle* h, Elm* e) {
+  const int st = elm_send(h, e, e->held_cols.data(), e->held_vals.data(), e->held_vals.size());
+  if (st) return st;
+  e->held_cols.clear();
+  e->held_vals.clear();
+  return CELG_OK;
+}
+
 // Whole rows in order with ascending columns, appended to dmat; *taken is
-// false (and nothing done) when the rows are not of that kind, or so few that
-// copies of their own (about 25 us a call) cost more than keeping them on the
-// host until the matrix is complete.
+// false (and nothing done) when the rows are not of that kind.  Copies of
+// their own cost about 25 us a call, so short pieces are held on the host
+// until kElmHold entries are together.
+constexpr size_t kElmHold = 4096;
 static int elm_append_rows(celg_handle* h, Elm* e, int first_row, int nrows, const int* row_ptr, const int* cols,
                            const double* vals, bool* taken) {
-  *taken = false;
+  *taken = nrows == 0;
+  if (*taken) return CELG_OK;
   const int base = row_ptr[0];
   const size_t total = (size_t)(row_ptr[nrows] - base);
   const int r0 = first_row - e->row_low;
   const size_t done = e->rp.empty() ? 0 : e->rp.size() - 1;  // rows begun so far
   const size_t at = e->rp.empty() ? 0 : (size_t)e->rp.back();
-  if (total < 4096 && nrows < e->n_local) return CELG_OK;
   if (r0 < (int)done || at + total >= (size_t)1 << 31 || (total > 0 && (!cols || !vals))) return CELG_OK;
   for (int i = 0; i < nrows; ++i)
     if (row_ptr[i + 1] < row_ptr[i]) return CELG_OK;
@@ -153,28 +202,21 @@ static int elm_append_rows(celg_handle* h, Elm* e, int first_row, int nrows, con
     for (int k = b + 1; k < end; ++k) bad |= cols[k] < cols[k - 1];
   }
   if (bad) return CELG_OK;
-  if (at + total > e->dcap || !e->dmat) {
-    celg_mat* m = new celg_mat();
-    m->h = h;
-    const size_t cap = std::max(std::max(at + total, e->hint), e->dmat ? 2 * e->dcap : 0);
-    if (const int st = alloc_csr_room(m, e->n_local, std::min(cap, ((size_t)1 << 31) - 1), e->n_local)) {
-      delete m;
-      return st;
+  const size_t held = e->held_vals.size();
+  int st = CELG_OK;
+  if (total < kElmHold) {
+    e->held_cols.insert(e->held_cols.end(), cols, cols + total);
+    e->held_vals.insert(e->held_vals.end(), vals, vals + total);
+    if (held + total >= kElmHold) st = elm_send_held(h, e);
+    if (st) {
+      e->held_cols.resize(held);
+      e->held_vals.resize(held);
     }
-    if (at) {
-      CELG_CUDA(cudaMemcpyAsync(m->csr.ci, e->dmat->csr.ci, sizeof(int) * at, cudaMemcpyDeviceToDevice, h->stream));
-      CELG_CUDA(cudaMemcpyAsync(m->csr.v, e->dmat->csr.v, sizeof(double) * at, cudaMemcpyDeviceToDevice, h->stream));
-    }
-    if (e->dmat) celg_mat_destroy(e->dmat);
-    e->dmat = m;
-    e->dcap = std::min(cap, ((size_t)1 << 31) - 1);
+  } else {
+    if (held) st = elm_send_held(h, e);
+    if (!st) st = elm_send(h, e, cols, vals, total);
   }
-  if (total) {
-    // (from pageable memory these return when the caller's arrays are read)
-    CELG_CUDA(cudaMemcpyAsync(e->dmat->csr.ci + at, cols, sizeof(int) * total, cudaMemcpyHostToDevice, h->stream));
-    CELG_CUDA(cudaMemcpyAsync(e->dmat->csr.v + at, vals, sizeof(double) * total, cudaMemcpyHostToDevice, h->stream));
-    CELG_CUDA(cudaStreamSynchronize(h->stream));
-  }
+  if (st) return st;
   if (e->rp.empty()) e->rp.push_back(0);
   e->rp.resize((size_t)r0 + 1, (int)at);  // rows left out are empty
   for (int i = 0; i < nrows; ++i) e->rp.push_back((int)at + row_ptr[i + 1] - base);
@@ -285,8 +327,10 @@ static int elm_complete_triplets(celg_handle* h, Elm* e, celg_mat** m) {
 static int elm_complete_direct(celg_handle* h, Elm* e, celg_mat** m) {
   const int nnz = e->rp.back();
   e->rp.resize((size_t)e->n_local + 1, nnz);
+  int st = elm_send_held(h, e);
+  if (st) return st;
   celg_mat* d = e->dmat;
-  int st = set_csr_entries(d, nnz);
+  st = set_csr_entries(d, nnz);
   if (st) return st;
   // (the row pointer is 1-based like the columns, for one conversion)
   for (int& v : e->rp) v += 1;
@@ -311,7 +355,7 @@ extern "C" int celg_elm_matrix_completed(celg_handle* h) {
   Elm* e = h->elm;
   if (e->completed || e->lost) return CELG_ERR_STATE;
   celg_mat* m = nullptr;
-  e->lost = e->direct && e->dmat;
+  e->lost = e->direct && !e->rp.empty();
   int st = e->lost ? elm_complete_direct(h, e, &m) : elm_complete_triplets(h, e, &m);
   if (st) return st;
   st = celg_mat_jacobi(m);

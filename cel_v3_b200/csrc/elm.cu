@@ -24,7 +24,7 @@ struct Elm {
   // pieces of a few rows are held here until there are enough for a copy.
   // Any other insertion moves the entries to rows/cols/vals above.
   bool direct = true;
-  bool lost = false;       // completing them failed: nothing is left to retry with
+  bool lost = false;       // a CUDA error while completing them: nothing is left to retry with
   std::vector<int> rp;     // one entry per row begun, and the end
   celg_mat* dmat = nullptr;
   size_t dcap = 0;         // entries dmat has room for
@@ -105,10 +105,11 @@ extern "C" int celg_elm_row_start(celg_handle* h, int row) {
   return CELG_OK;
 }
 
-// Leaves the direct mode: the entries so far become triplets on the host, in
-// the order they were inserted.
-static int elm_undirect(celg_handle* h, Elm* e) {
-  if (!e->direct) return CELG_OK;
+// Leaves the direct mode: the rows so far (`sent` of their entries in dmat, the
+// columns there from col_base; the rest held here) become triplets on the
+// host, in the order they were inserted.  vals_d: their values, null when
+// e->vals has them.
+static int elm_to_triplets(celg_handle* h, Elm* e, const double* vals_d, int col_base) {
   const size_t nnz = e->rp.empty() ? 0 : (size_t)e->rp.back();
   const size_t room = std::max(nnz, e->hint);
   e->rows.reserve(room);
@@ -119,8 +120,11 @@ static int elm_undirect(celg_handle* h, Elm* e) {
     e->vals.resize(nnz);
     if (e->sent) {
       CELG_CUDA(cudaMemcpyAsync(e->cols.data(), e->dmat->csr.ci, sizeof(int) * e->sent, cudaMemcpyDeviceToHost, h->stream));
-      CELG_CUDA(cudaMemcpyAsync(e->vals.data(), e->dmat->csr.v, sizeof(double) * e->sent, cudaMemcpyDeviceToHost, h->stream));
+      if (vals_d)
+        CELG_CUDA(cudaMemcpyAsync(e->vals.data(), vals_d, sizeof(double) * e->sent, cudaMemcpyDeviceToHost, h->stream));
       CELG_CUDA(cudaStreamSynchronize(h->stream));
+      if (col_base != 1)
+        for (size_t k = 0; k < e->sent; ++k) e->cols[k] += 1 - col_base;
     }
     std::copy(e->held_cols.begin(), e->held_cols.end(), e->cols.begin() + (long)e->sent);
     std::copy(e->held_vals.begin(), e->held_vals.end(), e->vals.begin() + (long)e->sent);
@@ -133,10 +137,16 @@ static int elm_undirect(celg_handle* h, Elm* e) {
   }
   if (e->dmat) celg_mat_destroy(e->dmat);
   e->dmat = nullptr;
+  e->rp.clear();
   e->held_cols.clear();
   e->held_vals.clear();
   e->direct = false;
   return CELG_OK;
+}
+
+static int elm_undirect(celg_handle* h, Elm* e) {
+  if (!e->direct) return CELG_OK;
+  return e->lost ? CELG_ERR_STATE : elm_to_triplets(h, e, e->dmat ? e->dmat->csr.v : nullptr, 1);
 }
 
 // Copies total entries (columns, values) behind those that dmat has.
@@ -324,7 +334,7 @@ static int elm_complete_triplets(celg_handle* h, Elm* e, celg_mat** m) {
 }
 
 // the rows are in place: their pointer follows
-static int elm_complete_direct(celg_handle* h, Elm* e, celg_mat** m) {
+static int elm_complete_direct(celg_handle* h, Elm* e) {
   const int nnz = e->rp.back();
   e->rp.resize((size_t)e->n_local + 1, nnz);
   int st = elm_send_held(h, e);
@@ -332,15 +342,29 @@ static int elm_complete_direct(celg_handle* h, Elm* e, celg_mat** m) {
   celg_mat* d = e->dmat;
   st = set_csr_entries(d, nnz);
   if (st) return st;
+  e->lost = true;  // until the columns, 0-based from here on, are known to be whole
   // (the row pointer is 1-based like the columns, for one conversion)
   for (int& v : e->rp) v += 1;
   const cudaError_t ce =
       cudaMemcpyAsync(d->csr.rp, e->rp.data(), sizeof(int) * e->rp.size(), cudaMemcpyHostToDevice, h->stream);
   st = ce == cudaSuccess ? finish_csr(h, d, 1) : cuda_status(ce, "ELM row pointer");
   for (int& v : e->rp) v -= 1;
-  if (st) return st;
-  *m = d;
-  e->dmat = nullptr;
+  if (!st) e->lost = false;
+  return st;
+}
+
+// Scaling overwrites the values that direct rows have on the device alone: a
+// copy of them for the forms whose set-up after it can run out of memory.
+static int elm_keep_values(celg_handle* h, Elm* e, const celg_mat* m, double** plain) {
+  const size_t bytes = sizeof(double) * (size_t)m->csr.nnz;
+  if (dev_alloc(h, plain, bytes) == cudaSuccess) {
+    CELG_CUDA(cudaMemcpyAsync(*plain, m->csr.v, bytes, cudaMemcpyDeviceToDevice, h->stream));
+    return CELG_OK;
+  }
+  (void)cudaGetLastError();
+  e->vals.resize((size_t)m->csr.nnz);
+  CELG_CUDA(cudaMemcpyAsync(e->vals.data(), m->csr.v, bytes, cudaMemcpyDeviceToHost, h->stream));
+  CELG_CUDA(cudaStreamSynchronize(h->stream));
   return CELG_OK;
 }
 
@@ -349,29 +373,59 @@ static int elm_complete_direct(celg_handle* h, Elm* e, celg_mat** m) {
 // src/fspmt/cel_sp_mat_module.f90:518-585; equal keys keep insertion order)
 // and the CSR row pointer (cel_sp_mat_to_csr, :430-456), both on the device;
 // then Jacobi, optional diagonal scaling (:375-388 of the ELM module), JAD
-// when selected.
+// when selected.  When a step fails (no memory left) the entries are kept, so
+// that the call can be repeated.
 extern "C" int celg_elm_matrix_completed(celg_handle* h) {
   if (!h || !h->elm) return CELG_ERR_STATE;
   Elm* e = h->elm;
   if (e->completed || e->lost) return CELG_ERR_STATE;
+  const bool direct = e->direct && !e->rp.empty();
   celg_mat* m = nullptr;
-  e->lost = e->direct && !e->rp.empty();
-  int st = e->lost ? elm_complete_direct(h, e, &m) : elm_complete_triplets(h, e, &m);
+  int st = direct ? elm_complete_direct(h, e) : elm_complete_triplets(h, e, &m);
   if (st) return st;
+  if (direct) m = e->dmat;
+  const size_t n = ((size_t)std::max(1, e->n_local) + 31) & ~(size_t)31;
+  const bool jad = e->params.fmt == CELG_FMT_JAD, fp32 = e->params.precision == CELG_PREC_FP32_IR;
+  double* plain = nullptr;
   st = celg_mat_jacobi(m);
-  if (!st && e->diag_scaling) st = celg_mat_scale_diagonal(m);
-  if (!st && e->params.fmt == CELG_FMT_JAD) st = celg_mat_to_jad(m, nullptr);
-  if (!st && e->params.precision == CELG_PREC_FP32_IR) st = celg_mat_make_fp32(m);
+  if (!st && !e->b_d && dev_alloc(h, &e->b_d, sizeof(double) * 2 * n) != cudaSuccess) {
+    (void)cudaGetLastError();
+    st = CELG_ERR_CUDA;
+  }
+  e->x_d = e->b_d + n;
+  if (!st && direct && e->diag_scaling && (jad || fp32)) st = elm_keep_values(h, e, m, &plain);
+  auto forms = [&]() -> int {
+    int s = e->diag_scaling ? celg_mat_scale_diagonal(m) : CELG_OK;
+    if (!s && jad) s = celg_mat_to_jad(m, nullptr);
+    if (!s && fp32) s = celg_mat_make_fp32(m);
+    return s;
+  };
+  if (!st) st = forms();
+  if (st && plain) {
+    // the copy may be what there was no room beside: to the host with it
+    e->vals.resize((size_t)m->csr.nnz);
+    if (cudaMemcpyAsync(e->vals.data(), plain, sizeof(double) * e->vals.size(), cudaMemcpyDeviceToHost, h->stream) ==
+            cudaSuccess &&
+        cudaStreamSynchronize(h->stream) == cudaSuccess) {
+      dev_free(h, plain, false);
+      plain = nullptr;
+      st = forms();
+    }
+  }
+  dev_free(h, plain);
   if (st) {
-    celg_mat_destroy(m);
+    if (!direct) {
+      celg_mat_destroy(m);
+    } else if (m->scaled && e->vals.empty()) {
+      e->lost = true;
+    } else {
+      e->lost = elm_to_triplets(h, e, m->scaled ? nullptr : m->csr.v, 0) != CELG_OK;
+    }
     return st;
   }
   e->mat = m;
-  const size_t n = ((size_t)std::max(1, e->n_local) + 31) & ~(size_t)31;
-  if (dev_alloc(h, &e->b_d, sizeof(double) * 2 * n) != cudaSuccess) return CELG_ERR_CUDA;
-  e->x_d = e->b_d + n;
+  e->dmat = nullptr;
   e->completed = true;
-  e->lost = false;
   std::vector<int>().swap(e->rp);
   std::vector<int>().swap(e->rows);
   std::vector<int>().swap(e->cols);

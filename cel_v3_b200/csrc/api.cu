@@ -21,6 +21,12 @@ int cuda_status(cudaError_t e, const char* what) {
   return CELG_ERR_CUDA;
 }
 
+bool out_of_memory(cudaError_t e) {
+  if (e != cudaErrorMemoryAllocation) return false;
+  (void)cudaGetLastError();
+  return true;
+}
+
 // ---- device blocks of a handle ------------------------------------------------
 
 cudaError_t dev_alloc_bytes(celg_handle* h, void** p, size_t bytes) {
@@ -296,16 +302,17 @@ constexpr int kCsrPad = 32;
 static size_t block(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
 
 // room for nnz_cap entries; the entry count and the padding are set later
-int alloc_csr_room(celg_mat* m, int n, size_t nnz_cap, int ncols) {
+cudaError_t alloc_csr_room(celg_mat* m, int n, size_t nnz_cap, int ncols) {
   m->csr.n = n;
   m->csr.ncols = ncols;
   const size_t rp = block(sizeof(int) * ((size_t)n + 1 + 8)), ci = block(sizeof(int) * (nnz_cap + kCsrPad));
   unsigned char* p = nullptr;
-  CELG_CUDA(dev_alloc(m->h, &p, rp + ci + sizeof(double) * (nnz_cap + kCsrPad)));
+  const cudaError_t e = dev_alloc(m->h, &p, rp + ci + sizeof(double) * (nnz_cap + kCsrPad));
+  if (e != cudaSuccess) return e;
   m->csr.rp = reinterpret_cast<int*>(p);
   m->csr.ci = reinterpret_cast<int*>(p + rp);
   m->csr.v = reinterpret_cast<double*>(p + rp + ci);
-  return CELG_OK;
+  return cudaSuccess;
 }
 
 int set_csr_entries(celg_mat* m, int nnz) {
@@ -316,8 +323,8 @@ int set_csr_entries(celg_mat* m, int nnz) {
 }
 
 int alloc_csr(celg_mat* m, int n, int nnz, int ncols) {
-  const int st = alloc_csr_room(m, n, (size_t)nnz, ncols);
-  return st ? st : set_csr_entries(m, nnz);
+  CELG_CUDA(alloc_csr_room(m, n, (size_t)nnz, ncols));
+  return set_csr_entries(m, nnz);
 }
 
 int finish_csr(celg_handle* h, celg_mat* m, int base) {

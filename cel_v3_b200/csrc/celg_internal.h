@@ -196,6 +196,10 @@ int cuda_status(cudaError_t e, const char* what);
     if (e_ != cudaSuccess) return ::celg::cuda_status(e_, #call); \
   } while (0)
 
+// e says that there was no memory (the error is cleared): what is only kept
+// for speed is then left out.
+bool out_of_memory(cudaError_t e);
+
 // Device memory of the handle's matrices.  Blocks given back are kept for
 // later requests on the handle, in the order of its stream, up to
 // kSpareBytes in all (getting and returning a block costs 0.1-0.2 ms each,
@@ -267,7 +271,7 @@ int row_forms_build(celg_handle* h, CsrDev& A, bool with_values);
 int row_forms_jacobi(celg_handle* h, CsrDev& A, const double* J);
 void row_forms_free(celg_handle* h, CsrDev& A, bool keep = true);
 int alloc_csr(celg_mat* m, int n, int nnz, int ncols);
-int alloc_csr_room(celg_mat* m, int n, size_t nnz_cap, int ncols);
+cudaError_t alloc_csr_room(celg_mat* m, int n, size_t nnz_cap, int ncols);
 int set_csr_entries(celg_mat* m, int nnz);
 int finish_csr(celg_handle* h, celg_mat* m, int base);
 void free_mat_arrays(celg_mat* m);

@@ -149,17 +149,26 @@ static int elm_undirect(celg_handle* h, Elm* e) {
   return e->lost ? CELG_ERR_STATE : elm_to_triplets(h, e, e->dmat ? e->dmat->csr.v : nullptr, 1);
 }
 
-// Copies total entries (columns, values) behind those that dmat has.
-static int elm_send(celg_handle* h, Elm* e, const int* cols, const double* vals, size_t total) {
+// Copies total entries (columns, values) behind those that dmat has; *room =
+// false (and nothing done) when there is no device memory for them.
+static int elm_send(celg_handle* h, Elm* e, const int* cols, const double* vals, size_t total, bool* room) {
+  *room = true;
   const size_t need = e->sent + total;
   if (need > e->dcap || !e->dmat) {
     celg_mat* m = new celg_mat();
     m->h = h;
-    const size_t cap =
+    size_t cap =
         std::min(std::max(std::max(need, e->hint), e->dmat ? 2 * e->dcap : 0), ((size_t)1 << 31) - 1);
-    if (const int st = alloc_csr_room(m, e->n_local, cap, e->n_local)) {
+    cudaError_t ce = alloc_csr_room(m, e->n_local, cap, e->n_local);
+    if (ce == cudaErrorMemoryAllocation && cap > need) {
+      (void)cudaGetLastError();
+      cap = need;
+      ce = alloc_csr_room(m, e->n_local, cap, e->n_local);
+    }
+    if (ce != cudaSuccess) {
       delete m;
-      return st;
+      *room = !out_of_memory(ce);
+      return *room ? cuda_status(ce, "ELM rows") : CELG_OK;
     }
     if (e->sent) {
       CELG_CUDA(cudaMemcpyAsync(m->csr.ci, e->dmat->csr.ci, sizeof(int) * e->sent, cudaMemcpyDeviceToDevice, h->stream));
@@ -179,16 +188,17 @@ static int elm_send(celg_handle* h, Elm* e, const int* cols, const double* vals,
   return CELG_OK;
 }
 
-static int elm_send_held(celg_handle* h, Elm* e) {
-  const int st = elm_send(h, e, e->held_cols.data(), e->held_vals.data(), e->held_vals.size());
-  if (st) return st;
+static int elm_send_held(celg_handle* h, Elm* e, bool* room) {
+  const int st = elm_send(h, e, e->held_cols.data(), e->held_vals.data(), e->held_vals.size(), room);
+  if (st || !*room) return st;
   e->held_cols.clear();
   e->held_vals.clear();
   return CELG_OK;
 }
 
 // Whole rows in order with ascending columns, appended to dmat; *taken is
-// false (and nothing done) when the rows are not of that kind.  Copies of
+// false (and nothing done) when the rows are not of that kind, or the device
+// has no room for them.  Copies of
 // their own cost about 25 us a call, so short pieces are held on the host
 // until kElmHold entries are together.
 constexpr size_t kElmHold = 4096;
@@ -214,19 +224,20 @@ static int elm_append_rows(celg_handle* h, Elm* e, int first_row, int nrows, con
   if (bad) return CELG_OK;
   const size_t held = e->held_vals.size();
   int st = CELG_OK;
+  bool room = true;
   if (total < kElmHold) {
     e->held_cols.insert(e->held_cols.end(), cols, cols + total);
     e->held_vals.insert(e->held_vals.end(), vals, vals + total);
-    if (held + total >= kElmHold) st = elm_send_held(h, e);
-    if (st) {
+    if (held + total >= kElmHold) st = elm_send_held(h, e, &room);
+    if (st || !room) {
       e->held_cols.resize(held);
       e->held_vals.resize(held);
     }
   } else {
-    if (held) st = elm_send_held(h, e);
-    if (!st) st = elm_send(h, e, cols, vals, total);
+    if (held) st = elm_send_held(h, e, &room);
+    if (!st && room) st = elm_send(h, e, cols, vals, total, &room);
   }
-  if (st) return st;
+  if (st || !room) return st;
   if (e->rp.empty()) e->rp.push_back(0);
   e->rp.resize((size_t)r0 + 1, (int)at);  // rows left out are empty
   for (int i = 0; i < nrows; ++i) e->rp.push_back((int)at + row_ptr[i + 1] - base);
@@ -333,12 +344,15 @@ static int elm_complete_triplets(celg_handle* h, Elm* e, celg_mat** m) {
   return st;
 }
 
-// the rows are in place: their pointer follows
+// the rows are in place: their pointer follows (without room for the last of
+// them they become triplets)
 static int elm_complete_direct(celg_handle* h, Elm* e) {
   const int nnz = e->rp.back();
   e->rp.resize((size_t)e->n_local + 1, nnz);
-  int st = elm_send_held(h, e);
-  if (st) return st;
+  bool room = true;
+  int st = elm_send_held(h, e, &room);
+  if (!st && !room) st = elm_undirect(h, e);
+  if (st || !room) return st;
   celg_mat* d = e->dmat;
   st = set_csr_entries(d, nnz);
   if (st) return st;
@@ -379,11 +393,11 @@ extern "C" int celg_elm_matrix_completed(celg_handle* h) {
   if (!h || !h->elm) return CELG_ERR_STATE;
   Elm* e = h->elm;
   if (e->completed || e->lost) return CELG_ERR_STATE;
-  const bool direct = e->direct && !e->rp.empty();
-  celg_mat* m = nullptr;
-  int st = direct ? elm_complete_direct(h, e) : elm_complete_triplets(h, e, &m);
+  int st = e->direct && !e->rp.empty() ? elm_complete_direct(h, e) : CELG_OK;
   if (st) return st;
-  if (direct) m = e->dmat;
+  const bool direct = e->direct && !e->rp.empty();
+  celg_mat* m = direct ? e->dmat : nullptr;
+  if (!direct && (st = elm_complete_triplets(h, e, &m))) return st;
   const size_t n = ((size_t)std::max(1, e->n_local) + 31) & ~(size_t)31;
   const bool jad = e->params.fmt == CELG_FMT_JAD, fp32 = e->params.precision == CELG_PREC_FP32_IR;
   double* plain = nullptr;

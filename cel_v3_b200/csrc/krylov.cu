@@ -789,7 +789,11 @@ static int gm_plan_orth(celg_handle* h, GmPlan* g) {
   CELG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gm_orth_kernel, kGmThreads, kGmSmem));
   if (per_sm < 1) return CELG_OK;
   const size_t bytes = 256 + sizeof(ulonglong2) * (size_t)(kGmMaxTiles + 1);
-  if (!h->gm_exch) CELG_CUDA(cudaMalloc(&h->gm_exch, bytes));
+  if (!h->gm_exch) {
+    const cudaError_t em = cudaMalloc(&h->gm_exch, bytes);
+    if (out_of_memory(em)) return CELG_OK;
+    CELG_CUDA(em);
+  }
   CELG_CUDA(cudaMemsetAsync(h->gm_exch, 0, bytes, h->stream));
   g->ex.count = static_cast<unsigned long long*>(h->gm_exch);
   g->ex.word = static_cast<ulonglong2*>(h->gm_exch) + 15;

@@ -986,7 +986,8 @@ static float*& sell_vals(CsrDev& A, const float*) { return A.sell_v32; }
 
 // Builds the sliced copy once; *ok = false when its padding is not worth it
 // (more than twice the entries plus one slice row per slice: a few very long
-// rows among short ones), which leaves the matrix to the graph of sweeps.
+// rows among short ones) or there is no memory for it, which leaves the
+// matrix to the graph of sweeps.
 template <typename VT>
 static int ensure_sell(celg_handle* h, CsrDev& A, const VT* vals, bool* ok) {
   *ok = false;
@@ -1021,6 +1022,7 @@ static int ensure_sell(celg_handle* h, CsrDev& A, const VT* vals, bool* ok) {
       dev_free(h, tmp);
       if (e != cudaSuccess || longest > kMaxWidth || 32L * total > 2L * A.nnz + 32 * nslices) {
         dev_free(h, base);
+        if (out_of_memory(e)) return CELG_OK;
         A.sell_total = 0;
         return e != cudaSuccess ? cuda_status(e, "sliced matrix") : CELG_OK;
       }
@@ -1041,7 +1043,7 @@ static int ensure_sell(celg_handle* h, CsrDev& A, const VT* vals, bool* ok) {
     }
     if (e != cudaSuccess) {
       sell_free(h, A);
-      return cuda_status(e, "sliced matrix");
+      return out_of_memory(e) ? CELG_OK : cuda_status(e, "sliced matrix");
     }
   }
   *ok = true;
@@ -1187,15 +1189,26 @@ static int onchip_launch(cudaStream_t stream, CsrDev& A, const PcgBind<VT>& B, c
                : launch_onchip<VT, false>(stream, a, q.grid, q.smem, done);
 }
 
-static int onchip_words(celg_handle* h, size_t words) {
-  if (words > h->oc_cap) {
-    CELG_CUDA(cudaStreamSynchronize(h->stream));
-    cudaFree(h->oc_slots);
-    h->oc_slots = nullptr;
-    h->oc_cap = 0;
-    CELG_CUDA(cudaMalloc(&h->oc_slots, sizeof(double) * words));
-    h->oc_cap = words;
-  }
+// *ok = false: no memory for a buffer of the handle's that has to grow to
+// `need` doubles
+static int onchip_grow(celg_handle* h, double** buf, size_t* cap, size_t need, bool* ok) {
+  *ok = true;
+  if (need <= *cap) return CELG_OK;
+  CELG_CUDA(cudaStreamSynchronize(h->stream));
+  cudaFree(*buf);
+  *buf = nullptr;
+  *cap = 0;
+  const cudaError_t e = cudaMalloc(buf, sizeof(double) * need);
+  *ok = !out_of_memory(e);
+  if (!*ok) return CELG_OK;
+  CELG_CUDA(e);
+  *cap = need;
+  return CELG_OK;
+}
+
+static int onchip_words(celg_handle* h, size_t words, bool* ok) {
+  const int st = onchip_grow(h, &h->oc_slots, &h->oc_cap, words, ok);
+  if (st || !*ok) return st;
   CELG_CUDA(cudaMemsetAsync(h->oc_slots, 0xff, sizeof(double) * words, h->stream));
   return CELG_OK;
 }
@@ -1208,8 +1221,8 @@ int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_param
   bool ok = false;
   int st = onchip_matrix<VT>(h, A, B.vals, q, &ok);
   if (st || !ok) return st;
-  st = onchip_words(h, q.words());
-  if (st) return st;
+  st = onchip_words(h, q.words(), &ok);
+  if (st || !ok) return st;
   return onchip_launch<VT>(h->stream, A, B, p, q, h->oc_slots, h->state_h, h->hist_d, hist_cap, done);
 }
 
@@ -1263,37 +1276,40 @@ int pcg_onchip_many(celg_handle* h, int count, celg_mat* const* mats, const doub
     longest = std::max(longest, t);
   }
   if (std::max(kernels, longest) >= sweeps + 24.0 * slowest) return CELG_OK;
+  bool ok = true;
+  std::vector<CsrDev*> built;
   for (const Job& j : jobs) {
-    bool ok = false;
     CsrDev& A = mats[j.sys]->csr;
+    const bool had = A.sell_v != nullptr;
     const int st = onchip_matrix<double>(h, A, A.v, j.q, &ok);
-    if (st || !ok) return st;
+    if (!had && A.sell_v) built.push_back(&A);
+    if (!st && ok) continue;
+    // one has none: the sweeps need no copy of the others
+    if (!st) CELG_CUDA(cudaStreamSynchronize(h->stream));
+    for (CsrDev* B : built) sell_free(h, *B);
+    return st;
   }
   // work vectors p and v of every lane, as long as the largest system
   size_t room = 32;
   for (const Job& j : jobs) room = std::max(room, ((size_t)mats[j.sys]->csr.n + 31) & ~(size_t)31);
   const size_t work = 2 * kOcLanes * room;
-  if (work > h->oc_work_cap) {
-    CELG_CUDA(cudaStreamSynchronize(h->stream));
-    cudaFree(h->oc_work);
-    h->oc_work = nullptr;
-    h->oc_work_cap = 0;
-    CELG_CUDA(cudaMalloc(&h->oc_work, sizeof(double) * work));
-    h->oc_work_cap = work;
-  }
+  int st = onchip_grow(h, &h->oc_work, &h->oc_work_cap, work, &ok);
+  if (st || !ok) return st;
   if (count > h->oc_states_cap) {
     cudaFreeHost(h->oc_states);
     h->oc_states = nullptr;
     h->oc_states_cap = 0;
-    CELG_CUDA(cudaMallocHost(&h->oc_states, sizeof(PcgState) * (size_t)count));
+    const cudaError_t e = cudaMallocHost(&h->oc_states, sizeof(PcgState) * (size_t)count);
+    if (out_of_memory(e)) return CELG_OK;
+    CELG_CUDA(e);
     h->oc_states_cap = count;
   }
   for (int l = 0; l < kOcLanes; ++l) {
     if (l && !h->oc_lane[l]) CELG_CUDA(cudaStreamCreateWithFlags(&h->oc_lane[l], cudaStreamNonBlocking));
     if (!h->oc_event[l]) CELG_CUDA(cudaEventCreateWithFlags(&h->oc_event[l], cudaEventDisableTiming));
   }
-  int st = onchip_words(h, std::max<size_t>(words, 1));
-  if (st) return st;
+  st = onchip_words(h, std::max<size_t>(words, 1), &ok);
+  if (st || !ok) return st;
   std::stable_sort(jobs.begin(), jobs.end(),
                    [&](const Job& a, const Job& c) { return mats[a.sys]->csr.n > mats[c.sys]->csr.n; });
   const Job* first = nullptr;

@@ -226,8 +226,8 @@ int row_forms_search(celg_handle* h, const CsrDev& A, bool with_values, const in
   return CELG_OK;
 }
 
-// Builds the forms the search found (the stream has been waited for).  On a
-// failed allocation the matrix keeps its plain columns.
+// Builds the forms the search found (the stream has been waited for).  Without
+// memory for them the matrix keeps its plain columns.
 int row_forms_build(celg_handle* h, CsrDev& A, bool with_values) {
   row_forms_free(h, A);
   if (A.n == 0 || A.nnz == 0) return CELG_OK;
@@ -245,7 +245,9 @@ int row_forms_build(celg_handle* h, CsrDev& A, bool with_values) {
     const size_t ints = (size_t)np * (kPatLen + 2);
     const size_t tab = ((ints * sizeof(int) + 15) & ~(size_t)15);
     const size_t bytes = (tab + (size_t)np * (kPatLen * 12) + kPatMax * 12 + (size_t)np * 8 + 64 + 255) & ~(size_t)255;
-    CELG_CUDA(dev_alloc(h, &A.pat, bytes + (size_t)A.n + 16));
+    const cudaError_t em = dev_alloc(h, &A.pat, bytes + (size_t)A.n + 16);
+    if (out_of_memory(em)) return CELG_OK;
+    CELG_CUDA(em);
     A.pid = reinterpret_cast<uint8_t*>(A.pat) + bytes;
     A.npat = np;
     A.plen = A.pat + (size_t)np * kPatLen;

@@ -37,6 +37,87 @@ def handle(celgpu, torch):
     return celgpu.Handle(0, torch.cuda.current_stream().cuda_stream)
 
 
+def band(n, half):
+    """Dense band: 2 half + 1 entries a row, no row patterns."""
+    import scipy.sparse as sp
+    off = list(range(-half, half + 1))
+    A = sp.diags([np.full(n - abs(o), -1.0 / (1 + abs(o)) if o else 8.0) for o in off], off).tocsr()
+    A.sort_indices()
+    return A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
+
+
+def test_pcg_without_room_for_the_sliced_copy(gpu, monkeypatch):
+    celgpu, _, torch = gpu
+    h = handle(celgpu, torch)
+    m = h.matrix_from_csr(*band(600000, 10)).jacobi()
+    b = torch.linspace(-1, 1, m.n, dtype=torch.float64, device="cuda")
+    x = torch.zeros_like(b)
+    kw = dict(eps_rel=1e-9, iter_max=400, x0_mode=celgpu.X0_ZERO)
+    monkeypatch.setenv("CELG_ONCHIP_ROWS", "0")
+    i = h.pcg_jacobi(m, b.data_ptr(), x.data_ptr(), **kw)
+    want = x.cpu().numpy()
+    monkeypatch.delenv("CELG_ONCHIP_ROWS")
+    f = Filled(torch, 64 * MB)
+    try:
+        j = h.pcg_jacobi(m, b.data_ptr(), x.data_ptr(), **kw)
+        got = x.cpu().numpy()
+    finally:
+        f.release()
+    assert j.status == celgpu.OK and j.iter_done == i.iter_done and np.array_equal(got, want)
+    j = h.pcg_jacobi(m, b.data_ptr(), x.data_ptr(), **kw)  # and on chip once there is room
+    assert j.iter_done == i.iter_done and np.array_equal(x.cpu().numpy(), want)
+    m.destroy()
+    h.close()
+
+
+def test_batch_without_room_for_its_kernels(gpu, monkeypatch):
+    celgpu, _, torch = gpu
+    h = handle(celgpu, torch)
+    mats = [h.matrix_from_csr(*band(n, 10)).jacobi() for n in (600000, 20000)]
+    b = [torch.linspace(-1, 1, m.n, dtype=torch.float64, device="cuda") for m in mats]
+    x = [torch.zeros_like(t) for t in b]
+    kw = dict(eps_rel=1e-9, iter_max=400, x0_mode=celgpu.X0_ZERO)
+
+    def batch():
+        i = h.pcg_batched(mats, [t.data_ptr() for t in b], [t.data_ptr() for t in x], **kw)
+        return [q.iter_done for q in i], [t.cpu().numpy() for t in x]
+
+    monkeypatch.setenv("CELG_ONCHIP_ROWS", "0")
+    want = batch()
+    monkeypatch.delenv("CELG_ONCHIP_ROWS")
+    f = Filled(torch, 64 * MB)
+    try:
+        got = batch()
+    finally:
+        f.release()
+    assert got[0] == want[0] and all(np.array_equal(p, q) for p, q in zip(got[1], want[1]))
+    for m in mats:
+        m.destroy()
+    h.close()
+
+
+def test_matrix_without_room_for_its_row_forms(gpu):
+    celgpu, _, torch = gpu
+    h = handle(celgpu, torch)
+    n = 48 * MB
+    rp = torch.arange(n + 1, dtype=torch.int32, device="cuda")
+    v = torch.full((n,), 3.0, dtype=torch.float64, device="cuda")
+    x = torch.linspace(-1, 1, n, dtype=torch.float64, device="cuda")
+    y = torch.zeros_like(x)
+    f = Filled(torch, 16 * n + 4 * MB)  # the CSR block, not the byte a row
+    try:
+        m = h.matrix_from_csr_device(n, n, rp.data_ptr(), rp.data_ptr(), v.data_ptr())
+        form = m.column_form()
+        h.spmv(m, x.data_ptr(), y.data_ptr())
+        torch.cuda.synchronize()
+    finally:
+        f.release()
+    assert form == celgpu.COLS_INT32
+    assert torch.equal(y, 3.0 * x)
+    m.destroy()
+    h.close()
+
+
 def elm_system():
     _, k = synth.lognormal_faces(np.random.default_rng(1), 90, 88, 86, 0.5)
     rp, ci, v = synth.diffusion7(90, 88, 86, *k)
@@ -75,6 +156,33 @@ def test_elm_completion_can_be_repeated(gpu, scaling):
             h.elm_insert_rows(1, rp, ci, w)
         h.elm_matrix_completed()
         got.append((h.elm_doit(b)[1], h.elm_collect_solution(n)))
+        h.elm_destroy()
+        h.close()
+    assert got[0][0] == got[1][0] and np.array_equal(got[0][1], got[1][1])
+
+
+def test_elm_rows_without_room_on_the_device(gpu):
+    """They wait on the host, as rows that come entry by entry do."""
+    celgpu, _, torch = gpu
+    rp, ci, v = elm_system()
+    n = rp.size - 1
+    b = np.random.default_rng(2).uniform(-1, 1, n)
+    got = []
+    for short in (False, True):
+        h = handle(celgpu, torch)
+        h.elm_init(n, nnz_hint=(0, 0))
+        h.elm_set_solver(celgpu.SOLVER_PCG, celgpu.params(eps_rel=1e-6, iter_max=300))
+        if short:
+            h.elm_insert_rows(1, rp[:2001], ci[:rp[2000]], v[:rp[2000]])
+            f = Filled(torch, 8 * MB)
+            try:
+                h.elm_insert_rows(2001, rp[2000:], ci[rp[2000]:], v[rp[2000]:])
+            finally:
+                f.release()
+        else:
+            h.elm_insert_rows(1, rp, ci, v)
+        h.elm_matrix_completed()
+        got.append((h.elm_doit(b)[1:], h.elm_collect_solution(n)))
         h.elm_destroy()
         h.close()
     assert got[0][0] == got[1][0] and np.array_equal(got[0][1], got[1][1])

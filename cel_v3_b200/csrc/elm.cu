@@ -157,8 +157,10 @@ static int elm_send(celg_handle* h, Elm* e, const int* cols, const double* vals,
   if (need > e->dcap || !e->dmat) {
     celg_mat* m = new celg_mat();
     m->h = h;
-    size_t cap =
-        std::min(std::max(std::max(need, e->hint), e->dmat ? 2 * e->dcap : 0), ((size_t)1 << 31) - 1);
+    // (a hint is taken up to twice what is there: it may be far too large, and
+    // the room stays with the matrix)
+    const size_t room_for = std::max(std::max(need, std::min(e->hint, 2 * need)), e->dmat ? 2 * e->dcap : 0);
+    size_t cap = std::min(room_for, ((size_t)1 << 31) - 1);
     cudaError_t ce = alloc_csr_room(m, e->n_local, cap, e->n_local);
     if (ce == cudaErrorMemoryAllocation && cap > need) {
       (void)cudaGetLastError();

@@ -161,6 +161,23 @@ def test_elm_completion_can_be_repeated(gpu, scaling):
     assert got[0][0] == got[1][0] and np.array_equal(got[0][1], got[1][1])
 
 
+def test_elm_hint_is_no_device_memory(gpu):
+    celgpu, _, torch = gpu
+    rp, ci, v = elm_system()
+    n = rp.size - 1
+    h = handle(celgpu, torch)
+    h.elm_init(n, nnz_hint=(300, 0))  # 2.4 GB if all of it were taken
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    h.elm_insert_rows(1, rp[:30001], ci[:rp[30000]], v[:rp[30000]])
+    assert before - torch.cuda.mem_get_info()[0] < 64 * MB
+    h.elm_insert_rows(30001, rp[30000:], ci[rp[30000]:], v[rp[30000]:])
+    assert before - torch.cuda.mem_get_info()[0] < 256 * MB
+    h.elm_matrix_completed()
+    h.elm_destroy()
+    h.close()
+
+
 def test_elm_rows_without_room_on_the_device(gpu):
     """They wait on the host, as rows that come entry by entry do."""
     celgpu, _, torch = gpu

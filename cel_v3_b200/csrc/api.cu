@@ -45,13 +45,18 @@ cudaError_t dev_alloc_bytes(celg_handle* h, void** p, size_t bytes) {
     *p = h->blocks.back().p;
     return cudaSuccess;
   }
+  const cudaError_t e = raw_alloc_bytes(h, p, bytes);
+  if (e == cudaSuccess) h->blocks.push_back({*p, bytes});
+  return e;
+}
+
+cudaError_t raw_alloc_bytes(celg_handle* h, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation && !h->spare.empty()) {
     (void)cudaGetLastError();
     dev_free_spare(h);
     e = cudaMalloc(p, bytes);
   }
-  if (e == cudaSuccess) h->blocks.push_back({*p, bytes});
   return e;
 }
 
@@ -73,7 +78,6 @@ void dev_free(celg_handle* h, void* p, bool keep) {
 }
 
 void dev_free_spare(celg_handle* h) {
-  cudaStreamSynchronize(h->stream);
   for (const celg_handle::DevBlock& b : h->spare) cudaFree(b.p);
   h->spare.clear();
   h->spare_bytes = 0;
@@ -225,7 +229,7 @@ int build_offset_dict_csr(celg_handle* h, CsrDev& A) {
   A.ndict = 0;
   if (A.n == 0 || A.nnz == 0) return CELG_OK;
   int* table = nullptr;
-  CELG_CUDA(cudaMalloc(&table, sizeof(int) * (kOffSlots + 2)));
+  CELG_CUDA(raw_alloc(h, &table, sizeof(int) * (kOffSlots + 2)));
   std::vector<int> init(kOffSlots + 2, kOffEmpty);
   init[kOffSlots] = 0;
   init[kOffSlots + 1] = 0;
@@ -243,8 +247,8 @@ int build_offset_dict_csr(celg_handle* h, CsrDev& A) {
     if (out[q] != kOffEmpty) dict.push_back(out[q]);
   std::sort(dict.begin(), dict.end());
   // on any failure the matrix keeps its int32 columns only
-  e = cudaMalloc(&A.dict, sizeof(int) * dict.size());
-  if (e == cudaSuccess) e = cudaMalloc(&A.ci8, (size_t)A.nnz + 32);
+  e = raw_alloc(h, &A.dict, sizeof(int) * dict.size());
+  if (e == cudaSuccess) e = raw_alloc(h, &A.ci8, (size_t)A.nnz + 32);
   if (e == cudaSuccess) e = cudaMemsetAsync(A.ci8 + A.nnz, 0, 32, h->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(A.dict, dict.data(), sizeof(int) * dict.size(), cudaMemcpyHostToDevice, h->stream);
@@ -369,15 +373,15 @@ static int build_jad(celg_mat* m) {
   int mmax = 0;
   cudaError_t e;
   do {
-    if ((e = cudaMalloc(&key, sizeof(int) * std::max(1, n))) != cudaSuccess) { fail(e, "jad"); break; }
-    if ((e = cudaMalloc(&key2, sizeof(int) * std::max(1, n))) != cudaSuccess) { fail(e, "jad"); break; }
-    if ((e = cudaMalloc(&idx, sizeof(int) * std::max(1, n))) != cudaSuccess) { fail(e, "jad"); break; }
-    if ((e = cudaMalloc(&J.perm, sizeof(int) * std::max(1, n))) != cudaSuccess) { fail(e, "jad"); break; }
+    if ((e = raw_alloc(h, &key, sizeof(int) * std::max(1, n))) != cudaSuccess) { fail(e, "jad"); break; }
+    if ((e = raw_alloc(h, &key2, sizeof(int) * std::max(1, n))) != cudaSuccess) { fail(e, "jad"); break; }
+    if ((e = raw_alloc(h, &idx, sizeof(int) * std::max(1, n))) != cudaSuccess) { fail(e, "jad"); break; }
+    if ((e = raw_alloc(h, &J.perm, sizeof(int) * std::max(1, n))) != cudaSuccess) { fail(e, "jad"); break; }
     cudaMemsetAsync(maxlen_d, 0, sizeof(int), h->stream);
     if (n > 0) row_len_kernel<<<ew_grid(h, n), 256, 0, h->stream>>>(n, m->csr.rp, key, idx, maxlen_d);
     cudaMemcpyAsync(&mmax, maxlen_d, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
     if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) { fail(e, "jad lengths"); break; }
-    if ((e = cudaMalloc(&hist, sizeof(int) * (size_t)(mmax + 1))) != cudaSuccess) { fail(e, "jad"); break; }
+    if ((e = raw_alloc(h, &hist, sizeof(int) * (size_t)(mmax + 1))) != cudaSuccess) { fail(e, "jad"); break; }
     cudaMemsetAsync(hist, 0, sizeof(int) * (size_t)(mmax + 1), h->stream);
     if (n > 0) jad_key_kernel<<<ew_grid(h, n), 256, 0, h->stream>>>(n, mmax, key, hist);
     int bits = 1;
@@ -385,7 +389,7 @@ static int build_jad(celg_mat* m) {
     size_t tmp_bytes = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, key, key2, idx, J.perm, n, 0, bits,
                                     h->stream);
-    if ((e = cudaMalloc(&tmp, std::max<size_t>(tmp_bytes, 16))) != cudaSuccess) { fail(e, "jad"); break; }
+    if ((e = raw_alloc(h, &tmp, std::max<size_t>(tmp_bytes, 16))) != cudaSuccess) { fail(e, "jad"); break; }
     if (n > 0 && (e = cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, key, key2, idx, J.perm, n, 0,
                                                       bits, h->stream)) != cudaSuccess) {
       fail(e, "radix sort");
@@ -402,9 +406,9 @@ static int build_jad(celg_mat* m) {
       above -= hh[(size_t)k];  // remove rows of length k
       jb[(size_t)k + 1] = jb[(size_t)k] + above;
     }
-    if ((e = cudaMalloc(&J.begin, sizeof(int) * (size_t)(mmax + 1))) != cudaSuccess) { fail(e, "jad"); break; }
-    if ((e = cudaMalloc(&J.ci, sizeof(int) * ((size_t)nnz + 8))) != cudaSuccess) { fail(e, "jad"); break; }
-    if ((e = cudaMalloc(&J.v, sizeof(double) * ((size_t)nnz + 8))) != cudaSuccess) { fail(e, "jad"); break; }
+    if ((e = raw_alloc(h, &J.begin, sizeof(int) * (size_t)(mmax + 1))) != cudaSuccess) { fail(e, "jad"); break; }
+    if ((e = raw_alloc(h, &J.ci, sizeof(int) * ((size_t)nnz + 8))) != cudaSuccess) { fail(e, "jad"); break; }
+    if ((e = raw_alloc(h, &J.v, sizeof(double) * ((size_t)nnz + 8))) != cudaSuccess) { fail(e, "jad"); break; }
     cudaMemcpyAsync(J.begin, jb.data(), sizeof(int) * (size_t)(mmax + 1), cudaMemcpyHostToDevice,
                     h->stream);
     if (n > 0)
@@ -412,7 +416,7 @@ static int build_jad(celg_mat* m) {
                                                           J.begin, J.ci, J.v);
     // the pattern index of each permuted row, when the matrix has row patterns
     if (m->csr.pid && n > 0) {
-      if ((e = cudaMalloc(&J.pid, (size_t)n + 16)) != cudaSuccess) { fail(e, "jad"); break; }
+      if ((e = raw_alloc(h, &J.pid, (size_t)n + 16)) != cudaSuccess) { fail(e, "jad"); break; }
       jad_pid_kernel<<<ew_grid(h, n), 256, 0, h->stream>>>(n, J.perm, m->csr.pid, J.pid);
     }
     if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) { fail(e, "jad fill"); break; }
@@ -896,8 +900,8 @@ extern "C" int celg_solve_host(celg_handle* h, celg_mat* m, int solver, const do
     h->sb = h->sx = nullptr;
     h->scap = 0;  // a failed allocation below leaves no stale capacity behind
     const size_t cap = std::max<size_t>(n, 1024);
-    CELG_CUDA(cudaMalloc(&h->sb, sizeof(double) * cap));
-    CELG_CUDA(cudaMalloc(&h->sx, sizeof(double) * cap));
+    CELG_CUDA(raw_alloc(h, &h->sb, sizeof(double) * cap));
+    CELG_CUDA(raw_alloc(h, &h->sx, sizeof(double) * cap));
     h->scap = cap;
   }
   // host -> device copies of this solve's inputs, on the handle's stream

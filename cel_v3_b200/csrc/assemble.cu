@@ -80,9 +80,9 @@ int coo_to_mat_device(celg_handle* h, int n, int ncols, int nnz, const int* rows
   const int grid = (int)std::max(1L, std::min(((long)nnz + 255) / 256, (long)h->sms * 16));
   int* bad = h->err_d + 2;
   if (!st) {
-    chk(cudaMalloc(&key, sizeof(*key) * nz)) && chk(cudaMalloc(&key2, sizeof(*key2) * nz)) &&
-        chk(cudaMalloc(&idx, sizeof(int) * nz)) && chk(cudaMalloc(&perm, sizeof(int) * nz)) &&
-        chk(cudaMalloc(&counts, sizeof(int) * ((size_t)n + 1)));
+    chk(raw_alloc(h, &key, sizeof(*key) * nz)) && chk(raw_alloc(h, &key2, sizeof(*key2) * nz)) &&
+        chk(raw_alloc(h, &idx, sizeof(int) * nz)) && chk(raw_alloc(h, &perm, sizeof(int) * nz)) &&
+        chk(raw_alloc(h, &counts, sizeof(int) * ((size_t)n + 1)));
     chk(cudaMemsetAsync(counts, 0, sizeof(int) * ((size_t)n + 1), h->stream));
     chk(cudaMemsetAsync(bad, 0, sizeof(int), h->stream));
     if (e == cudaSuccess && nnz > 0) {
@@ -99,7 +99,7 @@ int coo_to_mat_device(celg_handle* h, int n, int ncols, int nnz, const int* rows
     size_t sb = 0;
     if (e == cudaSuccess)
       chk(cub::DeviceScan::ExclusiveSum(nullptr, sb, counts, m->csr.rp, n + 1, h->stream));
-    if (e == cudaSuccess) chk(cudaMalloc(&tmp, std::max<size_t>(std::max(tb, sb), 16)));
+    if (e == cudaSuccess) chk(raw_alloc(h, &tmp, std::max<size_t>(std::max(tb, sb), 16)));
     if (e == cudaSuccess && nnz > 0)
       chk(cub::DeviceRadixSort::SortPairs(tmp, tb, key, key2, idx, perm, nnz, 0, end_bit, h->stream));
     // row pointer: exclusive scan of the counts over n+1 entries (the last
@@ -232,9 +232,9 @@ extern "C" int celg_mat_from_coo(celg_handle* h, int n, int ncols, int nnz, cons
   const size_t nz = (size_t)std::max(1, nnz);
   int *r_d = nullptr, *c_d = nullptr;
   double* v_d = nullptr;
-  cudaError_t e = cudaMalloc(&r_d, sizeof(int) * nz);
-  if (e == cudaSuccess) e = cudaMalloc(&c_d, sizeof(int) * nz);
-  if (e == cudaSuccess) e = cudaMalloc(&v_d, sizeof(double) * nz);
+  cudaError_t e = raw_alloc(h, &r_d, sizeof(int) * nz);
+  if (e == cudaSuccess) e = raw_alloc(h, &c_d, sizeof(int) * nz);
+  if (e == cudaSuccess) e = raw_alloc(h, &v_d, sizeof(double) * nz);
   if (e == cudaSuccess && nnz > 0) e = cudaMemcpyAsync(r_d, rows, sizeof(int) * nnz, cudaMemcpyHostToDevice, h->stream);
   if (e == cudaSuccess && nnz > 0) e = cudaMemcpyAsync(c_d, cols, sizeof(int) * nnz, cudaMemcpyHostToDevice, h->stream);
   if (e == cudaSuccess && nnz > 0)

@@ -866,15 +866,15 @@ static int batch_build(celg_handle* h, int count, celg_mat* const* mats, const s
   A.nnz = (int)NNZ;
   cudaError_t e = cudaSuccess;
   auto ok = [&](cudaError_t x) { if (e == cudaSuccess) e = x; return e == cudaSuccess; };
-  ok(cudaMalloc(&A.rp, sizeof(int) * ((size_t)N + 1 + 8)));
-  ok(cudaMalloc(&A.ci, sizeof(int) * ((size_t)NNZ + 8)));
-  ok(cudaMalloc(&A.v, sizeof(double) * ((size_t)NNZ + 8)));
-  ok(cudaMalloc(&bt->J, sizeof(double) * std::max<size_t>(N, 1)));
-  ok(cudaMalloc(&bt->B, sizeof(double) * std::max<size_t>(N, 1) * 6));
-  ok(cudaMalloc(&bt->tile_arrays, sizeof(int) * ((size_t)bt->NT + 2 * (size_t)count + 1)));
-  ok(cudaMalloc(&bt->sys_ticket, sizeof(unsigned) * (size_t)count));
-  ok(cudaMalloc(&bt->dstate, sizeof(double) * 8 * (size_t)count));
-  ok(cudaMalloc(&bt->istate, sizeof(int) * (5 * (size_t)count + 1)));
+  ok(raw_alloc(h, &A.rp, sizeof(int) * ((size_t)N + 1 + 8)));
+  ok(raw_alloc(h, &A.ci, sizeof(int) * ((size_t)NNZ + 8)));
+  ok(raw_alloc(h, &A.v, sizeof(double) * ((size_t)NNZ + 8)));
+  ok(raw_alloc(h, &bt->J, sizeof(double) * std::max<size_t>(N, 1)));
+  ok(raw_alloc(h, &bt->B, sizeof(double) * std::max<size_t>(N, 1) * 6));
+  ok(raw_alloc(h, &bt->tile_arrays, sizeof(int) * ((size_t)bt->NT + 2 * (size_t)count + 1)));
+  ok(raw_alloc(h, &bt->sys_ticket, sizeof(unsigned) * (size_t)count));
+  ok(raw_alloc(h, &bt->dstate, sizeof(double) * 8 * (size_t)count));
+  ok(raw_alloc(h, &bt->istate, sizeof(int) * (5 * (size_t)count + 1)));
   if (e != cudaSuccess) {
     batch_free(bt);
     return cuda_status(e, "batch allocation");
@@ -1312,13 +1312,13 @@ static int batch_ensure_f32(celg_handle* h, Batch* bt) {
   const size_t N = (size_t)std::max(1L, bt->N), NNZ = (size_t)bt->A.nnz, c = (size_t)bt->nsys;
   cudaError_t e = cudaSuccess;
   auto ok = [&](cudaError_t x) { if (e == cudaSuccess) e = x; return e == cudaSuccess; };
-  ok(cudaMalloc(&bt->A.v32, sizeof(float) * (NNZ + 32)));
-  ok(cudaMalloc(&bt->J32, sizeof(float) * N));
-  ok(cudaMalloc(&bt->F, sizeof(float) * N * 6));
-  ok(cudaMalloc(&bt->irs, sizeof(int) * (5 * c + 1)));
-  ok(cudaMalloc(&bt->irtau, sizeof(double) * c));
-  ok(cudaMalloc(&bt->dstate2, sizeof(double) * 8 * c));
-  ok(cudaMalloc(&bt->istate2, sizeof(int) * (5 * c + 1)));
+  ok(raw_alloc(h, &bt->A.v32, sizeof(float) * (NNZ + 32)));
+  ok(raw_alloc(h, &bt->J32, sizeof(float) * N));
+  ok(raw_alloc(h, &bt->F, sizeof(float) * N * 6));
+  ok(raw_alloc(h, &bt->irs, sizeof(int) * (5 * c + 1)));
+  ok(raw_alloc(h, &bt->irtau, sizeof(double) * c));
+  ok(raw_alloc(h, &bt->dstate2, sizeof(double) * 8 * c));
+  ok(raw_alloc(h, &bt->istate2, sizeof(int) * (5 * c + 1)));
   ok(cudaMemsetAsync(bt->F, 0, sizeof(float) * N * 6, h->stream));
   ok(cudaMemsetAsync(bt->A.v32 + NNZ, 0, sizeof(float) * 32, h->stream));
   if (e != cudaSuccess) return cuda_status(e, "batch FP32 allocation");
@@ -1589,8 +1589,8 @@ static int pcg_batched_ru(celg_handle* h, int count, celg_mat* const* mats, cons
   if (!st) st = batch_ensure_f32(h, bt);
   if (st) return st;
   const int c = bt->nsys;
-  if (!bt->rud) CELG_CUDA(cudaMalloc(&bt->rud, sizeof(double) * 3 * (size_t)c));
-  if (!bt->rui) CELG_CUDA(cudaMalloc(&bt->rui, sizeof(int) * (2 * (size_t)c + 1)));
+  if (!bt->rud) CELG_CUDA(raw_alloc(h, &bt->rud, sizeof(double) * 3 * (size_t)c));
+  if (!bt->rui) CELG_CUDA(raw_alloc(h, &bt->rui, sizeof(int) * (2 * (size_t)c + 1)));
   BatchRu u;
   u.maxr = bt->rud;
   u.rz_prev = u.maxr + c;

@@ -24,7 +24,7 @@ int ensure_partials(celg_handle* h, long ntiles, int nred) {
     h->partials = nullptr;
   }
   const size_t cap = std::max(need, (size_t)4096);
-  CELG_CUDA(cudaMalloc(&h->partials, cap * sizeof(double)));
+  CELG_CUDA(raw_alloc(h, &h->partials, cap * sizeof(double)));
   h->partials_cap = cap;
   return CELG_OK;
 }

@@ -266,7 +266,7 @@ extern "C" int celg_mat_block_jacobi(celg_mat* m, int block_size) {
   cudaFree(m->bjinv);
   m->bjinv = nullptr;
   m->bj_bs = 0;
-  CELG_CUDA(cudaMalloc(&m->bjinv, sizeof(double) * (size_t)std::max(1, n) * block_size));
+  CELG_CUDA(raw_alloc(m->h, &m->bjinv, sizeof(double) * (size_t)std::max(1, n) * block_size));
   int* bad = h->err_d + 2;
   CELG_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), h->stream));
   const long nblk = ((long)n + block_size - 1) / block_size;

@@ -203,7 +203,8 @@ bool out_of_memory(cudaError_t e);
 // Device memory of the handle's matrices.  Blocks given back are kept for
 // later requests on the handle, in the order of its stream, up to
 // kSpareBytes in all (getting and returning a block costs 0.1-0.2 ms each,
-// at times milliseconds); celg_destroy frees them.  keep = false: the block
+// at times milliseconds); celg_destroy frees them, and so does any allocation
+// of the handle that finds no other memory.  keep = false: the block
 // goes back to the device, which waits for all work on it, on every stream.
 constexpr size_t kSpareBlock = (size_t)32 << 20, kSpareBytes = (size_t)96 << 20;
 cudaError_t dev_alloc_bytes(celg_handle* h, void** p, size_t bytes);
@@ -213,6 +214,16 @@ template <typename T>
 cudaError_t dev_alloc(celg_handle* h, T** p, size_t bytes) {
   void* q = nullptr;
   const cudaError_t e = dev_alloc_bytes(h, &q, bytes);
+  *p = static_cast<T*>(q);
+  return e;
+}
+// cudaMalloc for everything else of a handle (given back with cudaFree): the
+// spare blocks make room when there is none left.
+cudaError_t raw_alloc_bytes(celg_handle* h, void** p, size_t bytes);
+template <typename T>
+cudaError_t raw_alloc(celg_handle* h, T** p, size_t bytes) {
+  void* q = nullptr;
+  const cudaError_t e = raw_alloc_bytes(h, &q, bytes);
   *p = static_cast<T*>(q);
   return e;
 }

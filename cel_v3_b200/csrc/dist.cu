@@ -319,9 +319,9 @@ static int dist_find_interior(celg_dist* d) {
   const CsrDev& A = d->m->csr;
   const long nt = ntiles_of(A.n);
   if (nt == 0) return CELG_OK;
-  CELG_CUDA(cudaMalloc(&d->part, sizeof(double) * (size_t)nt));
+  CELG_CUDA(raw_alloc(d->h, &d->part, sizeof(double) * (size_t)nt));
   int* flags = nullptr;
-  CELG_CUDA(cudaMalloc(&flags, sizeof(int) * (size_t)nt));
+  CELG_CUDA(raw_alloc(d->h, &flags, sizeof(int) * (size_t)nt));
   std::vector<int> f((size_t)nt);
   cudaError_t e = cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)nt, h->stream);
   if (e == cudaSuccess) {
@@ -374,7 +374,7 @@ extern "C" int celg_dist_create(celg_handle* h, celg_mat* m, const celg_params* 
   if (state_d) {
     d->st = static_cast<DistState*>(state_d);
   } else {
-    e = cudaMalloc(&d->st, CELG_DIST_STATE_BYTES);
+    e = raw_alloc(d->h, &d->st, CELG_DIST_STATE_BYTES);
     d->own_state = e == cudaSuccess;
   }
   if (e == cudaSuccess) e = cudaMallocHost(&d->host, sizeof(DistState));

@@ -131,9 +131,9 @@ static int solve_data(celg_dist* d, DistSolveData** out) {
     s->n = n;
     s->ncols = ncols;
     *slot = s;
-    CELG_CUDA(cudaMalloc(&s->r, sizeof(double) * (size_t)n));
-    CELG_CUDA(cudaMalloc(&s->v, sizeof(double) * (size_t)n));
-    CELG_CUDA(cudaMalloc(&s->p, sizeof(double) * (size_t)ncols));
+    CELG_CUDA(raw_alloc(h, &s->r, sizeof(double) * (size_t)n));
+    CELG_CUDA(raw_alloc(h, &s->v, sizeof(double) * (size_t)n));
+    CELG_CUDA(raw_alloc(h, &s->p, sizeof(double) * (size_t)ncols));
     CELG_CUDA(cudaMemsetAsync(s->p, 0, sizeof(double) * (size_t)ncols, h->stream));
   }
   *out = s;
@@ -178,8 +178,8 @@ extern "C" int celg_dist_set_exchange(celg_dist* d, int nneigh, const int* peers
   for (int q = 1; q < nneigh; ++q) s->send_off[q] = s->send_off[q - 1] + send_counts[q - 1];
   s->nsend = (int)nsend;
   if (nsend > 0) {
-    CELG_CUDA(cudaMalloc(&s->send_rows_d, sizeof(int) * (size_t)nsend));
-    CELG_CUDA(cudaMalloc(&s->send_buf_d, sizeof(double) * (size_t)nsend));
+    CELG_CUDA(raw_alloc(h, &s->send_rows_d, sizeof(int) * (size_t)nsend));
+    CELG_CUDA(raw_alloc(h, &s->send_buf_d, sizeof(double) * (size_t)nsend));
     CELG_CUDA(cudaMemcpy(s->send_rows_d, send_rows, sizeof(int) * (size_t)nsend,
                          cudaMemcpyHostToDevice));
   }

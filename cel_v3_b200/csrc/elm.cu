@@ -327,9 +327,9 @@ static int elm_complete_triplets(celg_handle* h, Elm* e, celg_mat** m) {
   const size_t nz = std::max<size_t>(nnz, 1);
   int *r_d = nullptr, *c_d = nullptr;
   double* v_d = nullptr;
-  cudaError_t ce = cudaMalloc(&r_d, sizeof(int) * nz);
-  if (ce == cudaSuccess) ce = cudaMalloc(&c_d, sizeof(int) * nz);
-  if (ce == cudaSuccess) ce = cudaMalloc(&v_d, sizeof(double) * nz);
+  cudaError_t ce = raw_alloc(h, &r_d, sizeof(int) * nz);
+  if (ce == cudaSuccess) ce = raw_alloc(h, &c_d, sizeof(int) * nz);
+  if (ce == cudaSuccess) ce = raw_alloc(h, &v_d, sizeof(double) * nz);
   if (ce == cudaSuccess && nnz)
     ce = cudaMemcpyAsync(r_d, e->rows.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice, h->stream);
   if (ce == cudaSuccess && nnz)

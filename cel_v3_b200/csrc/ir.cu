@@ -71,8 +71,8 @@ int ensure_f32(celg_handle* h, size_t n) {
   h->f32 = nullptr;
   h->ir_d = nullptr;
   const size_t cap = std::max<size_t>(n, 1024);
-  CELG_CUDA(cudaMalloc(&h->f32, sizeof(float) * cap * 6));  // 6 float vectors
-  CELG_CUDA(cudaMalloc(&h->ir_d, sizeof(double) * cap));
+  CELG_CUDA(raw_alloc(h, &h->f32, sizeof(float) * cap * 6));  // 6 float vectors
+  CELG_CUDA(raw_alloc(h, &h->ir_d, sizeof(double) * cap));
   h->f32cap = cap;
   h->ircap = cap;
   return CELG_OK;

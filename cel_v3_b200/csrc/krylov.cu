@@ -702,7 +702,7 @@ int cg_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const celg
 // V[0..M], Z[0..M-1] and H ((M+1) x M), plus the device state.
 static int ensure_gmres_work(celg_handle* h, size_t nn, int M) {
   const size_t need = nn * (size_t)(2 * M + 1) + (size_t)(M + 1) * M + 8;
-  if (!h->gm_state_d) CELG_CUDA(cudaMalloc(&h->gm_state_d, sizeof(GmState)));
+  if (!h->gm_state_d) CELG_CUDA(raw_alloc(h, &h->gm_state_d, sizeof(GmState)));
   if (!h->gm_state_h) CELG_CUDA(cudaMallocHost(&h->gm_state_h, sizeof(GmState)));
   if (need <= h->gm_cap && h->gm_work) return CELG_OK;
   CELG_CUDA(cudaStreamSynchronize(h->stream));
@@ -710,7 +710,7 @@ static int ensure_gmres_work(celg_handle* h, size_t nn, int M) {
   cudaFree(h->gm_work);
   h->gm_work = nullptr;
   h->gm_cap = 0;
-  CELG_CUDA(cudaMalloc(&h->gm_work, sizeof(double) * need));
+  CELG_CUDA(raw_alloc(h, &h->gm_work, sizeof(double) * need));
   h->gm_cap = need;
   return CELG_OK;
 }
@@ -790,7 +790,7 @@ static int gm_plan_orth(celg_handle* h, GmPlan* g) {
   if (per_sm < 1) return CELG_OK;
   const size_t bytes = 256 + sizeof(ulonglong2) * (size_t)(kGmMaxTiles + 1);
   if (!h->gm_exch) {
-    const cudaError_t em = cudaMalloc(&h->gm_exch, bytes);
+    const cudaError_t em = raw_alloc(h, &h->gm_exch, bytes);
     if (out_of_memory(em)) return CELG_OK;
     CELG_CUDA(em);
   }

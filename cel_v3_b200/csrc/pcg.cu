@@ -49,16 +49,16 @@ int ensure_work(celg_handle* h, size_t n) {
   h->wr = h->wp = h->wv = h->wq = nullptr;
   h->wcap = 0;  // a failed allocation below leaves no stale capacity behind
   const size_t cap = std::max<size_t>(n, 1024);
-  CELG_CUDA(cudaMalloc(&h->wr, cap * sizeof(double)));
-  CELG_CUDA(cudaMalloc(&h->wp, cap * sizeof(double)));
-  CELG_CUDA(cudaMalloc(&h->wv, cap * sizeof(double)));
-  CELG_CUDA(cudaMalloc(&h->wq, cap * sizeof(double)));
+  CELG_CUDA(raw_alloc(h, &h->wr, cap * sizeof(double)));
+  CELG_CUDA(raw_alloc(h, &h->wp, cap * sizeof(double)));
+  CELG_CUDA(raw_alloc(h, &h->wv, cap * sizeof(double)));
+  CELG_CUDA(raw_alloc(h, &h->wq, cap * sizeof(double)));
   h->wcap = cap;
   return CELG_OK;
 }
 
 int ensure_state(celg_handle* h, int hist_cap) {
-  if (!h->state_d) CELG_CUDA(cudaMalloc(&h->state_d, sizeof(PcgState)));
+  if (!h->state_d) CELG_CUDA(raw_alloc(h, &h->state_d, sizeof(PcgState)));
   if (!h->state_h) CELG_CUDA(cudaMallocHost(&h->state_h, sizeof(PcgState)));
   if (hist_cap > h->hist_cap) {
     CELG_CUDA(cudaStreamSynchronize(h->stream));
@@ -66,7 +66,7 @@ int ensure_state(celg_handle* h, int hist_cap) {
     cudaFree(h->hist_d);
     h->hist_d = nullptr;
     h->hist_cap = 0;
-    CELG_CUDA(cudaMalloc(&h->hist_d, sizeof(double) * (size_t)hist_cap));
+    CELG_CUDA(raw_alloc(h, &h->hist_d, sizeof(double) * (size_t)hist_cap));
     h->hist_cap = hist_cap;
   }
   return CELG_OK;
@@ -325,7 +325,7 @@ int pcg_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const cel
       cudaFree(h->wz);
       h->wz = nullptr;
       h->wzcap = std::max<size_t>((size_t)n, 1024);
-      CELG_CUDA(cudaMalloc(&h->wz, h->wzcap * sizeof(double)));
+      CELG_CUDA(raw_alloc(h, &h->wz, h->wzcap * sizeof(double)));
     }
     B.bj = m->bjinv;
     B.bs = m->bj_bs;

@@ -1198,7 +1198,7 @@ static int onchip_grow(celg_handle* h, double** buf, size_t* cap, size_t need, b
   cudaFree(*buf);
   *buf = nullptr;
   *cap = 0;
-  const cudaError_t e = cudaMalloc(buf, sizeof(double) * need);
+  const cudaError_t e = raw_alloc(h, buf, sizeof(double) * need);
   *ok = !out_of_memory(e);
   if (!*ok) return CELG_OK;
   CELG_CUDA(e);

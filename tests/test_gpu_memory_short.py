@@ -118,6 +118,27 @@ def test_matrix_without_room_for_its_row_forms(gpu):
     h.close()
 
 
+def test_spare_blocks_give_way(gpu, monkeypatch):
+    """Work vectors of a solve when what is left is held as spare blocks."""
+    celgpu, _, torch = gpu
+    h = handle(celgpu, torch)
+    monkeypatch.setenv("CELG_ONCHIP_ROWS", "0")
+    big = h.matrix_from_csr(*synth.poisson7(128)).jacobi()
+    b = torch.ones(big.n, dtype=torch.float64, device="cuda")
+    x = torch.zeros_like(b)
+    spare = [h.matrix_from_csr(*synth.poisson7(68)) for _ in range(3)]
+    for m in spare:
+        m.destroy()  # about 28 MB each
+    f = Filled(torch, 32 * MB)
+    try:
+        i = h.pcg_jacobi(big, b.data_ptr(), x.data_ptr(), eps_rel=1e-3, iter_max=100, x0_mode=celgpu.X0_ZERO)
+    finally:
+        f.release()
+    assert i.status == celgpu.ERR_NOCONV and i.iter_done == 100  # the cap, not an allocation
+    big.destroy()
+    h.close()
+
+
 def elm_system():
     _, k = synth.lognormal_faces(np.random.default_rng(1), 90, 88, 86, 0.5)
     rp, ci, v = synth.diffusion7(90, 88, 86, *k)

@@ -564,6 +564,7 @@ extern "C" int celg_set_stream(celg_handle* h, void* stream) {
   CELG_CUDA(cudaStreamSynchronize(h->stream));
   if (h->own_stream) cudaStreamDestroy(h->stream);
   h->own_stream = false;
+  h->coop_ok = h->coop_no = 0;  // a stream can have fewer SMs than another
   h->stream = (cudaStream_t)stream;
   if (!stream) {
     CELG_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));

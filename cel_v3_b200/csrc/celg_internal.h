@@ -120,6 +120,9 @@ struct celg_handle {
   std::vector<celg::GraphEntry> graphs;
   double* hist_d = nullptr;
   int hist_cap = 0;
+  // largest cooperative grid known to be accepted, smallest known to be
+  // refused (coop_fits; 0: none yet)
+  int coop_ok = 0, coop_no = 0;
   // exchange slots of the one-kernel solve (oc_cap doubles)
   double* oc_slots = nullptr;
   size_t oc_cap = 0;
@@ -273,6 +276,9 @@ int ensure_f32(celg_handle* h, size_t n);
 int ensure_offset_dict(celg_handle* h, celg_mat* m);
 // the same for any CSR array set (left unset beyond 256 distinct offsets)
 int build_offset_dict_csr(celg_handle* h, CsrDev& A);
+// pcg_onchip.cu: whether the driver accepts a cooperative grid of that many
+// CTAs, one per SM, on the handle's stream.
+int coop_fits(celg_handle* h, int grid, bool* fits);
 // pcg_onchip.cu: drop the sliced copy (the values changed, or the matrix goes)
 void sell_free(celg_handle* h, CsrDev& A);
 // row_forms.cu

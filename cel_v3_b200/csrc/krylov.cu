@@ -778,16 +778,18 @@ static int gm_orth(celg_handle* h, const GmPlan& g, int j) {
 }
 
 // Tiles per CTA of gm_orth_kernel, 0 when w does not fit the registers of the
-// resident CTAs (then the graph of sweeps runs; CELG_ONCHIP_ROWS as for PCG).
+// resident CTAs, the driver refuses the grid or there is no memory for its
+// words (then the graph of sweeps runs; CELG_ONCHIP_ROWS as for PCG).
 static int gm_plan_orth(celg_handle* h, GmPlan* g) {
   g->per_cta = 0;
   const long nt = ntiles_of(g->n);
   const char* e = std::getenv("CELG_ONCHIP_ROWS");
   if (g->n < 1 || nt > std::min((long)kGmTiles * h->sms, (long)kGmMaxTiles) || (e && g->n > std::atol(e))) return CELG_OK;
+  const int per = (int)((nt + h->sms - 1) / h->sms);
+  bool fits = false;
+  if (const int st = coop_fits(h, (int)((nt + per - 1) / per), &fits)) return st;
+  if (!fits) return CELG_OK;
   if (const int st = allow_dynamic_smem<gm_orth_kernel>(kGmSmem)) return st;
-  int per_sm = 0;
-  CELG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gm_orth_kernel, kGmThreads, kGmSmem));
-  if (per_sm < 1) return CELG_OK;
   const size_t bytes = 256 + sizeof(ulonglong2) * (size_t)(kGmMaxTiles + 1);
   if (!h->gm_exch) {
     const cudaError_t em = raw_alloc(h, &h->gm_exch, bytes);
@@ -797,7 +799,7 @@ static int gm_plan_orth(celg_handle* h, GmPlan* g) {
   CELG_CUDA(cudaMemsetAsync(h->gm_exch, 0, bytes, h->stream));
   g->ex.count = static_cast<unsigned long long*>(h->gm_exch);
   g->ex.word = static_cast<ulonglong2*>(h->gm_exch) + 15;
-  g->per_cta = (int)((nt + h->sms - 1) / h->sms);
+  g->per_cta = per;
   return CELG_OK;
 }
 

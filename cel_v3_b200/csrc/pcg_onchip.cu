@@ -1057,38 +1057,50 @@ static long onchip_max_rows() {
   return e ? std::atol(e) : 1L << 30;
 }
 
-// *done stays false when the device cannot hold the grid at once (fewer SMs
-// at this process's disposal than the device has).
+// A process or a stream can have fewer SMs at its disposal than the device
+// reports.  The driver then refuses cooperative grids that cannot all be
+// resident, but says so only at a launch (for a captured one, at the graph's),
+// and a batch must not be refused half way.  So an empty kernel that fills an
+// SM per CTA, as those that matter do, is launched for every new largest grid.
+__global__ void __launch_bounds__(kOcThreads, 1) coop_probe_kernel() {}
+
+int coop_fits(celg_handle* h, int grid, bool* fits) {
+  *fits = grid <= h->coop_ok;
+  if (*fits || (h->coop_no && grid >= h->coop_no)) return CELG_OK;
+  const int smem = kOcMaxSmem - 1024;
+  if (const int st = allow_dynamic_smem<coop_probe_kernel>(smem)) return st;
+  const cudaError_t e =
+      cudaLaunchCooperativeKernel((const void*)coop_probe_kernel, dim3(grid), dim3(kOcThreads), nullptr, smem, h->stream);
+  *fits = e == cudaSuccess;
+  if (*fits) {
+    h->coop_ok = grid;
+  } else if (e == cudaErrorCooperativeLaunchTooLarge) {
+    (void)cudaGetLastError();
+    h->coop_no = grid;
+  } else {
+    CELG_CUDA(e);
+  }
+  return CELG_OK;
+}
+
 template <typename VT, bool PAT>
-static int launch_onchip(cudaStream_t stream, const OcArgs<VT>& a, int grid, size_t smem, bool* done) {
+static int launch_onchip(cudaStream_t stream, const OcArgs<VT>& a, int grid, size_t smem) {
   if (const int st = allow_dynamic_smem<pcg_onchip_kernel<VT, PAT>>((int)smem)) return st;
   OcArgs<VT> arg = a;
   void* params[] = {&arg};
-  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)pcg_onchip_kernel<VT, PAT>, dim3(grid),
-                                                    dim3(kOcThreads), params, smem, stream);
-  if (e == cudaErrorCooperativeLaunchTooLarge) {
-    (void)cudaGetLastError();
-    return CELG_OK;
-  }
-  CELG_CUDA(e);
-  *done = true;
+  CELG_CUDA(cudaLaunchCooperativeKernel((const void*)pcg_onchip_kernel<VT, PAT>, dim3(grid), dim3(kOcThreads), params,
+                                        smem, stream));
   return CELG_OK;
 }
 
 template <int FORM>
-static int launch_wide(cudaStream_t stream, const OcArgs<double>& o, double* v, int per, int less, int grid, size_t smem,
-                       bool* done) {
+static int launch_wide(cudaStream_t stream, const OcArgs<double>& o, double* v, int per, int less, int grid,
+                       size_t smem) {
   if (const int st = allow_dynamic_smem<pcg_wide_kernel<FORM>>((int)smem)) return st;
   WideArgs arg{o, v, per, less};
   void* params[] = {&arg};
-  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)pcg_wide_kernel<FORM>, dim3(grid), dim3(kOcThreads),
-                                                    params, smem, stream);
-  if (e == cudaErrorCooperativeLaunchTooLarge) {
-    (void)cudaGetLastError();
-    return CELG_OK;
-  }
-  CELG_CUDA(e);
-  *done = true;
+  CELG_CUDA(cudaLaunchCooperativeKernel((const void*)pcg_wide_kernel<FORM>, dim3(grid), dim3(kOcThreads), params, smem,
+                                        stream));
   return CELG_OK;
 }
 
@@ -1146,7 +1158,7 @@ static int onchip_matrix(celg_handle* h, CsrDev& A, const VT* vals, const Onchip
 // words: q.words() doubles set to 0xff
 template <typename VT>
 static int onchip_launch(cudaStream_t stream, CsrDev& A, const PcgBind<VT>& B, const celg_params* p, const OnchipPlan& q,
-                         double* words, PcgState* out, double* hist, int hist_cap, bool* done) {
+                         double* words, PcgState* out, double* hist, int hist_cap) {
   OcArgs<VT> a;
   a.n = A.n;
   a.ntiles = (int)ntiles_of(A.n);
@@ -1180,13 +1192,12 @@ static int onchip_launch(cudaStream_t stream, CsrDev& A, const PcgBind<VT>& B, c
   a.eps_rel = p->eps_rel;
   if constexpr (sizeof(VT) == 8) {
     if (q.wide) {
-      if (a.rowv) return launch_wide<kFormTable>(stream, a, B.v, q.per, q.less, q.grid, q.smem, done);
-      return A.pid ? launch_wide<kFormPat>(stream, a, B.v, q.per, q.less, q.grid, q.smem, done)
-                   : launch_wide<kFormCols>(stream, a, B.v, q.per, q.less, q.grid, q.smem, done);
+      if (a.rowv) return launch_wide<kFormTable>(stream, a, B.v, q.per, q.less, q.grid, q.smem);
+      return A.pid ? launch_wide<kFormPat>(stream, a, B.v, q.per, q.less, q.grid, q.smem)
+                   : launch_wide<kFormCols>(stream, a, B.v, q.per, q.less, q.grid, q.smem);
     }
   }
-  return A.pid ? launch_onchip<VT, true>(stream, a, q.grid, q.smem, done)
-               : launch_onchip<VT, false>(stream, a, q.grid, q.smem, done);
+  return A.pid ? launch_onchip<VT, true>(stream, a, q.grid, q.smem) : launch_onchip<VT, false>(stream, a, q.grid, q.smem);
 }
 
 // *ok = false: no memory for a buffer of the handle's that has to grow to
@@ -1219,11 +1230,15 @@ int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_param
   OnchipPlan q;
   if (!onchip_plan<VT>(A, h->sms, &q)) return CELG_OK;
   bool ok = false;
-  int st = onchip_matrix<VT>(h, A, B.vals, q, &ok);
+  int st = coop_fits(h, q.grid, &ok);
+  if (st || !ok) return st;
+  st = onchip_matrix<VT>(h, A, B.vals, q, &ok);
   if (st || !ok) return st;
   st = onchip_words(h, q.words(), &ok);
   if (st || !ok) return st;
-  return onchip_launch<VT>(h->stream, A, B, p, q, h->oc_slots, h->state_h, h->hist_d, hist_cap, done);
+  st = onchip_launch<VT>(h->stream, A, B, p, q, h->oc_slots, h->state_h, h->hist_d, hist_cap);
+  *done = !st;
+  return st;
 }
 
 // ---- many systems ------------------------------------------------------------------
@@ -1277,11 +1292,15 @@ int pcg_onchip_many(celg_handle* h, int count, celg_mat* const* mats, const doub
   }
   if (std::max(kernels, longest) >= sweeps + 24.0 * slowest) return CELG_OK;
   bool ok = true;
+  int largest = 0;
+  for (const Job& j : jobs) largest = std::max(largest, j.q.grid);
+  int st = largest ? coop_fits(h, largest, &ok) : CELG_OK;
+  if (st || !ok) return st;
   std::vector<CsrDev*> built;
   for (const Job& j : jobs) {
     CsrDev& A = mats[j.sys]->csr;
     const bool had = A.sell_v != nullptr;
-    const int st = onchip_matrix<double>(h, A, A.v, j.q, &ok);
+    st = onchip_matrix<double>(h, A, A.v, j.q, &ok);
     if (!had && A.sell_v) built.push_back(&A);
     if (!st && ok) continue;
     // one has none: the sweeps need no copy of the others
@@ -1293,7 +1312,7 @@ int pcg_onchip_many(celg_handle* h, int count, celg_mat* const* mats, const doub
   size_t room = 32;
   for (const Job& j : jobs) room = std::max(room, ((size_t)mats[j.sys]->csr.n + 31) & ~(size_t)31);
   const size_t work = 2 * kOcLanes * room;
-  int st = onchip_grow(h, &h->oc_work, &h->oc_work_cap, work, &ok);
+  st = onchip_grow(h, &h->oc_work, &h->oc_work_cap, work, &ok);
   if (st || !ok) return st;
   if (count > h->oc_states_cap) {
     cudaFreeHost(h->oc_states);
@@ -1312,9 +1331,6 @@ int pcg_onchip_many(celg_handle* h, int count, celg_mat* const* mats, const doub
   if (st || !ok) return st;
   std::stable_sort(jobs.begin(), jobs.end(),
                    [&](const Job& a, const Job& c) { return mats[a.sys]->csr.n > mats[c.sys]->csr.n; });
-  const Job* first = nullptr;
-  for (const Job& j : jobs)
-    if (!first || j.lanes < first->lanes) first = &j;
   double load[kOcLanes] = {};
   auto stream_of = [&](int l) { return l ? h->oc_lane[l] : h->stream; };
   for (int lanes = 1; lanes <= kOcLanes && !st; lanes *= 2) {
@@ -1344,12 +1360,7 @@ int pcg_onchip_many(celg_handle* h, int count, celg_mat* const* mats, const doub
       B.J = m->jacobi;
       B.juni = m->csr.juni;
       B.jval = m->csr.jval;
-      bool launched = false;
-      st = onchip_launch<double>(stream_of(l), m->csr, B, p, j.q, h->oc_slots + j.words, h->oc_states + j.sys, nullptr,
-                                 0, &launched);
-      // (the largest shares come first: if the first is refused, nothing has run)
-      if (!st && !launched && &j == first) return CELG_OK;
-      if (!st && !launched) st = CELG_ERR_CUDA;
+      st = onchip_launch<double>(stream_of(l), m->csr, B, p, j.q, h->oc_slots + j.words, h->oc_states + j.sys, nullptr, 0);
     }
   }
   for (int l = 1; l < kOcLanes; ++l) {

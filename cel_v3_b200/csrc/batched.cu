@@ -1193,8 +1193,9 @@ static int pcg_batched_onchip(celg_handle* h, int count, celg_mat* const* mats, 
   CELG_CUDA(cudaEventRecord(h->ev0, h->stream));
   const int st = pcg_onchip_many(h, count, mats, b_d, x_d, p, &states, done);
   if (st || !*done) return st;
-  CELG_CUDA(cudaEventRecord(h->ev1, h->stream));
+  const cudaError_t er = cudaEventRecord(h->ev1, h->stream);
   CELG_CUDA(cudaStreamSynchronize(h->stream));
+  CELG_CUDA(er);
   cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1);
   int ret = CELG_OK, iters = 0;
   for (int s = 0; s < count; ++s) {

@@ -1333,12 +1333,17 @@ int pcg_onchip_many(celg_handle* h, int count, celg_mat* const* mats, const doub
                    [&](const Job& a, const Job& c) { return mats[a.sys]->csr.n > mats[c.sys]->csr.n; });
   double load[kOcLanes] = {};
   auto stream_of = [&](int l) { return l ? h->oc_lane[l] : h->stream; };
+  // what stream l does next comes after what stream `from` has been given
+  auto follow = [&](int l, int from, cudaEvent_t ev) {
+    cudaError_t e = cudaEventRecord(ev, stream_of(from));
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(stream_of(l), ev, 0);
+    if (e != cudaSuccess && !st) st = cuda_status(e, "batch lanes");
+  };
   for (int lanes = 1; lanes <= kOcLanes && !st; lanes *= 2) {
     // lane l of the upper half starts where lane l - lanes / 2 is now
     for (int l = lanes / 2; l < lanes && lanes > 1; ++l) {
       const int from = l - lanes / 2;
-      CELG_CUDA(cudaEventRecord(h->oc_event[l], stream_of(from)));
-      CELG_CUDA(cudaStreamWaitEvent(stream_of(l), h->oc_event[l], 0));
+      if (!st) follow(l, from, h->oc_event[l]);
       load[l] = load[from];
     }
     for (const Job& j : jobs) {
@@ -1363,9 +1368,12 @@ int pcg_onchip_many(celg_handle* h, int count, celg_mat* const* mats, const doub
       st = onchip_launch<double>(stream_of(l), m->csr, B, p, j.q, h->oc_slots + j.words, h->oc_states + j.sys, nullptr, 0);
     }
   }
-  for (int l = 1; l < kOcLanes; ++l) {
-    CELG_CUDA(cudaEventRecord(h->oc_event[l], h->oc_lane[l]));
-    CELG_CUDA(cudaStreamWaitEvent(h->stream, h->oc_event[l], 0));
+  for (int l = 1; l < kOcLanes && !st; ++l) follow(0, l, h->oc_event[l]);
+  if (st) {
+    // the kernels under way use the handle's buffers and the caller's vectors:
+    // they end before the error is reported
+    for (int l = 0; l < kOcLanes; ++l) cudaStreamSynchronize(stream_of(l));
+    (void)cudaGetLastError();
   }
   *states = h->oc_states;
   *done = !st;

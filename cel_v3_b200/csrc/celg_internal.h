@@ -301,6 +301,12 @@ int coo_to_mat_device(celg_handle* h, int n, int ncols, int nnz, const int* rows
 // dist.cu / dist_solve.cu: the one-call distributed solve's data on a celg_dist
 int dist_internals(celg_dist* d, celg_handle** h, int* n, int* ncols, void*** solve_slot);
 void dist_solve_free(void* solve);
+// pcg.cu: bytes of the matrix that one sweep reads, values of vt bytes: in the
+// most compact form it has, or (table = false) without the row table, or
+// (compact = false) with its int32 columns.
+double matrix_sweep_bytes(const CsrDev& A, int vt, bool compact = true, bool table = true);
+// pcg.cu: bytes of J that K2 and K3 of an iteration do not read
+double jacobi_saved_bytes(const CsrDev& A, int vt);
 void batch_free(::Batch* b);
 void multi_free(::Multi* m);
 void multi_forget_matrix(::Multi* m, const void* mat);

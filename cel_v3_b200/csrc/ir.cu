@@ -178,7 +178,7 @@ int ir_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const celg
   cudaEventDestroy(e1);
   if (st) return st;
   h->last_iters = inner_total;
-  h->last_bytes_per_iter = 8.0 * m->csr.nnz + 4.0 * (n + 1) + 50.0 * n;
+  // (last_bytes_per_iter: the inner solves', set by pcg_run)
   if (res) {
     res->iter_done = outer;
     res->final_norm2 = rn;

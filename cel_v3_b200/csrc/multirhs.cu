@@ -1857,6 +1857,19 @@ static int launch_mtile(celg_handle* h, long n, int k, const Op& op, bool vec4 =
   return CELG_OK;
 }
 
+// Bytes of the matrix that an SpMM reads: the 16-byte-gather kernel takes the
+// row table or patterns, else the columns are int32.
+static double multi_matrix_bytes(const CsrDev& A, int vt, bool vec) {
+  return matrix_sweep_bytes(A, vt, vec && A.pid);
+}
+
+// An iteration of the FP32 forms: SpMM (matrix; P gathered, V stored: 8 n k),
+// step (R, V read, R stored: 12 n k; J 4 n), direction (P, R, D read, P, D
+// stored: 20 n k; J 4 n).
+static double multi_f32_bytes(const CsrDev& A, int k) {
+  return multi_matrix_bytes(A, 4, k % 4 == 0) + 40.0 * (double)A.n * k + 8.0 * A.n;
+}
+
 }  // namespace celg
 
 struct Multi {
@@ -2183,7 +2196,8 @@ int pcg_multirhs(celg_handle* h, celg_mat* m, int k, const double* B, double* X,
     }
   }
   h->last_iters = iters;
-  h->last_bytes_per_iter = 12.0 * m->csr.nnz + 4.0 * (n + 1) + 76.0 * (double)nk + 16.0 * n;
+  // the variants from 10 on read the compact forms, the others int32 columns
+  h->last_bytes_per_iter = multi_matrix_bytes(m->csr, 8, cfg >= 10 && k % 2 == 0) + 76.0 * (double)nk + 16.0 * n;
   return ret;
 }
 
@@ -2362,6 +2376,7 @@ static int multirhs_ir(celg_handle* h, celg_mat* m, int k, const double* B, doub
     }
   }
   h->last_iters = inner_most;
+  h->last_bytes_per_iter = multi_f32_bytes(m->csr, k);
   return ret;
 }
 
@@ -2531,12 +2546,7 @@ static int multirhs_ru(celg_handle* h, celg_mat* m, int k, const double* B, doub
     }
   }
   h->last_iters = iters;
-  // FP32 SpMM (matrix; P gathered, V stored: 8 n k), step (R, V read, R
-  // stored: 12 n k; J 4 n), direction (P, R, D read, P, D stored: 20 n k;
-  // J 4 n); 4 bytes per non-zero and one per row on row patterns, else 5
-  // per non-zero with the 1-byte offsets, 8 with int32 columns
-  const double mat = m->csr.pid ? 4.0 * m->csr.nnz + n : (m->csr.ci8 ? 5.0 : 8.0) * m->csr.nnz;
-  h->last_bytes_per_iter = mat + 4.0 * (n + 1) + 40.0 * (double)nk + 8.0 * n;
+  h->last_bytes_per_iter = multi_f32_bytes(m->csr, k);
   return ret;
 }
 

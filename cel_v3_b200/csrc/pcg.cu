@@ -219,6 +219,17 @@ static std::string pcg_key(const PcgBind<VT>& B, const celg_params* p, int hist_
   return std::string(buf);
 }
 
+double matrix_sweep_bytes(const CsrDev& A, int vt, bool compact, bool table) {
+  const double n = A.n, nnz = A.nnz;
+  if (compact && table && A.rowv) return n;                   // one index byte a row
+  if (compact && A.pid) return vt * nnz + n + 4.0 * (n + 1);  // and the values
+  return (vt + (compact && A.ci8 ? 1 : 4)) * nnz + 4.0 * (n + 1);
+}
+
+double jacobi_saved_bytes(const CsrDev& A, int vt) {
+  return A.juni ? 2.0 * vt * A.n : A.jtab_ok ? 2.0 * (vt - 1) * A.n : 0.0;
+}
+
 template <typename VT>
 int pcg_run(celg_handle* h, const PcgBind<VT>& B, const celg_params* p, const void* mat,
             PcgState* out_state) {
@@ -236,6 +247,14 @@ int pcg_run(celg_handle* h, const PcgBind<VT>& B, const celg_params* p, const vo
     st = pcg_onchip<VT>(h, *B.A, B, p, hist_cap, &onchip);
     if (st) return st;
     if (onchip) CELG_CUDA(cudaEventRecord(h->ev1, h->stream));
+  }
+  if (!onchip) {
+    // K1 (matrix, p gathered, v stored), K2 (r, v, J read, r stored) and K3,
+    // paired: p, q, r, J, x read and p or q and x stored, x once per two
+    // iterations (11.5 vectors in all; unpaired 12)
+    const int vt = (int)sizeof(VT);
+    h->last_bytes_per_iter = matrix_sweep_bytes(*B.A, vt, true, !B.jad) + (B.q ? 11.5 : 12.0) * vt * (double)n -
+                             (B.jtab || B.juni ? jacobi_saved_bytes(*B.A, vt) : 0.0);
   }
   if (onchip) {
     // one kernel, which leaves its state in h->state_h
@@ -339,16 +358,6 @@ int pcg_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const cel
   std::memset(&s, 0, sizeof(s));
   const int ret = pcg_run<double>(h, B, p, m, &s);
   h->last_iters = s.iter;
-  // K1 reads one byte per row with the row table; 8 bytes per non-zero and
-  // one per row with the row patterns, 9 per non-zero with the 1-byte offsets,
-  // else 12, and the row pointer; the paired K3 reads and stores x once per
-  // two iterations (92 instead of 96 bytes per row), and with the Jacobi table
-  // K2 and K3 read a byte instead of J (14 less)
-  const double mat_bytes =
-      (jad || !m->csr.rowv ? (m->csr.pid ? 8.0 * m->csr.nnz + 1.0 * n : (B.dict ? 9.0 : 12.0) * m->csr.nnz) +
-                                 4.0 * (n + 1)
-                           : 1.0 * n);
-  h->last_bytes_per_iter = mat_bytes + ((B.q ? 92.0 : 96.0) - (B.juni ? 16.0 : B.jtab ? 14.0 : 0.0)) * n;
   if (res) {
     res->iter_done = s.iter;
     res->final_norm2 = s.norm;

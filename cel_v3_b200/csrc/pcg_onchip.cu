@@ -1148,6 +1148,17 @@ static bool onchip_plan(const CsrDev& A, int sms, OnchipPlan* out) {
   return true;
 }
 
+// What an iteration of such a kernel moves between the SMs and L2: p stored and
+// gathered, and the matrix, but for the units whose values are kept; the wide
+// form v, x and J too, and (int32 columns) two words of the row pointer.
+template <typename VT>
+static double onchip_bytes(const CsrDev& A, const OnchipPlan& q) {
+  const double vt = sizeof(VT), n = A.n, nnz = A.nnz;
+  if (!q.wide) return 2 * vt * n + (A.pid ? vt * nnz * (q.slots - q.ncache) / q.slots : (vt + 4) * nnz);
+  const double J = A.rowv && A.juni ? 0.0 : 2 * vt * n;
+  return 6 * vt * n + J + (A.rowv ? n : A.pid ? vt * nnz + n : (vt + 4) * nnz + 8 * n);
+}
+
 // the sliced values, where the kernel reads them
 template <typename VT>
 static int onchip_matrix(celg_handle* h, CsrDev& A, const VT* vals, const OnchipPlan& q, bool* ok) {
@@ -1238,6 +1249,7 @@ int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_param
   if (st || !ok) return st;
   st = onchip_launch<VT>(h->stream, A, B, p, q, h->oc_slots, h->state_h, h->hist_d, hist_cap);
   *done = !st;
+  h->last_bytes_per_iter = onchip_bytes<VT>(A, q);
   return st;
 }
 

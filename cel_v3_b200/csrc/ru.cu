@@ -404,11 +404,8 @@ int ru_solve(celg_handle* h, celg_mat* m, const double* b, double* x, const celg
   else if (s.s.err) ret = s.s.err;
   else if (!(s.norm64 <= s.s.eps)) ret = CELG_ERR_NOCONV;
   h->last_iters = s.s.iter;
-  // K1 (matrix, p gathered, v stored: 8 n), K2 (r, v, J read, r stored:
-  // 16 n), K3 (p, r, J read, p stored, d read and stored once per pair of
-  // iterations: 20 n on average); 5 bytes per non-zero with the 1-byte
-  // column offsets, else 8
-  h->last_bytes_per_iter = (m->csr.pid ? 4.0 : m->csr.ci8 ? 5.0 : 8.0) * m->csr.nnz + 4.0 * (n + 1) + 44.0 * n;
+  // as pcg_run's sweeps, the correction in place of x
+  h->last_bytes_per_iter = matrix_sweep_bytes(m->csr, 4) + 46.0 * n - jacobi_saved_bytes(m->csr, 4);
   if (res) {
     res->iter_done = s.s.iter;
     res->final_norm2 = s.norm64;

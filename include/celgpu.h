@@ -461,7 +461,12 @@ int celg_elm_doit(celg_handle* h, const double* b, int* iierr, int* niter, doubl
 int celg_elm_redoit(celg_handle* h, const double* b, int* iierr, int* niter, double* ftol);
 /* cel_elmSolverCollectSolution (:790-815): x into a caller-owned buffer of n_local */
 int celg_elm_collect_solution(celg_handle* h, double* x);
-/* cel_elmSolverPerformance (:879-900): last solve's device time and counters */
+/* cel_elmSolverPerformance (:879-900): last solve's device time and counters.
+ * bytes_per_iter, after a PCG solve (any precision; several right-hand sides:
+ * of all of them): what one iteration's sweeps read and write, the matrix and
+ * J in the form they are read in and every vector once a sweep.  A solve that
+ * ran as one kernel keeps part of that on chip: what it moves between the SMs
+ * and the memory behind them. */
 int celg_elm_performance(celg_handle* h, double* solve_ms, int* iters, double* bytes_per_iter);
 int celg_elm_destroy(celg_handle* h);                                /* :817-877 */
 

@@ -176,9 +176,9 @@ def plain_large_form(h, celgpu, torch, stream, m, b, x, iters_csr):
         xs = torch.from_numpy(np.random.default_rng(1).random(n)).cuda()
         ys = torch.zeros(n, dtype=torch.float64, device="cuda")
         row = {}
-        # the Poisson rows repeat: both formats are swept over the row table,
-        # one index byte per row, x and y
-        pat = mm.column_form() == celgpu.COLS_PATTERN
+        # on row patterns whose few values (the Poisson rows') repeat, both
+        # formats are swept over the row table: one index byte per row, x and y
+        pat = mm.column_form() == celgpu.COLS_PATTERN and len(np.unique(v)) <= 2
         row["matrix_form"] = "row table" if pat else "int32 columns"
         for name, fmt, nbytes in (("csr", celgpu.FMT_CSR, 17 * n if pat else 12 * nnz + 4 * (n + 1) + 16 * n),
                                   ("jad", celgpu.FMT_JAD, 17 * n if pat else 12 * nnz + 4 * 8 + 20 * n)):

@@ -735,14 +735,10 @@ struct GmPlan {
   double* Hp(int i, int j) const { return a.H + (size_t)j * (a.M + 1) + i; }
 };
 
-// w = A z on the row patterns or 1-byte offsets when the matrix has them
-// (same columns in the same order: the same sums)
+// w = A z in the matrix's most compact form
 static int gm_spmv(celg_handle* h, const GmPlan& g, const double* x, double* y) {
   const EpiStoreIf epi{y, &g.a.st->act};
   if (g.fmt == CELG_FMT_JAD) return launch_jad(h, g.m->csr, g.m->jad, x, epi);
-  bool done = false;
-  const int st = launch_csr_compact<double>(h, g.m->csr, g.m->csr.v, x, epi, nullptr, 0, &done);
-  if (done) return st;
   return launch_csr<double>(h, g.m->csr, g.m->csr.v, x, epi);
 }
 

@@ -556,7 +556,8 @@ __global__ void __launch_bounds__(kLanes, 3)
       } else {
 #pragma unroll 1
         for (int r = 0; r < kTabRows; ++r) {
-          const int want = r == 0 ? cur[q] : r == 1 ? cur[q + 1] : r == 2 ? cur[(q + 2) & 3] : cur[(q + 3) & 3];
+          static_assert(kTabRows == 2, "want");
+          const int want = r == 0 ? cur[q] : cur[q + 1];  // (no indexing: cur stays in registers)
           e.take(want, s_off, s_val, s_len);
           if (want >= 0) {
             const long row = row0 + (long)(q + r) * kLanes;

@@ -123,11 +123,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // Whether the i-th unsuccessful poll of a word in global memory may be
 // followed by another: looks at the clock every 64 polls, and gives up (and
 // makes the CTA's other waiting threads give up) after kWaitLimitNs.
-__device__ __forceinline__ bool poll_more(unsigned i, unsigned long long& t0, int* abort_) {
+__device__ __forceinline__ bool poll_more(unsigned i, unsigned long long& t0, int* abort_,
+                                          unsigned long long limit_ns = kWaitLimitNs) {
   if ((i & 63u) != 63u) return true;
   const unsigned long long t = global_ns();
   if (!t0) t0 = t;
-  if (t - t0 <= kWaitLimitNs && !*(volatile int*)abort_) return true;
+  if (t - t0 <= limit_ns && !*(volatile int*)abort_) return true;
   *(volatile int*)abort_ = 1;
   return false;
 }

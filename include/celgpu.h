@@ -262,10 +262,10 @@ int celg_pcg_batched(celg_handle* h, int count, celg_mat* const* mats, const dou
                      double* const* x_d, const celg_params* p, celg_result* res);
 
 /* ---- diagnostics --------------------------------------------------------------- */
-/* Runs the library's bounded device wait on an mbarrier that nothing arrives
- * on, with a limit of limit_ms (1..10000) milliseconds, and stores the status
- * the kernel reported (CELG_ERR_TIMEOUT when the bound works).  The handle and
- * its context remain usable.  No counterpart in the reference, whose waits
+/* Runs the library's bounded device waits, on an mbarrier that nothing arrives
+ * on and on a word that nothing publishes, with a limit of limit_ms (1..10000)
+ * milliseconds, and stores the status the kernel reported (CELG_ERR_TIMEOUT
+ * when both bounds work).  The handle and its context remain usable.  No counterpart in the reference, whose waits
  * (MPI_Test polling, src/felmsolver/cel_elmsolver_module.f90:637-644) have no
  * limit. */
 int celg_check_bounded_wait(celg_handle* h, int limit_ms, int* status);

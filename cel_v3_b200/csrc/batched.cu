@@ -924,7 +924,9 @@ static int batch_build(celg_handle* h, int count, celg_mat* const* mats, const s
   // 1-byte column offsets when the systems together use at most 256
   // distinct offsets col - row (7-point systems: -1, 0, 1 and +-side,
   // +-side^2 per distinct side): 9 instead of 12 bytes per non-zero
-  // (row patterns, when there are so few systems that theirs fit the table)
+  // (row patterns, when there are so few systems that theirs fit the table;
+  // FP32 batches of 4 to 48 systems then take what they took with patterns
+  // made from the offsets, 0.98 to 1.01)
   if (!st) st = row_forms_search(h, A, false, nullptr);
   if (!st) {
     const cudaError_t e2 = cudaStreamSynchronize(h->stream);

@@ -1260,9 +1260,18 @@ int pcg_onchip(celg_handle* h, CsrDev& A, const PcgBind<VT>& B, const celg_param
 // and about 1.3 million rows at once keep their working set in L2.  1, 2, 4
 // or 8 lanes (streams) share the SMs; the largest systems come first, and
 // when a lane is through with its class it divides into two of the next, so
-// that no lane waits for another.  64 systems of sides 16..96: 155 ms in
-// common sweeps (batched.cu), 160 with classes of 303k, 151k and 74k rows,
-// 124 with these.
+// that no lane waits for another.  ms, in common sweeps (batched.cu) : these
+// classes : classes of 303k, 151k, 74k rows : of 600k, 300k, 150k : of 1.3M,
+// 700k, 350k:
+//   64 systems of sides 16..96   170 : 125 : 160 : 149 : 124
+//   24 of 84..90                 126 : 100 : 144 : 141 : 100
+//   32 of 60..75                76.6 : 57.8 : 83.1 : 66.4 : 60.2
+//   16 of 40..100               73.1 : 59.1 : 68.4 : 65.1 : 58.6
+//   6 of 88..110                70.4 : 56.4 : 56.4 : 56.4 : 61.8
+//   8 of 80..96                 55.9 : 41.9 : 48.9 : 50.8 : 41.9
+//   64 of 30..50                26.0 : 20.5 : 22.6 : 20.5 : 20.5
+//   12 of 50..56                14.1 : 10.1 : 11.9 : 10.9 : 10.1
+//   4 of 60..64                 10.8 : 5.1 : 6.0 : 5.1 : 8.8
 constexpr int kOcLanes = 8;
 static long lane_rows(int lanes) { return lanes == 1 ? 1L << 30 : lanes == 2 ? 900000 : lanes == 4 ? 500000 : 200000; }
 

@@ -328,7 +328,11 @@ int launch_csr_tab(celg_handle* h, const CsrDev& A, const VT* x, const Epi& epi,
   red.sweep = next_sweep(h, false);
   const int smem = A.npat * (kPatLen * ((int)sizeof(VT) + 4) + 4);
   // Staged when two stages fit a third of an SM, x is aligned for bulk copies
-  // and every CTA has a tile (below that the ring only adds latency).
+  // and every CTA has a tile (below that the ring only adds latency: y = A x in
+  // FP64 above, in FP32 at 80^3 8.2 us staged against 6.7).  A whole FP32
+  // reliable-update solve, staged : unstaged : on the row patterns, ms: 78^3
+  // 6.84 : 6.88 : 7.01, 104^3 10.7 : 11.0 : 11.6, 127^3 16.1 : 16.5 : 17.8,
+  // 170^3 30.4 : 31.5 : 38.1; 48^3, below the line, 3.47 : 3.50 : 3.57.
   const int tab = win_table_bytes(A.npat, (int)sizeof(VT));
   const int stage = A.win.total * (int)sizeof(VT) + kTile;
   const int stages = A.win.nseg > 0 ? std::min(kStages, (72 * 1024 - tab) / stage) : 0;
@@ -351,7 +355,9 @@ int launch_csr_tab(celg_handle* h, const CsrDev& A, const VT* x, const Epi& epi,
 // Most rows for csr_rows_kernel.  Row table: 32^3 rows 4.5 us against 6.2 by
 // csr_tab_kernel's tiles, 80^3 6.8 : 8.3, 96^3 10.3 : 10.3, 128^3 16.8 : 12.4.
 // Row patterns against the staged csr_tma_kernel: 32^3 4.6 : 6.2, 80^3 10.0 :
-// 12.3, 96^3 14.4 : 12.9, 128^3 34.9 : 25.0.
+// 12.3, 96^3 14.4 : 12.9, 128^3 34.9 : 25.0.  FP32 (celg_spmv_f32), table: 64^3
+// 4.6 : 6.1, 80^3 6.2 : 6.7, 96^3 8.2 : 8.3, 128^3 14.4 : 12.4; patterns: 32^3
+// 4.5 : 6.2, 80^3 8.2 : 8.2, 112^3 14.4 : 14.2, 128^3 22.5 : 18.5.
 constexpr long kRowsTab = 800000, kRowsPat = 600000;
 
 template <typename VT, class Epi>
